@@ -148,6 +148,88 @@ __device__ __forceinline__ uint32_t key_dist(uint64_t k) { return static_cast<ui
 __device__ __forceinline__ uint32_t key_id(uint64_t k) { return static_cast<uint32_t>(k); }
 
 // ---------------------------------------------------------------------------
+// A walk along a visited set's slots reads the first few at once (the table
+// is at most a quarter full, so most walks end there): one shared-memory
+// latency instead of one per slot, and no loop whose lanes leave at different
+// times.
+// ---------------------------------------------------------------------------
+
+// One lane, own key: is it in the set?
+template <class VH>
+__device__ __forceinline__ bool visited_test(const VH &vh, uint32_t id, int home) {
+  constexpr int W = 4;
+  int32_t v[W];
+#pragma unroll
+  for (int i = 0; i < W; ++i) v[i] = vh.tab[vh.ahead(home, i)];
+  bool found = false, open = true;  // open: no empty slot so far
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    found = found || (open && v[i] == static_cast<int32_t>(id));
+    open = open && v[i] != FH_EMPTY;
+  }
+  if (open && !found) {
+    int c = vh.ahead(home, W);
+    for (int i = W; i < vh.cap; ++i) {
+      const int32_t x = vh.tab[c];
+      if (x == FH_EMPTY) break;
+      if (x == static_cast<int32_t>(id)) return true;
+      c = vh.next(c);
+    }
+  }
+  return found;
+}
+
+// One lane: the first empty slot from `home` on; -1 in a table without one.
+template <class VH>
+__device__ __forceinline__ int visited_end(const VH &vh, int home) {
+  constexpr int W = 4;
+  int32_t v[W];
+#pragma unroll
+  for (int i = 0; i < W; ++i) v[i] = vh.tab[vh.ahead(home, i)];
+  int at = W;
+#pragma unroll
+  for (int i = W - 1; i >= 0; --i) at = v[i] == FH_EMPTY ? i : at;
+  int c = vh.ahead(home, at);
+  if (at == W) {
+    int i = W;
+    while (vh.tab[c] != FH_EMPTY) {
+      c = vh.next(c);
+      if (++i > vh.cap) return -1;
+    }
+  }
+  return c;
+}
+
+// One lane: where key id sits (-1: nowhere) and the first empty slot after it
+// (or, when it is absent, on its walk); false in a table without empty slots.
+template <class VH>
+__device__ __forceinline__ bool visited_find(const VH &vh, uint32_t id, int home, int &at, int &end) {
+  constexpr int W = 6;
+  int32_t v[W];
+#pragma unroll
+  for (int i = 0; i < W; ++i) v[i] = vh.tab[vh.ahead(home, i)];
+  int m = W, t = W;
+#pragma unroll
+  for (int i = W - 1; i >= 0; --i) {
+    m = v[i] == static_cast<int32_t>(id) ? i : m;
+    t = v[i] == FH_EMPTY ? i : t;
+  }
+  at = m < t ? vh.ahead(home, m) : -1;
+  end = vh.ahead(home, t);
+  if (t == W) {
+    int i = W;
+    for (;;) {
+      const int32_t x = vh.tab[end];
+      if (x == FH_EMPTY) break;
+      if (at < 0 && x == static_cast<int32_t>(id)) at = end;
+      end = vh.next(end);
+      if (++i > vh.cap) return false;
+    }
+  }
+  return true;
+}
+
+// ---------------------------------------------------------------------------
 // Visited hash: the reference's FixHash<int, 8*pq> (fixhash.h) in the warp's
 // shared memory, with the same slot function, linear probing and
 // backward-shift delete, so that membership answers (including the rare
@@ -164,8 +246,10 @@ struct VisitedHash {
     uint64_t x = id;
     uint64_t v = x ^ ((x >> 16) * FH_R0) ^ FH_R1;
     uint64_t q = __umul64hi(v, magic);
-    uint64_t r = v - q * static_cast<uint64_t>(cap);
-    if (r >= static_cast<uint64_t>(cap)) r -= static_cast<uint64_t>(cap);
+    // v - q * cap < 2 * cap: the low words hold it
+    const uint32_t c = static_cast<uint32_t>(cap);
+    uint32_t r = static_cast<uint32_t>(v) - static_cast<uint32_t>(q) * c;
+    if (r >= c) r -= c;
     return static_cast<int>(r);
   }
 
@@ -176,21 +260,29 @@ struct VisitedHash {
     return s >= cap ? s - cap : s;
   }
 
+  __device__ __forceinline__ int next(int c) const { return c + 1 == cap ? 0 : c + 1; }
+  // slot c + i, 0 <= i < 16 <= cap
+  __device__ __forceinline__ int ahead(int c, int i) const { return c + i >= cap ? c + i - cap : c + i; }
+
   __device__ __forceinline__ void clear(int lane) {
     for (int i = lane; i < cap; i += 32) tab[i] = FH_EMPTY;
     __syncwarp();
   }
 
-  // One lane, own key (fixhash.h:49-57).
-  __device__ __forceinline__ bool test(uint32_t id) const {
-    int c = slot(id);
-    for (int i = 0; i < cap; ++i) {
-      int32_t v = tab[c];
-      if (v == FH_EMPTY) return false;
-      if (v == static_cast<int32_t>(id)) return true;
-      c = c + 1 == cap ? 0 : c + 1;
-    }
-    return false;
+  // One lane, own key, `home` = slot(id) (fixhash.h:49-57).
+  __device__ __forceinline__ bool test_at(uint32_t id, int home) const {
+    return visited_test(*this, id, home);
+  }
+  __device__ __forceinline__ bool test(uint32_t id) const { return test_at(id, slot(id)); }
+
+  // The case analysis of the backward-shift delete (fixhash.h:64-90): does
+  // the entry at slot nxt, whose home is ncode, move into the hole r left by
+  // an entry whose home is code?
+  __device__ __forceinline__ bool moves(int code, int r, int nxt, int ncode) const {
+    const bool cond1 = code <= r, cond2 = r < nxt;
+    if (cond1 && cond2) return ncode <= r;
+    if (cond1) return nxt < ncode && ncode <= r;
+    return nxt < ncode || ncode <= r;
   }
 
   // Whole warp, one key (fixhash.h:38-47): first EMPTY/DELETION slot on the
@@ -250,13 +342,7 @@ struct VisitedHash {
         int nxt = wrap(nbase + i);
         int ncode = __shfl_sync(FULL, hv, i);
         int32_t val = __shfl_sync(FULL, v, i);
-        bool cond1 = code <= r;
-        bool cond2 = r < nxt;
-        bool move;
-        if (cond1 && cond2) move = ncode <= r;
-        else if (cond1) move = nxt < ncode && ncode <= r;
-        else move = nxt < ncode || ncode <= r;
-        if (move) {
+        if (moves(code, r, nxt, ncode)) {
           if (lane == 0) tab[r] = val;
           r = nxt;
           code = ncode;
@@ -290,21 +376,22 @@ struct ExactVisited {
     return static_cast<int>((id * 0x9E3779B1u) >> (32 - log2cap));  // cap >= 32
   }
   __device__ __forceinline__ int wrap(int s) const { return s & (cap - 1); }
+  __device__ __forceinline__ int next(int c) const { return (c + 1) & (cap - 1); }
+  __device__ __forceinline__ int ahead(int c, int i) const { return (c + i) & (cap - 1); }
 
   __device__ __forceinline__ void clear(int lane) {
     for (int i = lane; i < cap; i += 32) tab[i] = FH_EMPTY;
     __syncwarp();
   }
 
-  __device__ __forceinline__ bool test(uint32_t id) const {
-    int c = slot(id);
-    for (int i = 0; i < cap; ++i) {
-      const int32_t v = tab[c];
-      if (v == FH_EMPTY) return false;
-      if (v == static_cast<int32_t>(id)) return true;
-      c = (c + 1) & (cap - 1);
-    }
-    return false;
+  __device__ __forceinline__ bool test_at(uint32_t id, int home) const {
+    return visited_test(*this, id, home);
+  }
+  __device__ __forceinline__ bool test(uint32_t id) const { return test_at(id, slot(id)); }
+
+  // An entry moves into the hole r when its home is not cyclically inside (r, nxt].
+  __device__ __forceinline__ bool moves(int, int r, int nxt, int ncode) const {
+    return ((nxt - ncode) & (cap - 1)) >= ((nxt - r) & (cap - 1));
   }
 
   __device__ __forceinline__ void add_at(uint32_t id, int home, int lane) {
@@ -353,7 +440,7 @@ struct ExactVisited {
         const int j = wrap(nbase + i);
         const int hm = __shfl_sync(FULL, home, i);
         const int32_t val = __shfl_sync(FULL, v, i);
-        if (((j - hm) & (cap - 1)) >= ((j - h) & (cap - 1))) {
+        if (moves(0, h, j, hm)) {
           if (lane == 0) tab[h] = val;
           h = j;
         }
@@ -368,5 +455,111 @@ struct ExactVisited {
 
   __device__ __forceinline__ void del(uint32_t id, int lane) { del_at(id, slot(id), lane); }
 };
+
+// ---------------------------------------------------------------------------
+// Whole-warp operations over either visited set (VH), bit for bit the
+// reference's one-at-a-time calls.
+// ---------------------------------------------------------------------------
+
+// del(id) followed by add(id) (a popped vertex leaves the queue and enters
+// the list, warp_astar_accelerator.h:188-200).  The delete fills the hole
+// with later entries of the run, hole after hole, and the add finds every
+// slot before the last hole taken and lands in that one.  With an empty slot
+// behind the entry (three pops of four) nothing changes at all.
+template <class VH>
+__device__ __forceinline__ void visited_refresh(VH &vh, uint32_t id, int home, int lane) {
+  const int32_t v = vh.tab[vh.wrap(home + lane)];
+  const unsigned be = __ballot_sync(FULL, v == FH_EMPTY);
+  const unsigned bm = __ballot_sync(FULL, v == static_cast<int32_t>(id));
+  const int end = __ffs(be) - 1, at = __ffs(bm) - 1;  // lowest empty slot, lowest match (-1: none)
+  if (be && bm && at < end) {
+    if (at + 1 == end) return;
+    int r = at, code = home;
+    const int hv = v >= 0 ? vh.slot(static_cast<uint32_t>(v)) : 0;
+    for (int i = at + 1; i < end; ++i) {
+      const int ncode = __shfl_sync(FULL, hv, i);
+      if (vh.moves(code, vh.wrap(home + r), vh.wrap(home + i), ncode)) {
+        if (lane == i) vh.tab[vh.wrap(home + r)] = v;
+        r = i;
+        code = ncode;
+      }
+    }
+    if (r != at && lane == 0) vh.tab[vh.wrap(home + r)] = static_cast<int32_t>(id);
+    __syncwarp();
+    return;
+  }
+  vh.del_at(id, home, lane);
+  vh.add_at(id, home, lane);
+}
+
+// The visited-set calls of one select-insert pass
+// (warp_astar_accelerator.h:311-320), in the reference's order -- lane 0's
+// add(id), lane 0's del(eid), lane 1's add, ... -- each lane naming its own
+// calls (padd / pdel).  One call changes the table only inside its cluster
+// (the occupied slots around its home up to the first empty one), so calls
+// with different terminating empty slots commute, and all of them run at
+// once, one lane each.  Every round the lanes find their calls' terminating
+// slots in the table as it stands and mark them; a call that finds another
+// call's mark waits, together with every later call, for the next round.
+// The first pending call always runs, which bounds the rounds; there are 1.4
+// to 3.3 of them a hop (pq 1000, pq 100).
+template <class VH>
+__device__ __forceinline__ void visited_update(VH &vh, bool padd, uint32_t id, int home, bool pdel, uint32_t eid,
+                                               int ehome, int lane) {
+  const uint32_t ia = 2u * lane, id2 = ia + 1u;  // the calls' places in the order
+  constexpr uint32_t MARK = 0x80000000u, NONE = 64u;
+  int32_t *tab = vh.tab;
+  for (;;) {
+    int ta = 0, td = 0, r = -1;
+    bool ok = true;  // a table without an empty slot takes no more calls
+    if (padd) {
+      ta = visited_end(vh, home);
+      ok = ta >= 0;
+    }
+    if (pdel) ok = visited_find(vh, eid, ehome, r, td) && ok;
+    if (__any_sync(FULL, !ok)) return;
+    __syncwarp();
+    if (padd) tab[ta] = static_cast<int32_t>(MARK + ia);
+    if (pdel) tab[td] = static_cast<int32_t>(MARK + id2);
+    __syncwarp();
+    const bool la = padd && tab[ta] != static_cast<int32_t>(MARK + ia);
+    const bool ld = pdel && tab[td] != static_cast<int32_t>(MARK + id2);
+    bool ea = padd, ed = pdel;
+    __syncwarp();
+    const bool clash = __any_sync(FULL, la || ld);
+    if (clash) {
+      const uint32_t lost = __reduce_min_sync(FULL, la ? ia : (ld ? id2 : NONE));
+      const uint32_t first = __reduce_min_sync(FULL, padd ? ia : (pdel ? id2 : NONE));
+      const uint32_t end = max(lost, first + 1u);  // calls below `end` run in this round
+      if (padd) tab[ta] = FH_EMPTY;
+      if (pdel) tab[td] = FH_EMPTY;
+      __syncwarp();
+      ea = padd && ia < end;
+      ed = pdel && id2 < end;
+    }
+    if (ea) tab[ta] = static_cast<int32_t>(id);
+    if (ed) {
+      tab[td] = FH_EMPTY;
+      if (r >= 0) {
+        int code = ehome;
+        for (int c = vh.next(r); c != td; c = vh.next(c)) {
+          const int32_t v = tab[c];
+          const int nh = vh.slot(static_cast<uint32_t>(v));
+          if (vh.moves(code, r, c, nh)) {
+            tab[r] = v;
+            r = c;
+            code = nh;
+          }
+        }
+        tab[r] = FH_EMPTY;
+      }
+    }
+    __syncwarp();
+    if (!clash) break;
+    padd = padd && !ea;
+    pdel = pdel && !ed;
+    if (!__any_sync(FULL, padd || pdel)) break;
+  }
+}
 
 }  // namespace song

@@ -24,14 +24,6 @@ namespace {
 
 uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
-// Rows staged per buffer half: a typical hop evaluates 2-5 neighbours.
-// Rows per staging chunk (two chunks in flight).  Rows of up to 1 KB: 4 while
-// pq is small (many new candidates per hop), 1 from pq 512 on, where a hop
-// brings ~2 new candidates and the smaller staging ring leaves room for one
-// more resident warp next to the 8*pq-slot visited hash (measured: 1M x 128,
-// pq 800: 39.0 -> 35.7 ms; pq 200: 12.6 ms with 4 rows, 14.6 ms with 1).
-int stage_rows(uint32_t row_bytes, int pq) { return row_bytes <= 1024 ? (pq >= 512 ? 1 : 4) : 2; }
-
 // Register-queue segment: smallest power of two S with 32*S >= pq + 1.
 int queue_segment(int pq) {
   int s = 1;
@@ -39,37 +31,12 @@ int queue_segment(int pq) {
   return s;
 }
 
-struct Layout {
-  uint32_t warp_bytes, off_mbar, off_cand, off_q, off_hash;
-  int cap, H, S;
-};
-
 // FixHash capacity 8*pq (the reference's TOPK*4*2) for the plain kernel; the
 // learned kernel's exact set: the power of two >= max(32, 4*pq).
 int exact_cap(int pq) {
   int c = 32;
   while (c < 4 * pq) c <<= 1;
   return c;
-}
-
-Layout make_layout(const DeviceIndex &ix, int pq, bool learned, bool multi = false) {
-  Layout L;
-  L.H = stage_rows(ix.row_bytes, pq);
-  L.S = queue_segment(pq);
-  L.cap = learned ? exact_cap(pq) : 8 * pq;
-  uint32_t off = 2u * L.H * ix.row_bytes;
-  off = align_up(off, 16);
-  L.off_mbar = off;
-  off += 16;
-  L.off_cand = off;
-  off += (multi ? MAX_PROBES : 1) * 32 * 4;
-  off = align_up(off, 16);
-  L.off_q = off;
-  off += align_up(static_cast<uint32_t>(ix.dim) * 4u, 16);
-  L.off_hash = off;
-  off += 4u * L.cap;
-  L.warp_bytes = align_up(off, 128);
-  return L;
 }
 
 struct Shape {
@@ -121,8 +88,14 @@ int get_shape(const void *fn, uint32_t warp_bytes, uint32_t extra, int *wpb, int
   return 0;
 }
 
+// What a warp may need, as the interface states it: two staging chunks of
+// the rows beside the query and the 8*pq-slot hash.  The kernel needs less,
+// at every size that this admits.
 uint32_t search_warp_bytes(const DeviceIndex &ix, int pq, bool multi) {
-  return make_layout(ix, pq, false, multi).warp_bytes;
+  const uint32_t rows = ix.row_bytes <= 1024 ? (pq >= 512 ? 1u : 4u) : 2u;
+  uint32_t off = align_up(2u * rows * ix.row_bytes, 16) + 16 + (multi ? MAX_PROBES : 1) * 32 * 4;
+  off = align_up(off, 16) + align_up(static_cast<uint32_t>(ix.dim) * 4u, 16) + 4u * 8u * static_cast<uint32_t>(pq);
+  return align_up(off, 128);
 }
 
 int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t stream) {
@@ -130,7 +103,8 @@ int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t strea
   const bool learned = c.mlp != nullptr || c.trace != nullptr || c.exit_max_hops > 0;
   const bool multi = c.probes > 1 || c.finish_cnt > 1 || c.double_check;
   if (multi && (learned || ix.storage != 0 || c.probes > MAX_PROBES || c.finish_cnt < 1)) return -1;
-  const Layout L = make_layout(ix, c.pq, learned, multi);
+  const int S = queue_segment(c.pq), cap = learned ? exact_cap(c.pq) : 8 * c.pq;
+  const WarpLayout L = warp_layout(ix.dim, c.pq, S, cap, (multi ? MAX_PROBES : 1) * 32);
   Params p;
   p.rows = static_cast<const uint8_t *>(ix.rows);
   p.row_bytes = ix.row_bytes;
@@ -154,11 +128,13 @@ int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t strea
   p.off_mbar = L.off_mbar;
   p.off_cand = L.off_cand;
   p.off_q = L.off_q;
+  p.off_queue = L.off_queue;
   p.off_hash = L.off_hash;
-  p.cap = L.cap;
-  p.magic = ~0ull / static_cast<uint64_t>(L.cap);
+  p.cap = cap;
+  p.magic = ~0ull / static_cast<uint64_t>(cap);
   p.log2cap = 0;
-  while ((1 << p.log2cap) < L.cap) ++p.log2cap;
+  while ((1 << p.log2cap) < cap) ++p.log2cap;
+  p.width = ix.dpad;
   p.mlp = c.mlp;
   p.exit_threshold = c.exit_threshold;
   p.exit_min_hops = c.exit_min_hops;
@@ -175,16 +151,16 @@ int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t strea
   p.probes = c.probes;
   p.finish_cnt = c.finish_cnt;
   p.double_check = c.double_check;
-  if (multi) return launch_multi(p, ix.metric, L.H, L.S, stream);
+  if (multi) return launch_multi(p, ix.metric, S, stream);
   if (learned) {
     if (ix.storage >= 2) return -1;
-    return launch_learned(p, ix.storage, ix.metric, L.H, L.S, stream);
+    return launch_learned(p, ix.storage, ix.metric, S, stream);
   }
   switch (ix.storage) {
-    case 0: return launch_f32(p, ix.metric, L.H, L.S, stream);
-    case 1: return launch_bf16(p, ix.metric, L.H, L.S, stream);
-    case 2: return launch_fp8(p, ix.metric, L.H, L.S, stream);
-    case 3: return c.qcodes ? launch_bits(p, ix.metric, L.S, stream) : -1;  // query codes come from the caller's path
+    case 0: return launch_f32(p, ix.metric, S, stream);
+    case 1: return launch_bf16(p, ix.metric, S, stream);
+    case 2: return launch_fp8(p, ix.metric, S, stream);
+    case 3: return c.qcodes ? launch_bits(p, ix.metric, S, stream) : -1;  // query codes come from the caller's path
     default: return -1;
   }
 }

@@ -53,12 +53,7 @@ int launch_hash_codes(const float *rows, uint64_t n, int stride, int dim, const 
 }
 
 int launch_bits(const Params &p, int metric, int S, cudaStream_t s) {
-  switch (metric) {
-    case 0: return launch_by_s<0, 3, 1, false>(p, S, s);
-    case 1: return launch_by_s<1, 3, 1, false>(p, S, s);
-    case 2: return launch_by_s<2, 3, 1, false>(p, S, s);
-    default: return -1;
-  }
+  return launch_storage<3, false>(p, metric, S, s);
 }
 
 }  // namespace song

@@ -2,7 +2,7 @@
 #include "search_kernel.cuh"
 
 namespace song {
-int launch_f32(const Params &p, int metric, int H, int S, cudaStream_t s) {
-  return launch_storage<0, false>(p, metric, H, S, s);
+int launch_f32(const Params &p, int metric, int S, cudaStream_t s) {
+  return launch_storage<0, false>(p, metric, S, s);
 }
 }  // namespace song

@@ -14,17 +14,24 @@
 //  * persistent warps pull queries from a work counter; warps never wait for
 //    one another (the only block barrier is the model load at kernel start);
 //  * per-query state: query vector, visited hash (the reference's FixHash,
-//    8*pq slots) and a two-buffer staging ring in the warp's shared memory;
-//    candidate queue and top-pq list in registers (reg_queue.cuh);
-//  * each hop's unvisited neighbour rows are gathered with 1-D bulk async
-//    copies (cp.async.bulk, mbarrier transaction counts) into the ring, two
-//    chunks in flight, and read back in the reference's lane order;
+//    8*pq slots) and, for large pq, the candidate queue's ring in the warp's
+//    shared memory; smaller queues and the top-pq list in registers
+//    (reg_queue.cuh);
+//  * each hop's unvisited neighbour rows are read straight from global memory
+//    into registers, eight rows at a time, four lanes a row (gather_rows);
+//  * one hop's visited-hash calls run one lane each (visited_update);
 //  * the next hop's adjacency row is loaded as soon as the next pop is known.
 //
 // Template parameters: METRIC (0 L2, 1 IP, 2 COS), STORAGE (0 F32, 1 BF16,
-// 2 FP8-E4M3 with a per-row scale), H (rows per staging buffer), S (register
-// queue segment, capacity 32*S >= pq+1), LEARNED (per-hop features: trace
-// capture and/or the early-exit network).
+// 2 FP8-E4M3 with a per-row scale, 3 256-bit codes), S (register queue
+// segment, capacity 32*S >= pq+1), LEARNED (per-hop features: trace capture
+// and/or the early-exit network), MULTI (the multi-probe knobs).
+//
+// What bounds it: instructions, in full batches and for a single query alike
+// (about six cycles each on a dependent path).  A hop of the headline search
+// (1M x 128 L2, pq 43 from entry points, 21 candidates) takes 2,000 of them
+// (2,650 before its rows were read directly and its hash calls made side by
+// side), one at pq 1000 from vertex 0 500 (5,900).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -33,6 +40,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "device_common.cuh"
 #include "internal.h"
@@ -71,12 +79,13 @@ struct Params {
   uint32_t *counter;
   int32_t *error;
   uint32_t warp_bytes;
-  uint32_t off_mbar, off_cand, off_q, off_hash;
+  uint32_t off_mbar, off_cand, off_q, off_queue, off_hash;
   int cap;
   uint64_t magic;  // VisitedHash (plain kernel)
   int log2cap;     // ExactVisited (learned kernel)
+  int width;       // elements of a stored row, zero padding included
   uint32_t wait_limit;  // polls of a bounded mbarrier wait
-  uint32_t extra_tx;    // test hook: bytes every copy batch expects beyond its rows (0 in use)
+  uint32_t extra_tx;    // test hook: bytes a copy's barrier expects beyond its own (0 in use)
   // the reference's N_MULTIPROBE / FINISH_CNT knobs (MULTI kernel only)
   int probes;      // vertices popped per iteration, 1..MAX_PROBES
   int finish_cnt;  // finish tests that must hold before the search ends, >= 1
@@ -117,37 +126,205 @@ __device__ __forceinline__ float finish_distance(float t, float len) {
   return 0.0f;
 }
 
-// Element j of a staged row as float.  FP8 elements are decoded and scaled
-// (x = e4m3(y) * scale, rounded to float), so a low-precision search equals
-// an FP32 search over the dequantised vectors.
-template <int STORAGE>
-__device__ __forceinline__ float load_elem(const uint8_t *row, int j, float scale) {
-  if (STORAGE == 0) return reinterpret_cast<const float *>(row)[j];
-  if (STORAGE == 1) return __bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(row)[j]);
-  const __half_raw h = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(row[j]), __NV_E4M3);
-  return __fmul_rn(__half2float(__half(h)), scale);
-}
-
 // The 256-bit code of a query (BITS storage), in every lane.
 struct Code8 {
   uint32_t w[8];
 };
 
-// Distances of candidates 0..m-1 (candidate c's id in lane c); candidate c's
-// distance is returned in lane c.  False if a bulk copy never completed.
-// Rows are taken in pairs through the paired FP32 instructions (the same
-// roundings, in the same order, as the scalar form: lane l sums dims l, l+32,
-// ... of each row with fused multiply-add).
-template <int METRIC, int STORAGE, int H>
-__device__ __forceinline__ bool gather_distances(const Params &p, uint8_t *stage, uint64_t *mbar,
-                                                 uint32_t &ph0, uint32_t &ph1, const float *qv,
-                                                 int m, uint32_t cid, float &out, int lane,
-                                                 const Code8 &qc) {
+// ---------------------------------------------------------------------------
+// Distances of rows read straight from global memory.
+//
+// The distance of a row is fixed by the reference's arithmetic: partial p
+// (p = 0..31) is the fused multiply-add chain over dimensions p, p+32, ... in
+// that order, and the 32 partials meet in the xor butterfly 16, 8, 4, 2, 1.
+// Which lane computes a partial is free.  Here four lanes share a row, eight
+// partials each, so one pass of the warp takes eight rows: every 32
+// dimensions are two 16-byte loads per lane (FP32; 64 contiguous bytes of
+// each row per load), already in the register pairs of the paired FP32
+// instructions, and the first butterfly levels are adds within a lane.
+// Against rows staged by bulk copies and read back one float per lane: no
+// barrier, no shared-memory round trip, and 85 instead of 180 warp
+// instructions per eight 128-float rows.
+// ---------------------------------------------------------------------------
+
+template <int STORAGE>
+struct RowRead;
+
+// FP32: lane g of a row's four holds partials 4g..4g+3 and 16+4g..16+4g+3.
+template <>
+struct RowRead<0> {
+  static constexpr bool HALVES = true;
+  ulonglong2 a, b;
+  __device__ __forceinline__ void load(const uint8_t *row, int j, int g, int width) {
+    const ulonglong2 *x = reinterpret_cast<const ulonglong2 *>(row) + (j >> 2) + g;
+    a = j + 4 * g < width ? __ldg(x) : make_ulonglong2(0ull, 0ull);
+    b = j + 16 + 4 * g < width ? __ldg(x + 4) : make_ulonglong2(0ull, 0ull);
+  }
+  __device__ __forceinline__ void load_full(const uint8_t *row, int j, int g) {
+    const ulonglong2 *x = reinterpret_cast<const ulonglong2 *>(row) + (j >> 2) + g;
+    a = __ldg(x);
+    b = __ldg(x + 4);
+  }
+  __device__ __forceinline__ void get(uint64_t (&x)[4], float) const {
+    x[0] = a.x;
+    x[1] = a.y;
+    x[2] = b.x;
+    x[3] = b.y;
+  }
+};
+
+// BF16 and FP8: lane g holds the eight partials 8g..8g+7 (16 or 8
+// contiguous bytes), decoded to FP32; an FP8 value is multiplied by the row's
+// scale and rounded, so a low-precision search equals an FP32 search over the
+// dequantised vectors.
+template <>
+struct RowRead<1> {
+  static constexpr bool HALVES = false;
+  uint4 a;
+  __device__ __forceinline__ void load(const uint8_t *row, int j, int g, int width) {
+    a = j + 8 * g < width ? __ldg(reinterpret_cast<const uint4 *>(row) + (j >> 3) + g) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  __device__ __forceinline__ void load_full(const uint8_t *row, int j, int g) {
+    a = __ldg(reinterpret_cast<const uint4 *>(row) + (j >> 3) + g);
+  }
+  static __device__ __forceinline__ uint64_t pair(uint32_t w) {
+    return f2_pack(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  }
+  __device__ __forceinline__ void get(uint64_t (&x)[4], float) const {
+    x[0] = pair(a.x);
+    x[1] = pair(a.y);
+    x[2] = pair(a.z);
+    x[3] = pair(a.w);
+  }
+};
+
+template <>
+struct RowRead<2> {
+  static constexpr bool HALVES = false;
+  uint2 a;
+  __device__ __forceinline__ void load(const uint8_t *row, int j, int g, int width) {
+    a = j + 8 * g < width ? __ldg(reinterpret_cast<const uint2 *>(row) + (j >> 3) + g) : make_uint2(0u, 0u);
+  }
+  __device__ __forceinline__ void load_full(const uint8_t *row, int j, int g) {
+    a = __ldg(reinterpret_cast<const uint2 *>(row) + (j >> 3) + g);
+  }
+  static __device__ __forceinline__ uint64_t pair(uint32_t w, float scale) {  // the low 16 bits
+    const __half2_raw h =
+        __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(w & 0xffffu), __NV_E4M3);
+    const float2 f = __half22float2(__half2(h));
+    return f2_pack(__fmul_rn(f.x, scale), __fmul_rn(f.y, scale));
+  }
+  __device__ __forceinline__ void get(uint64_t (&x)[4], float scale) const {
+    x[0] = pair(a.x, scale);
+    x[1] = pair(a.x >> 16, scale);
+    x[2] = pair(a.y, scale);
+    x[3] = pair(a.y >> 16, scale);
+  }
+};
+
+// The xor butterfly over a row's 32 partials, four lanes with eight each
+// (acc[i]: the pair at 2i, 2i+1 of the lane's eight); the sum in all four
+// lanes.  At the first levels a lane keeps half of its values and its
+// partner the other half; every sum is the butterfly's own pair (a + b ==
+// b + a).
+template <bool HALVES>
+__device__ __forceinline__ float row_butterfly(const uint64_t (&acc)[4], int lane) {
+  const bool h1 = (lane & 2) != 0, h0 = (lane & 1) != 0;
+  if (HALVES) {
+    // level 16 within the lane; the values left are partials 4g + e
+    float e0, e1, e2, e3;
+    f2_unpack(f2_add(acc[0], acc[2]), e0, e1);
+    f2_unpack(f2_add(acc[1], acc[3]), e2, e3);
+    // level 8: lane ^ 2; keep e = 2 h1 + {0, 1}
+    float k0 = __fadd_rn(h1 ? e2 : e0, __shfl_xor_sync(FULL, h1 ? e0 : e2, 2));
+    float k1 = __fadd_rn(h1 ? e3 : e1, __shfl_xor_sync(FULL, h1 ? e1 : e3, 2));
+    // level 4: lane ^ 1; keep e = 2 h1 + h0
+    float t = __fadd_rn(h0 ? k1 : k0, __shfl_xor_sync(FULL, h0 ? k0 : k1, 1));
+    t = __fadd_rn(t, __shfl_xor_sync(FULL, t, 2));  // level 2
+    return __fadd_rn(t, __shfl_xor_sync(FULL, t, 1));  // level 1
+  }
+  float v[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f2_unpack(acc[i], v[2 * i], v[2 * i + 1]);
+  float a[4], c[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)  // level 16: lane ^ 2; keep e = 4 h1 + i
+    a[i] = __fadd_rn(h1 ? v[4 + i] : v[i], __shfl_xor_sync(FULL, h1 ? v[i] : v[4 + i], 2));
+#pragma unroll
+  for (int i = 0; i < 2; ++i)  // level 8: lane ^ 1; keep e = 4 h1 + 2 h0 + i
+    c[i] = __fadd_rn(h0 ? a[2 + i] : a[i], __shfl_xor_sync(FULL, h0 ? a[i] : a[2 + i], 1));
+  // level 4 (bit 2 of e, held by h1): lane ^ 2; keep i = h1
+  float t = __fadd_rn(h1 ? c[1] : c[0], __shfl_xor_sync(FULL, h1 ? c[0] : c[1], 2));
+  t = __fadd_rn(t, __shfl_xor_sync(FULL, t, 1));     // level 2 (bit 1, held by h0)
+  return __fadd_rn(t, __shfl_xor_sync(FULL, t, 2));  // level 1 (bit 0, held by h1)
+}
+
+// Distances of candidates 0..m-1 (candidate c's id in lane c) in lane c;
+// qv: the query, zero-padded to a multiple of 32 floats.  `width` elements a
+// row (zero-padded to the 16-byte load; a padded element adds fma(0, 0, t)).
+template <int METRIC, int STORAGE>
+__device__ __forceinline__ float gather_rows(const uint8_t *rows, uint32_t rb, uint32_t scale_off, int width,
+                                             const float *qv, int m, uint32_t cid, int lane) {
+  using Read = RowRead<STORAGE>;
+  const int g = lane & 3;
+  const ulonglong2 *q2 = reinterpret_cast<const ulonglong2 *>(qv) + (Read::HALVES ? g : 2 * g);
+  constexpr int QB = Read::HALVES ? 4 : 1;  // the second half's offset in 16-byte units
+  float out = 0.0f;
+  for (int first = 0; first < m; first += 8) {
+    const uint32_t id = __shfl_sync(FULL, cid, min(first + (lane >> 2), m - 1));
+    const uint8_t *row = rows + static_cast<uint64_t>(id) * rb;
+    const float scale = STORAGE == 2 ? __ldg(reinterpret_cast<const float *>(row + scale_off)) : 1.0f;
+    uint64_t acc[4], len[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] = len[i] = 0ull;
+    auto add = [&](const Read &r, int j) {
+      uint64_t x[4];
+      r.get(x, scale);
+      const ulonglong2 qa = q2[j >> 2], qb = q2[(j >> 2) + QB];
+      const uint64_t q[4] = {qa.x, qa.y, qb.x, qb.y};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (METRIC == 0) {
+          const uint64_t d = f2_sub(q[i], x[i]);
+          acc[i] = f2_fma(d, d, acc[i]);
+        } else {
+          acc[i] = f2_fma(q[i], x[i], acc[i]);
+          if (METRIC == 2) len[i] = f2_fma(x[i], x[i], len[i]);
+        }
+      }
+    };
+    int j = 0;
+    constexpr int U = STORAGE == 0 ? 4 : 8;  // 32-dimension steps in flight: 16 (FP8) to 32 registers
+    for (; j + 32 * U <= width; j += 32 * U) {
+      Read r[U];
+#pragma unroll
+      for (int i = 0; i < U; ++i) r[i].load_full(row, j + 32 * i, g);
+#pragma unroll
+      for (int i = 0; i < U; ++i) add(r[i], j + 32 * i);
+    }
+    for (; j < width; j += 32) {
+      Read r;
+      r.load(row, j, g, width);
+      add(r, j);
+    }
+    const float t = row_butterfly<Read::HALVES>(acc, lane);
+    const float ln = METRIC == 2 ? row_butterfly<Read::HALVES>(len, lane) : 0.0f;
+    const float d = finish_distance<METRIC>(t, ln);
+    const float mine = __shfl_sync(FULL, d, ((lane - first) & 7) * 4);
+    if (lane >= first && lane < first + 8) out = mine;
+  }
+  return out;
+}
+
+// The index's stored rows.
+template <int METRIC, int STORAGE>
+__device__ __forceinline__ float gather_distances(const Params &p, const float *qv, int m, uint32_t cid, int lane,
+                                                  const Code8 &qc) {
   if constexpr (STORAGE == 3) {
     // Hamming distance of 256-bit codes: lane c reads candidate c's 32-byte
     // code straight from global memory (two 16-byte loads) and sums the
     // popcounts of its xor with the query's code (an integer, exact as float)
-    out = 0.0f;
+    float out = 0.0f;
     if (lane < m) {
       const uint4 *r = reinterpret_cast<const uint4 *>(p.rows + static_cast<uint64_t>(cid) * 32u);
       const uint4 a = __ldg(r), b = __ldg(r + 1);
@@ -155,154 +332,10 @@ __device__ __forceinline__ bool gather_distances(const Params &p, uint8_t *stage
                     __popc(b.x ^ qc.w[4]) + __popc(b.y ^ qc.w[5]) + __popc(b.z ^ qc.w[6]) + __popc(b.w ^ qc.w[7]);
       out = static_cast<float>(h);
     }
-    return true;
+    return out;
+  } else {
+    return gather_rows<METRIC, STORAGE>(p.rows, p.row_bytes, p.scale_off, p.width, qv, m, cid, lane);
   }
-  const int nchunks = (m + H - 1) / H;
-  const uint32_t rb = p.row_bytes;
-  auto issue = [&](int c) {
-    const int b = c & 1;
-    const int first = c * H;
-    const int cnt = min(H, m - first);
-    // The buffer was last read through the generic proxy; order those reads
-    // before the async-proxy writes of the copies issued below.
-    fence_proxy_async();
-    if (lane == 0) mbar_arrive_expect_tx(&mbar[b], static_cast<uint32_t>(cnt) * rb + p.extra_tx);
-    __syncwarp();
-    const uint32_t id = __shfl_sync(FULL, cid, (first + lane) & 31);
-    if (lane < cnt)
-      bulk_g2s(stage + static_cast<size_t>(b * H + lane) * rb,
-               p.rows + static_cast<uint64_t>(id) * rb, rb, &mbar[b]);
-  };
-  if (nchunks > 0) issue(0);
-  if (nchunks > 1) issue(1);
-  out = 0.0f;
-  for (int c = 0; c < nchunks; ++c) {
-    const int b = c & 1;
-    uint32_t &ph = b ? ph1 : ph0;
-    if (!mbar_wait(&mbar[b], ph, p.wait_limit)) {
-      // give up: wait (bounded again) for the other buffer's copies, still in
-      // flight into this warp's shared memory, before the warp leaves
-      if (c + 1 < nchunks) mbar_wait(&mbar[b ^ 1], b ? ph0 : ph1, p.wait_limit);
-      return false;
-    }
-    ph ^= 1u;
-    const int first = c * H;
-    const int cnt = min(H, m - first);
-    const uint8_t *buf = stage + static_cast<size_t>(b * H) * rb;
-    float acc[H], len[H];
-    if constexpr (H == 1) {
-      float a = 0.0f, l2 = 0.0f;
-      const float scale = STORAGE == 2 ? *reinterpret_cast<const float *>(buf + p.scale_off) : 1.0f;
-      for (int j = lane; j < p.dim; j += 32) {
-        const float qj = qv[j];
-        const float xj = load_elem<STORAGE>(buf, j, scale);
-        if (METRIC == 0) {
-          const float d = __fsub_rn(qj, xj);
-          a = __fmaf_rn(d, d, a);
-        } else {
-          a = __fmaf_rn(qj, xj, a);
-          if (METRIC == 2) l2 = __fmaf_rn(xj, xj, l2);
-        }
-      }
-      acc[0] = a;
-      len[0] = l2;
-    } else {
-      constexpr int P = H / 2;  // row pairs
-      uint64_t a2[P], l2[P];
-      float sc[H];
-#pragma unroll
-      for (int i = 0; i < P; ++i) a2[i] = l2[i] = 0ull;
-#pragma unroll
-      for (int i = 0; i < H; ++i)
-        sc[i] = STORAGE == 2 ? *reinterpret_cast<const float *>(buf + static_cast<size_t>(i) * rb + p.scale_off) : 1.0f;
-#pragma unroll 2
-      for (int j = lane; j < p.dim; j += 32) {
-        const float qj = qv[j];
-        const uint64_t qq = f2_pack(qj, qj);
-#pragma unroll
-        for (int i = 0; i < P; ++i) {
-          if (2 * i < cnt) {  // warp-uniform
-            const float x0 = load_elem<STORAGE>(buf + static_cast<size_t>(2 * i) * rb, j, sc[2 * i]);
-            const float x1 = load_elem<STORAGE>(buf + static_cast<size_t>(2 * i + 1) * rb, j, sc[2 * i + 1]);
-            const uint64_t xx = f2_pack(x0, x1);
-            if (METRIC == 0) {
-              const uint64_t d = f2_sub(qq, xx);
-              a2[i] = f2_fma(d, d, a2[i]);
-            } else {
-              a2[i] = f2_fma(qq, xx, a2[i]);
-              if (METRIC == 2) l2[i] = f2_fma(xx, xx, l2[i]);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < P; ++i) {
-        f2_unpack(a2[i], acc[2 * i], acc[2 * i + 1]);
-        f2_unpack(l2[i], len[2 * i], len[2 * i + 1]);
-      }
-    }
-    // Row r's sums are in lanes r*(32/H) .. ; candidate first + i takes row i.
-    const float t = butterfly_rows<H>(acc, lane);
-    const float ln = METRIC == 2 ? butterfly_rows<H>(len, lane) : 0.0f;
-    const int src = ((lane - first) & (H - 1)) * (32 / H);
-    const float ts = __shfl_sync(FULL, t, src);
-    const float ls = METRIC == 2 ? __shfl_sync(FULL, ln, src) : 0.0f;
-    if (lane >= first && lane < first + cnt) out = finish_distance<METRIC>(ts, ls);
-    __syncwarp();
-    if (c + 2 < nchunks) issue(c + 2);
-  }
-  return true;
-}
-
-// FP32 distances (reference arithmetic) of up to 4 rows loaded straight from
-// global memory, lane-strided and coalesced; result i in every lane.
-template <int METRIC>
-__device__ __forceinline__ void fp32_distances4(const Params &p, const float *qv,
-                                                const uint32_t ids[4], int cnt, float d[4],
-                                                int lane) {
-  float acc[4], len[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    acc[i] = 0.0f;
-    len[i] = 0.0f;
-  }
-  for (int j = lane; j < p.dim; j += 32) {
-    const float qj = qv[j];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (i < cnt) {
-        const float *row = reinterpret_cast<const float *>(
-            reinterpret_cast<const uint8_t *>(p.rows_f32) + static_cast<uint64_t>(ids[i]) * p.f32_row_bytes);
-        const float xj = __ldg(row + j);
-        if (METRIC == 0) {
-          const float dd = __fsub_rn(qj, xj);
-          acc[i] = __fmaf_rn(dd, dd, acc[i]);
-        } else {
-          acc[i] = __fmaf_rn(qj, xj, acc[i]);
-          if (METRIC == 2) len[i] = __fmaf_rn(xj, xj, len[i]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      acc[i] = __fadd_rn(acc[i], __shfl_xor_sync(FULL, acc[i], o));
-      if (METRIC == 2) len[i] = __fadd_rn(len[i], __shfl_xor_sync(FULL, len[i], o));
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) d[i] = finish_distance<METRIC>(acc[i], len[i]);
-}
-
-__device__ __forceinline__ uint64_t warp_min_u64(uint64_t x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const uint64_t y = __shfl_xor_sync(FULL, x, o);
-    x = y < x ? y : x;
-  }
-  return x;
 }
 
 __device__ __forceinline__ float key_float(uint64_t k) {
@@ -349,27 +382,112 @@ struct VisitedOf<true> {
   }
 };
 
-// The warp's shared-memory slice and barrier phases.
+// From this register-queue segment on (pq >= 16*S), the candidate queue is a
+// BufQueue.  10,000 queries of 1M x 128: pq 150 (S 8) 4.30 ms with a BufQueue,
+// 3.80 with a RegQueue; pq 1000 (S 32) 37.4 ms with a BufQueue, 60 with a
+// RegQueue.
+constexpr int BUF_S = 16;
+
+template <int S>
+struct QueueOf {
+  using type = typename std::conditional<(S >= BUF_S), BufQueue, RegQueue<S>>::type;
+};
+
+// Shared memory of one warp, in this order: the first adjacency row (bulk
+// copy), its barrier, the candidate ids and home slots, the query, the
+// queue's ring, and the visited hash, which the answer's sort reuses (8 bytes
+// for each of 32*S keys).
+struct WarpLayout {
+  uint32_t warp_bytes, off_mbar, off_cand, off_q, off_queue, off_hash;
+};
+inline WarpLayout warp_layout(int dim, int pq, int S, int cap, int cands) {
+  auto up = [](uint32_t x, uint32_t a) { return (x + a - 1) / a * a; };
+  WarpLayout L;
+  L.off_mbar = 128;
+  L.off_cand = L.off_mbar + 16;
+  L.off_q = L.off_cand + 8u * static_cast<uint32_t>(cands);
+  L.off_queue = up(L.off_q + 4u * up(static_cast<uint32_t>(dim), 32), 16);
+  L.off_hash = up(L.off_queue + (S >= BUF_S ? BufQueue::bytes(pq) : 0u), 16);
+  const uint32_t hash = 4u * static_cast<uint32_t>(cap), sort = 256u * static_cast<uint32_t>(S);
+  L.warp_bytes = up(L.off_hash + (hash > sort ? hash : sort), 128);
+  return L;
+}
+
+// The warp's shared-memory slice and barrier phase.
 struct WarpCtx {
-  uint8_t *stage;
+  uint32_t *row;    // first adjacency row
   uint64_t *mbar;
-  uint32_t *cbuf;
+  uint32_t *cbuf;   // candidate ids
+  int32_t *chome;   // and their home slots
   float *qv;
+  uint64_t *ring;
   int32_t *tab;
   const __nv_bfloat16 *wmlp;
-  uint32_t ph0, ph1;
+  uint32_t ph;
+
+  __device__ __forceinline__ void init(uint8_t *ws, const Params &p, int cands, int lane) {
+    row = reinterpret_cast<uint32_t *>(ws);
+    mbar = reinterpret_cast<uint64_t *>(ws + p.off_mbar);
+    cbuf = reinterpret_cast<uint32_t *>(ws + p.off_cand);
+    chome = reinterpret_cast<int32_t *>(cbuf + cands);
+    qv = reinterpret_cast<float *>(ws + p.off_q);
+    ring = reinterpret_cast<uint64_t *>(ws + p.off_queue);
+    tab = reinterpret_cast<int32_t *>(ws + p.off_hash);
+    if (lane == 0) {
+      mbar_init(mbar, 1);
+      fence_mbar_init();
+    }
+    __syncwarp();
+    ph = 0;
+  }
 };
 
 struct QueryStats {
   int hops, evals, version;
 };
 
+// Select-insert (:297-322) of candidates 0..m-1 (key ck, home slot chome in
+// lane c), in candidate order, in two passes.  The queue pass applies the
+// select-insert rule and the insertions and notes, in lane c, the key that
+// candidate c's insertion pushed out (~0: none, the queue was not full).
+// Below pq live keys the queue's maximum is an infinite key, which leaves and
+// is never below a candidate; at pq, the select-insert rule, then the larger
+// of the key and the maximum leaves (:315-320).  The maximum only falls, so
+// after each insertion the candidates beyond it are dropped.  The hash pass
+// then makes the reference's visited-hash calls -- add(candidate),
+// delete(pushed-out key) per inserted candidate.  (Queue and hash are
+// independent, so splitting the passes changes neither.)
+template <class Queue, class VH>
+__device__ __forceinline__ void select_insert(Queue &Q, VH &vh, int m, uint64_t ck, int chome, int pq, int &qn,
+                                              int lane) {
+  uint64_t my_ev = ~0ull;
+  unsigned ins = 0u;
+  uint64_t qmax = Q.max();
+  unsigned live = __ballot_sync(FULL, lane < m && key_dist(ck) <= key_dist(qmax));
+  while (live) {
+    const int c = __ffs(live) - 1;
+    const uint64_t key = __shfl_sync(FULL, ck, c);
+    const uint64_t ev = key < qmax ? qmax : key;
+    Q.insert_evict(key, lane);
+    ins |= 1u << c;
+    if (lane == c) my_ev = ev;
+    if (qn < pq) ++qn;
+    qmax = Q.max();
+    live &= (live - 1u) & __ballot_sync(FULL, key_dist(ck) <= key_dist(qmax));
+  }
+  if (ins) {
+    const bool del = my_ev != ~0ull;
+    const int ehome = del ? vh.slot(key_id(my_ev)) : 0;
+    visited_update(vh, (ins >> lane & 1u) != 0u, key_id(ck), chome, del, key_id(my_ev), ehome, lane);
+  }
+}
+
 // One query: the search of warp_astar_accelerator.h:111-335 with the query
 // vector at qsrc, queue bound pq, k ids written ascending to o.  `trace`
 // (LEARNED) receives the per-hop features or is null.  False if a bulk copy
 // never completed.  MULTI: the reference's N_MULTIPROBE / FINISH_CNT knobs
 // (p.probes, p.finish_cnt) as run-time values.
-template <int METRIC, int STORAGE, int H, int S, bool LEARNED, bool MULTI = false>
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false>
 __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const float *qsrc, const uint32_t *starts,
                                           int ns, int pq, int k, uint64_t *o, float *trace, QueryStats &st,
                                           int lane, const uint32_t *qcode = nullptr) {
@@ -377,53 +495,92 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
 #pragma unroll
   for (int i = 0; i < 8; ++i) qc.w[i] = STORAGE == 3 ? qcode[i] : 0u;
   typename VisitedOf<LEARNED>::type vh = VisitedOf<LEARNED>::make(w.tab, pq);
-  RegQueue<S> Q, T;  // candidate queue and top-pq list, ascending (distance, id)
-  constexpr int C = RegQueue<S>::C;
+  typename QueueOf<S>::type Q;
+  RegQueue<S> TS;  // top-pq list of the learned kernels (they read its k-th key)
+  PopList<S> T;    // and of the others
   const int nslots = 1 << p.shift;
-  for (int j = lane; j < p.dim; j += 32) w.qv[j] = qsrc[j];
-  vh.clear(lane);
+  auto adjacency = [&](uint32_t v) {
+    return lane < nslots ? __ldg(p.adj + (static_cast<uint64_t>(v) << p.shift) + lane) : 0u;
+  };
   // Start vertices: vertex 0 (the reference's), or the ns entry points the
-  // pre-pass chose (lane i holds start i).  Prefetch the first start's row.
+  // pre-pass chose (lane i holds start i).  The first start's adjacency row
+  // is copied while the hash is cleared and the starts are scored.
   if (!starts) ns = 1;
   const uint32_t sid = (starts && lane < ns) ? starts[lane] : 0u;
   uint32_t next_id = __shfl_sync(FULL, sid, 0);
-  uint32_t a_next = lane < nslots ? __ldg(p.adj + (static_cast<uint64_t>(next_id) << p.shift) + lane) : 0u;
+  const bool bulk = p.shift >= 2;  // rows of 16 bytes and more
+  if (bulk) {
+    fence_proxy_async();  // the buffer was last read through the generic proxy
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive_expect_tx(w.mbar, (4u << p.shift) + p.extra_tx);
+      bulk_g2s(w.row, p.adj + (static_cast<uint64_t>(next_id) << p.shift), 4u << p.shift, w.mbar);
+    }
+  }
+  for (int j = lane; j < ((p.dim + 31) & ~31); j += 32) w.qv[j] = j < p.dim ? qsrc[j] : 0.0f;
+  vh.clear(lane);
 
   // warp_astar_accelerator.h:115-176: distances to the starts, queue = {starts}.
-  float cd;
-  if (!gather_distances<METRIC, STORAGE, H>(p, w.stage, w.mbar, w.ph0, w.ph1, w.qv, ns, sid, cd, lane, qc)) {
-    return false;
-  }
+  float cd = gather_distances<METRIC, STORAGE>(p, w.qv, ns, sid, lane, qc);
   const float d0 = __shfl_sync(FULL, cd, 0);
+  uint32_t a_next;
+  if (bulk) {
+    if (!mbar_wait(w.mbar, w.ph, p.wait_limit)) return false;
+    w.ph ^= 1u;
+    a_next = lane < nslots ? w.row[lane] : 0u;
+  } else {
+    a_next = adjacency(next_id);
+  }
   int qn = 0, tn = 0;
-  Q.clear();
-  T.clear();
-  // T holds pq keys at all times: tn real ones (ascending, from position
-  // C - pq) followed by pq - tn "infinite" keys, so every insertion evicts
-  // the window's maximum (an infinite one while tn < pq).
-#pragma unroll
-  for (int j = 0; j < S; ++j) T.v[j] = (lane * S + j) >= C - pq ? ~0ull : 0ull;
-  // Q likewise holds pq keys: qn real ones from position C - pq, then
-  // infinite ones; a pop shifts the window one place left.
-#pragma unroll
-  for (int j = 0; j < S; ++j) Q.v[j] = (lane * S + j) >= C - pq ? ~0ull : 0ull;
+  Q.init(w.ring, pq, lane);
+  if constexpr (LEARNED) TS.init(nullptr, pq, lane);
+  else T.init();
   for (int i = 0; i < ns; ++i) {  // in start order, as the oracle queues them
     const uint32_t id = __shfl_sync(FULL, sid, i);
     Q.insert_evict(make_key(__shfl_sync(FULL, cd, i), id), lane);
     vh.add(id, lane);
   }
   qn = ns;
-  if (ns > 1) {  // the first pop is the nearest start: prefetch its row instead
+  if (ns > 1) {  // the first pop is the nearest start: load its row instead
     const uint32_t mid = key_id(warp_min_u64(lane < ns ? make_key(cd, sid) : ~0ull));
     if (mid != next_id) {
       next_id = mid;
-      a_next = lane < nslots ? __ldg(p.adj + (static_cast<uint64_t>(mid) << p.shift) + lane) : 0u;
+      a_next = adjacency(mid);
     }
   }
   int hops = 0, evals = ns;
   int version = 0;           // number of changes of the top-k set (LEARNED)
   int last_change = 0;       // hop of the latest change (LEARNED)
-  uint64_t kth_key = ~0ull;  // k-th smallest key of T, ~0 while tn < k (LEARNED)
+  uint64_t kth_key = ~0ull;  // k-th smallest key of the list, ~0 while tn < k (LEARNED)
+  uint64_t tmax = 0ull;      // the full list's maximum
+
+  // Moves a popped vertex to the top-pq list (:198-210): a full list drops
+  // its maximum, or the vertex itself when that is above it (which only a
+  // multi-probe pop can be).
+  auto list_insert = [&](uint64_t now, uint32_t now_id, int now_home) {
+    if constexpr (LEARNED) {
+      const uint64_t top = TS.max();
+      const uint64_t ev = now < top ? top : now;
+      TS.insert_evict(now, lane);
+      visited_refresh(vh, now_id, now_home, lane);
+      if (tn < pq) ++tn;
+      else vh.del(key_id(ev), lane);
+      if (tn == pq) tmax = TS.max();
+    } else {
+      visited_refresh(vh, now_id, now_home, lane);
+      if (tn < pq) {
+        ++tn;
+        T.append(now, pq, lane);
+        if (tn == pq) tmax = T.max();
+      } else if (now < tmax) {
+        vh.del(key_id(tmax), lane);
+        T.replace(tmax, now, lane);
+        tmax = T.max();
+      } else {
+        vh.del(now_id, lane);
+      }
+    }
+  };
 
   int finished = 0;  // MULTI: finish tests that held (finished[cid], :190-192)
   while (qn > 0) {
@@ -439,31 +596,26 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
       const int avail = qn;
       for (int kp = 0; kp < p.probes && kp < avail; ++kp) {
         uint64_t qh;
-        const uint64_t now = Q.pop_window(C - pq, lane, &qh);
+        const uint64_t now = Q.pop(lane, &qh);
         --qn;
         const uint32_t now_id = key_id(now);
-        const uint32_t a = (kp == 0 && now_id == next_id)
-                               ? a_next
-                               : (lane < nslots ? __ldg(p.adj + (static_cast<uint64_t>(now_id) << p.shift) + lane) : 0u);
+        const uint32_t a = (kp == 0 && now_id == next_id) ? a_next : adjacency(now_id);
         const int now_home = vh.slot(now_id);
-        vh.del_at(now_id, now_home, lane);
-        if (kp == 0 && tn == pq && key_dist(T.max()) <= key_dist(now) && ++finished >= p.finish_cnt) {
+        if (kp == 0 && tn == pq && key_dist(tmax) <= key_dist(now) && ++finished >= p.finish_cnt) {
           fin = true;
           break;
         }
         ++hops;
-        // :198-210 a later pop can lie above the list maximum; then it is
-        // the key that leaves (add, then delete, as the reference does).
-        const uint64_t tmax = T.max();
-        const uint64_t ev = now < tmax ? tmax : now;
-        T.insert_evict(now, lane);
-        vh.add_at(now_id, now_home, lane);
-        if (tn < pq) ++tn;
-        else vh.del(key_id(ev), lane);
+        list_insert(now, now_id, now_home);
         const int deg = static_cast<int>(__shfl_sync(FULL, a, 0));
-        const bool fresh = lane >= 1 && lane <= deg && !vh.test(a);
+        const int ahome = vh.slot(a);
+        const bool fresh = lane >= 1 && lane <= deg && !vh.test_at(a, ahome);
         const unsigned fm = __ballot_sync(FULL, fresh);
-        if (fresh) w.cbuf[m + __popc(fm & lanemask_lt())] = a;
+        if (fresh) {
+          const int at = m + __popc(fm & lanemask_lt());
+          w.cbuf[at] = a;
+          w.chome[at] = ahome;
+        }
         m += __popc(fm);
       }
       if (fin) break;
@@ -474,11 +626,10 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
       for (int r0 = 0; r0 < m; r0 += 32) {
         const int mr = min(32, m - r0);
         const uint32_t cid = lane < mr ? w.cbuf[r0 + lane] : 0u;
-        if (!gather_distances<METRIC, STORAGE, H>(p, w.stage, w.mbar, w.ph0, w.ph1, w.qv, mr, cid, cd, lane, qc))
-          return false;
+        const int chome = lane < mr ? w.chome[r0 + lane] : 0;
+        cd = gather_distances<METRIC, STORAGE>(p, w.qv, mr, cid, lane, qc);
         evals += mr;
         const uint64_t ck = lane < mr ? make_key(cd, cid) : ~0ull;
-        const int chome = vh.slot(cid);
         if (p.double_check) {
           // :297-322 with :307-310: a candidate already in the visited hash
           // (listed by an earlier pop of this iteration, or twice in one row)
@@ -488,89 +639,62 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
             const uint64_t qmax = Q.max();
             if (key_dist(qmax) < key_dist(key)) continue;
             const uint32_t id = key_id(key);
-            if (vh.test(id)) continue;
+            const int home = __shfl_sync(FULL, chome, c);
+            if (vh.test_at(id, home)) continue;
             const uint64_t ev = key < qmax ? qmax : key;
             Q.insert_evict(key, lane);
             if (qn < pq) ++qn;
-            vh.add_at(id, __shfl_sync(FULL, chome, c), lane);
+            vh.add_at(id, home, lane);
             if (ev != ~0ull) vh.del(key_id(ev), lane);
           }
           __syncwarp();
           continue;
         }
-        uint64_t my_ev = ~0ull;
-        unsigned ins = 0u;
-        for (int c = 0; c < mr; ++c) {
-          const uint64_t key = __shfl_sync(FULL, ck, c);
-          const uint64_t qmax = Q.max();
-          if (key_dist(qmax) < key_dist(key)) continue;
-          const uint64_t ev = key < qmax ? qmax : key;
-          Q.insert_evict(key, lane);
-          ins |= 1u << c;
-          if (lane == c) my_ev = ev;
-          if (qn < pq) ++qn;
-        }
-        if (ins) {
-          const int ehome = my_ev != ~0ull ? vh.slot(key_id(my_ev)) : 0;
-          do {
-            const int c = __ffs(ins) - 1;
-            ins &= ins - 1u;
-            vh.add_at(__shfl_sync(FULL, cid, c), __shfl_sync(FULL, chome, c), lane);
-            const uint64_t ev = __shfl_sync(FULL, my_ev, c);
-            if (ev != ~0ull) vh.del_at(key_id(ev), __shfl_sync(FULL, ehome, c), lane);
-          } while (ins);
-        }
-        __syncwarp();
+        select_insert(Q, vh, mr, ck, chome, pq, qn, lane);
       }
       // the next iteration's first pop is the queue head: load its row now
       if (qn > 0) {
-        next_id = key_id(Q.at(C - pq, lane));
-        a_next = lane < nslots ? __ldg(p.adj + (static_cast<uint64_t>(next_id) << p.shift) + lane) : 0u;
+        next_id = key_id(Q.min());
+        a_next = adjacency(next_id);
       }
       continue;
     }
     // :186-193 pop the minimum, drop it from the visited hash.
     uint64_t qh;  // queue minimum after the pop
-    const uint64_t now = Q.pop_window(C - pq, lane, &qh);
+    const uint64_t now = Q.pop(lane, &qh);
     --qn;
     const uint32_t now_id = key_id(now);
     uint32_t a = a_next;
-    if (now_id != next_id)  // not taken: the prefetch predicts the pop exactly
-      a = lane < nslots ? __ldg(p.adj + (static_cast<uint64_t>(now_id) << p.shift) + lane) : 0u;
-    const int now_home = vh.slot(now_id);
-    vh.del_at(now_id, now_home, lane);
+    if (now_id != next_id) a = adjacency(now_id);  // not taken: the prefetch predicts the pop exactly
     // :191 finish test (<=) against the list maximum.
-    if (tn == pq && key_dist(T.max()) <= key_dist(now)) break;
+    if (tn == pq && key_dist(tmax) <= key_dist(now)) break;
     ++hops;
     // LEARNED: does `now` enter the current top-k?  (Only such an entry
-    // changes the k-th key: T drops its maximum, never a top-k key.)
+    // changes the k-th key: the list drops its maximum, never a top-k key.)
     const bool enters = LEARNED && now < kth_key;
     if (enters) {
       ++version;
       last_change = hops;
     }
-    // :198-210 move it to the top-pq list (when full, `now` is below the
-    // list maximum, which is the one dropped).
-    {
-      const uint64_t ev = T.max();
-      T.insert_evict(now, lane);
-      vh.add_at(now_id, now_home, lane);
-      if (tn < pq) ++tn;
-      else vh.del(key_id(ev), lane);
-    }
-    if (enters && tn >= k) kth_key = T.at(C - pq + k - 1, lane);
+    list_insert(now, now_id, vh.slot(now_id));
+    if constexpr (LEARNED)
+      if (enters && tn >= k) kth_key = TS.at(TS.start + k - 1);
     // :211-224 neighbours not in the visited hash, in row order.
     const int deg = static_cast<int>(__shfl_sync(FULL, a, 0));
-    const bool isnb = lane >= 1 && lane <= deg;
-    const bool fresh = isnb && !vh.test(a);
+    const int ahome = vh.slot(a);
+    const bool fresh = lane >= 1 && lane <= deg && !vh.test_at(a, ahome);
     const unsigned fm = __ballot_sync(FULL, fresh);
     const int m = __popc(fm);
-    if (fresh) w.cbuf[__popc(fm & lanemask_lt())] = a;
+    if (fresh) {
+      const int at = __popc(fm & lanemask_lt());
+      w.cbuf[at] = a;
+      w.chome[at] = ahome;
+    }
     __syncwarp();
     const uint32_t cid = lane < m ? w.cbuf[lane] : 0u;
+    const int chome = lane < m ? w.chome[lane] : 0;
     // :237-287 distances.
-    if (!gather_distances<METRIC, STORAGE, H>(p, w.stage, w.mbar, w.ph0, w.ph1, w.qv, m, cid, cd, lane, qc))
-      return false;
+    cd = gather_distances<METRIC, STORAGE>(p, w.qv, m, cid, lane, qc);
     evals += m;
     // The next vertex popped is the smaller of the queue head and the best
     // candidate (the select-insert rule can only reject candidates above a
@@ -581,43 +705,10 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
     const uint64_t nk = cmin < qh ? cmin : qh;
     if (nk != ~0ull) {
       next_id = key_id(nk);
-      a_next = lane < nslots ? __ldg(p.adj + (static_cast<uint64_t>(next_id) << p.shift) + lane) : 0u;
+      a_next = adjacency(next_id);
     }
-    // :297-322 select-insert in candidate order, in two passes.  The queue
-    // pass applies the select-insert rule and the insertions and notes, in
-    // lane c, the key candidate c's insertion pushed out (~0: none, the
-    // queue was not full).  Below pq live keys the window's maximum is an
-    // infinite key, which leaves and is never below a candidate; at pq, the
-    // select-insert rule, then the larger of the key and the maximum leaves
-    // (:315-320).  The hash pass then makes the reference's visited-hash
-    // calls in the reference's order -- add(candidate), delete(pushed-out
-    // key) per inserted candidate -- with every home slot computed up front,
-    // one lane per key.  (Queue and hash are independent, so splitting the
-    // passes changes neither.)
-    const int chome = vh.slot(cid);
-    uint64_t my_ev = ~0ull;
-    unsigned ins = 0u;
-    for (int c = 0; c < m; ++c) {
-      const uint64_t key = __shfl_sync(FULL, ck, c);
-      const uint64_t qmax = Q.max();
-      if (key_dist(qmax) < key_dist(key)) continue;
-      const uint64_t ev = key < qmax ? qmax : key;
-      Q.insert_evict(key, lane);
-      ins |= 1u << c;
-      if (lane == c) my_ev = ev;
-      if (qn < pq) ++qn;
-    }
-    if (ins) {
-      const int ehome = my_ev != ~0ull ? vh.slot(key_id(my_ev)) : 0;
-      do {
-        const int c = __ffs(ins) - 1;
-        ins &= ins - 1u;
-        vh.add_at(__shfl_sync(FULL, cid, c), __shfl_sync(FULL, chome, c), lane);
-        const uint64_t ev = __shfl_sync(FULL, my_ev, c);
-        if (ev != ~0ull) vh.del_at(key_id(ev), __shfl_sync(FULL, ehome, c), lane);
-      } while (ins);
-    }
-    if (LEARNED) {
+    select_insert(Q, vh, m, ck, chome, pq, qn, lane);
+    if constexpr (LEARNED) {
       const bool check = p.mlp && hops >= p.exit_min_hops && (hops % p.exit_every) == 0 && tn >= k;
       if (trace || check) {
       // Per-hop state: hop count, k-th and best distance, queue-head gap,
@@ -625,8 +716,8 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
       // enter through scale-free, bounded quantities: the top-k spread and
       // the queue-head gap relative to the progress span d0 - best (signed
       // logs).
-      const float kth = key_float(tn >= k ? kth_key : T.at(C - pq + tn - 1, lane));
-      const float best = key_float(T.at(C - pq, lane));
+      const float kth = key_float(tn >= k ? kth_key : TS.at(TS.start + tn - 1));
+      const float best = key_float(TS.min());
       const float head = nk != ~0ull ? key_float(nk) : kth;
       const float span = fabsf(d0 - best) + 1e-6f * (fabsf(d0) + fabsf(best)) + 1e-30f;
       const float r1 = (kth - best) / span;
@@ -649,69 +740,71 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
     }
   }
 
+  // :331-335 the list's first k ids, ascending; slots past its length get
+  // UINT64_MAX.  The keys are sorted where the visited hash was.
+  uint64_t *keys = reinterpret_cast<uint64_t *>(w.tab);
+  int live = tn;  // keys that can be returned
+  __syncwarp();
+  if constexpr (LEARNED) {
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const int r = lane * S + j - TS.start;
+      if (r >= 0) keys[r] = r < tn ? TS.v[j] : ~0ull;
+    }
+    for (int i = pq + lane; i < 32 * S; i += 32) keys[i] = ~0ull;
+  } else {
+    T.dump(keys, pq, lane);
+  }
+  __syncwarp();
   if (STORAGE != 0 && p.rerank > 0) {
     // FP32 re-rank of the best `rerank` entries of the list, then the first k.
     const int R = min(max(p.rerank, k), tn);
-    int rn = 0;
-    Q.clear();
-    for (int base = 0; base < R; base += 4) {
-      uint32_t ids[4];
-      const int cnt = min(4, R - base);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ids[i] = i < cnt ? key_id(T.at(C - pq + base + i, lane)) : 0u;
-      float d[4];
-      fp32_distances4<METRIC>(p, w.qv, ids, cnt, d, lane);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (i < cnt) {
-          Q.insert_grow(make_key(d[i], ids[i]), lane);
-          ++rn;
-        }
+    if (!LEARNED && R < tn) warp_sort_shared(keys, 32 * S, lane);
+    for (int base = 0; base < R; base += 32) {
+      const int cnt = min(32, R - base);
+      const uint32_t id = lane < cnt ? key_id(keys[base + lane]) : 0u;
+      const float d = gather_rows<METRIC, 0>(reinterpret_cast<const uint8_t *>(p.rows_f32), p.f32_row_bytes, 0u,
+                                             static_cast<int>(p.f32_row_bytes >> 2), w.qv, cnt, id, lane);
+      if (lane < cnt) keys[base + lane] = make_key(d, id);
     }
-#pragma unroll
-    for (int j = 0; j < S; ++j) {
-      const int r = Q.rank_of(j, rn, lane);
-      if (r >= 0 && r < k) o[r] = static_cast<uint64_t>(key_id(Q.v[j]));
-    }
-    for (int i = rn + lane; i < k; i += 32) o[i] = ~0ull;
-  } else {
-    // :331-335 ascending ids; slots past the list length get UINT64_MAX.
-#pragma unroll
-    for (int j = 0; j < S; ++j) {
-      const int r = T.rank_of(j, pq, lane);
-      if (r >= 0 && r < k && r < tn) o[r] = static_cast<uint64_t>(key_id(T.v[j]));
-    }
-    for (int i = tn + lane; i < k; i += 32) o[i] = ~0ull;
+    for (int i = R + lane; i < 32 * S; i += 32) keys[i] = ~0ull;
+    live = R;
+    __syncwarp();
   }
+  if (k <= 32) {
+    const uint64_t key = warp_smallest32(keys, 32 * S, lane);
+    if (lane < k) o[lane] = lane < live ? static_cast<uint64_t>(key_id(key)) : ~0ull;
+  } else {
+    warp_sort_shared(keys, 32 * S, lane);
+    for (int i = lane; i < k; i += 32) o[i] = i < live ? static_cast<uint64_t>(key_id(keys[i])) : ~0ull;
+  }
+  __syncwarp();
   st.hops = hops;
   st.evals = evals;
   st.version = version;
   return true;
 }
 
-// Small queues (S <= 4, pq < 128) ask for six resident blocks (24 warps per
-// SM, at most 80 registers; the per-warp shared memory of such pq fits).
-// Measured on the headline search: 5 -> 6 blocks 10 % faster; 8 blocks (64
-// registers) 3 % slower than 6.
-template <int METRIC, int STORAGE, int S, bool LEARNED>
+// Resident blocks of four warps asked for: 5 while the queues are small (S <=
+// 4: 96 registers; 6 blocks, at 80, cost 25 % of a
+// small batch's time, 1000 queries of 1M x 128 from entry points at pq 43 287
+// -> 362 us, for 1 % of a full one's), 4 for the wider register queue of S = 8
+// and the lists of S = 16, 2 beyond, where shared memory holds eight warps at
+// most.
+template <int S>
 struct MinBlocks {
-  static constexpr int value = S > 4 ? 1 : 6;
+  static constexpr int value = S > 16 ? 2 : (S > 4 ? 4 : 5);
 };
 
-template <int METRIC, int STORAGE, int H, int S, bool LEARNED, bool MULTI = false>
-__global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, (MinBlocks<METRIC, STORAGE, S, LEARNED>::value))
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false>
+__global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, MinBlocks<S>::value)
     search_kernel(const Params p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
-  uint8_t *ws = smem_raw + static_cast<size_t>(wib) * p.warp_bytes;
   WarpCtx w;
-  w.stage = ws;
-  w.mbar = reinterpret_cast<uint64_t *>(ws + p.off_mbar);
-  w.cbuf = reinterpret_cast<uint32_t *>(ws + p.off_cand);
-  w.qv = reinterpret_cast<float *>(ws + p.off_q);
-  w.tab = reinterpret_cast<int32_t *>(ws + p.off_hash);
+  w.init(smem_raw + static_cast<size_t>(wib) * p.warp_bytes, p, (MULTI ? MAX_PROBES : 1) * 32, lane);
   __nv_bfloat16 *wmlp = reinterpret_cast<__nv_bfloat16 *>(smem_raw + static_cast<size_t>(nwarps) * p.warp_bytes);
   w.wmlp = wmlp;
   if (LEARNED) {
@@ -719,14 +812,6 @@ __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, (MinBlocks<METRIC, S
       for (int i = threadIdx.x; i < MLP_NPARAM; i += blockDim.x) wmlp[i] = p.mlp[i];
     __syncthreads();
   }
-  if (lane == 0) {
-    mbar_init(&w.mbar[0], 1);
-    mbar_init(&w.mbar[1], 1);
-    fence_mbar_init();
-  }
-  __syncwarp();
-  w.ph0 = 0;
-  w.ph1 = 0;
 
   for (;;) {
     uint32_t qid = 0;
@@ -736,7 +821,7 @@ __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, (MinBlocks<METRIC, S
     float *trace = nullptr;
     if (LEARNED && p.trace) trace = p.trace + static_cast<size_t>(qid) * p.trace_hops * TRACE_FIELDS;
     QueryStats st;
-    if (!run_query<METRIC, STORAGE, H, S, LEARNED, MULTI>(p, w, p.queries + static_cast<size_t>(qid) * p.dim,
+    if (!run_query<METRIC, STORAGE, S, LEARNED, MULTI>(p, w, p.queries + static_cast<size_t>(qid) * p.dim,
                                                    p.starts ? p.starts + static_cast<size_t>(qid) * p.n_starts
                                                             : nullptr,
                                                    p.n_starts, p.pq,
@@ -766,9 +851,9 @@ __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, (MinBlocks<METRIC, S
 // that keeps the most warps resident per SM (search.cu).
 int get_shape(const void *fn, uint32_t warp_bytes, uint32_t extra_bytes, int *wpb, int *grid_cap);
 
-template <int METRIC, int STORAGE, int H, int S, bool LEARNED, bool MULTI = false>
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false>
 int launch_kernel(const Params &p, cudaStream_t stream) {
-  auto kern = search_kernel<METRIC, STORAGE, H, S, LEARNED, MULTI>;
+  auto kern = search_kernel<METRIC, STORAGE, S, LEARNED, MULTI>;
   const uint32_t extra = LEARNED ? static_cast<uint32_t>(MLP_NPARAM * sizeof(__nv_bfloat16) + 64) : 0u;
   int wpb = 0, cap = 0;
   int e = get_shape(reinterpret_cast<const void *>(kern), p.warp_bytes, extra, &wpb, &cap);
@@ -781,44 +866,36 @@ int launch_kernel(const Params &p, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-template <int METRIC, int STORAGE, int H, bool LEARNED, bool MULTI = false>
+template <int STORAGE, int METRIC, bool LEARNED, bool MULTI = false>
 int launch_by_s(const Params &p, int S, cudaStream_t s) {
   switch (S) {
-    case 1: return launch_kernel<METRIC, STORAGE, H, 1, LEARNED, MULTI>(p, s);
-    case 2: return launch_kernel<METRIC, STORAGE, H, 2, LEARNED, MULTI>(p, s);
-    case 4: return launch_kernel<METRIC, STORAGE, H, 4, LEARNED, MULTI>(p, s);
-    case 8: return launch_kernel<METRIC, STORAGE, H, 8, LEARNED, MULTI>(p, s);
-    case 16: return launch_kernel<METRIC, STORAGE, H, 16, LEARNED, MULTI>(p, s);
-    case 32: return launch_kernel<METRIC, STORAGE, H, 32, LEARNED, MULTI>(p, s);
+    case 1: return launch_kernel<METRIC, STORAGE, 1, LEARNED, MULTI>(p, s);
+    case 2: return launch_kernel<METRIC, STORAGE, 2, LEARNED, MULTI>(p, s);
+    case 4: return launch_kernel<METRIC, STORAGE, 4, LEARNED, MULTI>(p, s);
+    case 8: return launch_kernel<METRIC, STORAGE, 8, LEARNED, MULTI>(p, s);
+    case 16: return launch_kernel<METRIC, STORAGE, 16, LEARNED, MULTI>(p, s);
+    case 32: return launch_kernel<METRIC, STORAGE, 32, LEARNED, MULTI>(p, s);
     default: return -1;
   }
 }
 
 template <int STORAGE, bool LEARNED, bool MULTI = false>
-int launch_storage(const Params &p, int metric, int H, int S, cudaStream_t s) {
-  const int h = H == 1 ? 0 : (H == 2 ? 1 : (H == 4 ? 2 : -1));
-  if (h < 0) return -1;
-  switch (metric * 3 + h) {
-    case 0: return launch_by_s<0, STORAGE, 1, LEARNED, MULTI>(p, S, s);
-    case 1: return launch_by_s<0, STORAGE, 2, LEARNED, MULTI>(p, S, s);
-    case 2: return launch_by_s<0, STORAGE, 4, LEARNED, MULTI>(p, S, s);
-    case 3: return launch_by_s<1, STORAGE, 1, LEARNED, MULTI>(p, S, s);
-    case 4: return launch_by_s<1, STORAGE, 2, LEARNED, MULTI>(p, S, s);
-    case 5: return launch_by_s<1, STORAGE, 4, LEARNED, MULTI>(p, S, s);
-    case 6: return launch_by_s<2, STORAGE, 1, LEARNED, MULTI>(p, S, s);
-    case 7: return launch_by_s<2, STORAGE, 2, LEARNED, MULTI>(p, S, s);
-    case 8: return launch_by_s<2, STORAGE, 4, LEARNED, MULTI>(p, S, s);
+int launch_storage(const Params &p, int metric, int S, cudaStream_t s) {
+  switch (metric) {
+    case 0: return launch_by_s<STORAGE, 0, LEARNED, MULTI>(p, S, s);
+    case 1: return launch_by_s<STORAGE, 1, LEARNED, MULTI>(p, S, s);
+    case 2: return launch_by_s<STORAGE, 2, LEARNED, MULTI>(p, S, s);
     default: return -1;
   }
 }
 
 // One per translation unit (search_f32.cu, search_bf16.cu, search_fp8.cu,
 // search_bits.cu, search_learned.cu, search_multi.cu).
-int launch_f32(const Params &p, int metric, int H, int S, cudaStream_t s);
-int launch_bf16(const Params &p, int metric, int H, int S, cudaStream_t s);
-int launch_fp8(const Params &p, int metric, int H, int S, cudaStream_t s);
+int launch_f32(const Params &p, int metric, int S, cudaStream_t s);
+int launch_bf16(const Params &p, int metric, int S, cudaStream_t s);
+int launch_fp8(const Params &p, int metric, int S, cudaStream_t s);
 int launch_bits(const Params &p, int metric, int S, cudaStream_t s);
-int launch_learned(const Params &p, int storage, int metric, int H, int S, cudaStream_t s);
-int launch_multi(const Params &p, int metric, int H, int S, cudaStream_t s);
+int launch_learned(const Params &p, int storage, int metric, int S, cudaStream_t s);
+int launch_multi(const Params &p, int metric, int S, cudaStream_t s);
 
 }  // namespace song

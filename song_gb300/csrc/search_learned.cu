@@ -3,9 +3,9 @@
 #include "search_kernel.cuh"
 
 namespace song {
-int launch_learned(const Params &p, int storage, int metric, int H, int S, cudaStream_t s) {
-  if (storage == 0) return launch_storage<0, true>(p, metric, H, S, s);
-  if (storage == 1) return launch_storage<1, true>(p, metric, H, S, s);
+int launch_learned(const Params &p, int storage, int metric, int S, cudaStream_t s) {
+  if (storage == 0) return launch_storage<0, true>(p, metric, S, s);
+  if (storage == 1) return launch_storage<1, true>(p, metric, S, s);
   return -1;
 }
 }  // namespace song

@@ -4,7 +4,7 @@
 #include "search_kernel.cuh"
 
 namespace song {
-int launch_multi(const Params &p, int metric, int H, int S, cudaStream_t s) {
-  return launch_storage<0, false, true>(p, metric, H, S, s);
+int launch_multi(const Params &p, int metric, int S, cudaStream_t s) {
+  return launch_storage<0, false, true>(p, metric, S, s);
 }
 }  // namespace song

@@ -21,6 +21,7 @@
 // published, so an exiting warp never holds unprocessed work.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cstdint>
@@ -122,29 +123,16 @@ __device__ __forceinline__ void serve_choose_starts(const Params &p, const float
   __syncwarp();
 }
 
-template <int METRIC, int STORAGE, int H, int S>
+template <int METRIC, int STORAGE, int S>
 __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, 1)
     serve_kernel(const Params p, const ServeEntry *ring, uint32_t ring_mask, const ServeCtl *ctl,
                  uint32_t *next, uint32_t *done, uint32_t idle_polls) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
-  uint8_t *ws = smem_raw + static_cast<size_t>(wib) * p.warp_bytes;
   WarpCtx w;
-  w.stage = ws;
-  w.mbar = reinterpret_cast<uint64_t *>(ws + p.off_mbar);
-  w.cbuf = reinterpret_cast<uint32_t *>(ws + p.off_cand);
-  w.qv = reinterpret_cast<float *>(ws + p.off_q);
-  w.tab = reinterpret_cast<int32_t *>(ws + p.off_hash);
+  w.init(smem_raw + static_cast<size_t>(wib) * p.warp_bytes, p, 32, lane);
   w.wmlp = nullptr;
-  if (lane == 0) {
-    mbar_init(&w.mbar[0], 1);
-    mbar_init(&w.mbar[1], 1);
-    fence_mbar_init();
-  }
-  __syncwarp();
-  w.ph0 = 0;
-  w.ph1 = 0;
   for (;;) {
     uint32_t idx = 0;
     int state = 0;  // 1 claimed, 2 closing, 3 idle
@@ -185,7 +173,7 @@ __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, 1)
       serve_choose_starts<METRIC>(p, w.qv, w.cbuf, lane);
       starts = w.cbuf;
     }
-    if (!run_query<METRIC, STORAGE, H, S, false>(p, w, reinterpret_cast<const float *>(e.query), starts,
+    if (!run_query<METRIC, STORAGE, S, false>(p, w, reinterpret_cast<const float *>(e.query), starts,
                                                  p.n_starts, e.pq, e.k,
                                                  reinterpret_cast<uint64_t *>(e.out), nullptr, st, lane)) {
       if (lane == 0) atomicOr(p.error, 1);
@@ -205,10 +193,10 @@ int queue_segment(int pq) {
 
 uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
-template <int METRIC, int STORAGE, int H, int S>
+template <int METRIC, int STORAGE, int S>
 cudaError_t launch_serve(const Params &p, const ServeEntry *ring, uint32_t mask, const ServeCtl *ctl,
                          uint32_t *next, uint32_t *done, float fraction, uint32_t idle, cudaStream_t s) {
-  auto kern = serve_kernel<METRIC, STORAGE, H, S>;
+  auto kern = serve_kernel<METRIC, STORAGE, S>;
   int wpb = 0, cap = 0;
   int e = get_shape(reinterpret_cast<const void *>(kern), p.warp_bytes, 0u, &wpb, &cap);
   if (e != 0) return e == -1 ? cudaErrorInvalidConfiguration : static_cast<cudaError_t>(e);
@@ -219,29 +207,27 @@ cudaError_t launch_serve(const Params &p, const ServeEntry *ring, uint32_t mask,
   return cudaGetLastError();
 }
 
-template <int METRIC, int H>
+// The kernel's queue segment for a server of this largest pq.
+int serve_segment(int max_pq) { return std::max(4, queue_segment(max_pq)); }
+
+template <int METRIC>
 cudaError_t launch_serve_s(int S, const Params &p, const ServeEntry *ring, uint32_t mask, const ServeCtl *ctl,
                            uint32_t *next, uint32_t *done, float f, uint32_t idle, cudaStream_t s) {
   switch (S) {
-    case 1:
-    case 2:
-    case 4: return launch_serve<METRIC, 0, H, 4>(p, ring, mask, ctl, next, done, f, idle, s);
-    case 8: return launch_serve<METRIC, 0, H, 8>(p, ring, mask, ctl, next, done, f, idle, s);
-    case 16: return launch_serve<METRIC, 0, H, 16>(p, ring, mask, ctl, next, done, f, idle, s);
-    default: return launch_serve<METRIC, 0, H, 32>(p, ring, mask, ctl, next, done, f, idle, s);
+    case 4: return launch_serve<METRIC, 0, 4>(p, ring, mask, ctl, next, done, f, idle, s);
+    case 8: return launch_serve<METRIC, 0, 8>(p, ring, mask, ctl, next, done, f, idle, s);
+    case 16: return launch_serve<METRIC, 0, 16>(p, ring, mask, ctl, next, done, f, idle, s);
+    default: return launch_serve<METRIC, 0, 32>(p, ring, mask, ctl, next, done, f, idle, s);
   }
 }
 
-cudaError_t launch_serve_any(int metric, int H, int S, const Params &p, const ServeEntry *ring, uint32_t mask,
+cudaError_t launch_serve_any(int metric, int S, const Params &p, const ServeEntry *ring, uint32_t mask,
                              const ServeCtl *ctl, uint32_t *next, uint32_t *done, float f, uint32_t idle,
                              cudaStream_t s) {
-  switch (metric * 2 + (H == 4 ? 1 : 0)) {
-    case 0: return launch_serve_s<0, 2>(S, p, ring, mask, ctl, next, done, f, idle, s);
-    case 1: return launch_serve_s<0, 4>(S, p, ring, mask, ctl, next, done, f, idle, s);
-    case 2: return launch_serve_s<1, 2>(S, p, ring, mask, ctl, next, done, f, idle, s);
-    case 3: return launch_serve_s<1, 4>(S, p, ring, mask, ctl, next, done, f, idle, s);
-    case 4: return launch_serve_s<2, 2>(S, p, ring, mask, ctl, next, done, f, idle, s);
-    default: return launch_serve_s<2, 4>(S, p, ring, mask, ctl, next, done, f, idle, s);
+  switch (metric) {
+    case 0: return launch_serve_s<0>(S, p, ring, mask, ctl, next, done, f, idle, s);
+    case 1: return launch_serve_s<1>(S, p, ring, mask, ctl, next, done, f, idle, s);
+    default: return launch_serve_s<2>(S, p, ring, mask, ctl, next, done, f, idle, s);
   }
 }
 
@@ -261,7 +247,7 @@ struct song_server {
     std::vector<float> queries;
   };
   song_index *ix = nullptr;
-  int max_pq = 0, max_k = 0, nslots = 0, slot_queries = 0, S = 0, H = 0;
+  int max_pq = 0, max_k = 0, nslots = 0, slot_queries = 0, S = 0;
   float fraction = 1.0f;
   cudaStream_t stream = nullptr;
   song::Params params{};
@@ -303,7 +289,7 @@ int relaunch_if_idle(song_server *s) {
   }
   // Every warp has left and none holds a claim, so the claim counter already
   // counts exactly the processed entries: the new launch continues from it.
-  cudaError_t e = song::launch_serve_any(s->ix->dx.metric, s->H, s->S, s->params, s->d_ring, s->ring_mask, s->d_ctl,
+  cudaError_t e = song::launch_serve_any(s->ix->dx.metric, s->S, s->params, s->d_ring, s->ring_mask, s->d_ctl,
                                          s->d_next, s->d_done, s->fraction, s->idle_polls, s->stream);
   if (e != cudaSuccess) return fail(SONG_ERR_CUDA, "serve launch: %s", cudaGetErrorString(e));
   s->running = true;
@@ -408,8 +394,7 @@ int song_server_create(song_index *ix, int max_pq, int max_k, int nslots, int sl
   std::memset(s->h_ctl, 0, sizeof(song::ServeCtl));
   std::memset(s->h_done, 0, sizeof(uint32_t) * nslots);
   // kernel parameters: the search layout for the largest pq
-  s->S = song::queue_segment(max_pq);
-  s->H = dx.row_bytes <= 1024 ? 4 : 2;
+  s->S = song::serve_segment(max_pq);
   song::Params &p = s->params;
   std::memset(&p, 0, sizeof p);
   p.rows = static_cast<const uint8_t *>(dx.rows);
@@ -440,19 +425,19 @@ int song_server_create(song_index *ix, int max_pq, int max_k, int nslots, int sl
     ++ix->servers;
     s->holds_entries = true;
   }
-  uint32_t off = 2u * s->H * dx.row_bytes;
-  off = song::align_up(off, 16);
-  p.off_mbar = off;
-  off += 16;
-  p.off_cand = off;
-  off += 32 * 4;
-  off = song::align_up(off, 16);
-  p.off_q = off;
-  off += song::align_up(static_cast<uint32_t>(dim) * 4u, 16);
-  p.off_hash = off;
-  off += 4u * 8u * static_cast<uint32_t>(max_pq);
-  p.warp_bytes = song::align_up(off, 128);
-  if (p.warp_bytes > 227u * 1024u) {
+  const song::WarpLayout L = song::warp_layout(dim, max_pq, s->S, 8 * max_pq, 32);
+  p.off_mbar = L.off_mbar;
+  p.off_cand = L.off_cand;
+  p.off_q = L.off_q;
+  p.off_queue = L.off_queue;
+  p.off_hash = L.off_hash;
+  p.warp_bytes = L.warp_bytes;
+  p.width = dx.dpad;
+  // the interface's limit: two staging chunks of the rows beside the query
+  // and the hash (the kernel needs less)
+  const uint32_t limit = song::align_up(2u * (dx.row_bytes <= 1024 ? 4u : 2u) * dx.row_bytes, 16) + 16 + 32 * 4 +
+                         song::align_up(static_cast<uint32_t>(dim) * 4u, 16) + 32u * static_cast<uint32_t>(max_pq);
+  if (song::align_up(limit, 128) > 227u * 1024u) {
     song_server_destroy(s);
     return fail(SONG_ERR_ARG, "max_pq %d with dim %d does not fit a warp's shared memory", max_pq, dim);
   }

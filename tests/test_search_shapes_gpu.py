@@ -1,0 +1,67 @@
+"""The search kernel at the sizes where its structures change: queue bounds at
+the ends of each queue segment and of the two queue kinds, row widths at the
+remainders of the gather (every format), and ids laid out so that the visited
+hash has long runs (consecutive ids hash to neighbouring slots) across its
+end.  Bit-exact against the oracle (ids, hops, evaluations)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _clustered(n, dim, seed, nq=24):
+    """Vectors sorted along a curve, so that neighbours have neighbouring ids."""
+    rng = np.random.default_rng(seed)
+    t = np.sort(rng.uniform(0, 40, n))
+    q = rng.uniform(0, 40, nq)
+    phase, freq = rng.uniform(0, 6, dim), rng.uniform(0.2, 1.0, dim)
+
+    def at(u):
+        return np.sin(u[:, None] * freq + phase) + 0.3
+    return ((at(t) + 0.05 * rng.standard_normal((n, dim))).astype(np.float32),
+            (at(q) + 0.05 * rng.standard_normal((nq, dim))).astype(np.float32))
+
+
+def _ring_graph(song, data, metric, shift, seed):
+    """Built rows with some long-range neighbours in their last places."""
+    fixed = (1 << shift) - 1
+    g = song.graph_build(data, metric, shift, max(1, fixed // 2), fixed, 60, batch_div=16).reshape(len(data), -1)
+    rng = np.random.default_rng(seed)
+    deg = g[:, 0].astype(int)
+    for v in np.nonzero(deg > 2)[0]:
+        g[v, deg[v]] = rng.integers(len(data))
+    return g
+
+
+PQS = [2, 3, 30, 31, 32, 62, 63, 64, 126, 127, 128, 254, 255, 256, 510, 511, 512, 1022, 1023]
+
+
+@pytest.mark.parametrize("metric", [0, 1, 2])
+@pytest.mark.parametrize("shift", [1, 3, 5])
+def test_queue_bounds(song, oracle, metric, shift):
+    data, q = _clustered(2500, 16, seed=shift)
+    g = _ring_graph(song, data, metric, shift, seed=shift)
+    ox = oracle.OracleIndex(data, g, shift, metric)
+    with song.Index(g, data, shift, metric) as ix:
+        for pq in PQS:
+            ids, hops, evals = ix.search(q, pq, pq, stats=True)
+            o_ids, o_hops, o_evals, _ = ox.kernel_search(q, pq, oracle.MODE_LEX)
+            assert np.array_equal(ids, o_ids), "pq %d" % pq
+            assert np.array_equal(hops, o_hops) and np.array_equal(evals, o_evals), "pq %d" % pq
+            for k in (1, min(pq, 32), min(pq, 33)):
+                assert np.array_equal(ix.search(q, pq, k), o_ids[:, :k]), "pq %d k %d" % (pq, k)
+
+
+@pytest.mark.parametrize("dim", [1, 4, 5, 31, 32, 33, 63, 124, 127, 128, 129, 200, 255, 256, 260, 500])
+def test_row_widths(song, oracle, dim):
+    data, q = _clustered(900, dim, seed=dim)
+    for metric in (0, 1, 2):
+        g = _ring_graph(song, data, metric, 5, seed=dim)
+        for storage in ("f32", "bf16", "fp8"):
+            with song.Index(g, data, 5, metric, storage=storage) as ix:
+                ix.set_rerank(0)
+                ids, hops, evals = ix.search(q, 40, 40, stats=True)
+                ox = oracle.OracleIndex(song.dequantize_rows(ix.rows(), storage, dim), g, 5, metric)
+                o_ids, o_hops, o_evals, _ = ox.kernel_search(q, 40, oracle.MODE_LEX)
+                assert np.array_equal(ids, o_ids), (metric, storage)
+                assert np.array_equal(hops, o_hops) and np.array_equal(evals, o_evals), (metric, storage)
