@@ -7,16 +7,11 @@
 // the entry with the smallest search distance, ties to the smaller id, and
 // the search starts there.  Nothing else in the search changes.
 //
-// The distance is the search kernel's, bit for bit, on the FP32 rows: lane l
-// of the search sums dims l, l+32, ... with fused multiply-adds and the 32
-// partial sums meet in an xor butterfly (16, 8, 4, 2, 1).  Here one thread
-// computes a whole distance: it keeps the 32 partial sums, adds each element
-// to the partial of its lane in dimension order, and then adds them in the
-// butterfly's pairs, which gives every lane's (identical) result.  The entry
-// rows are copied once into a contiguous block, which stays in L2.  The
-// two-level choice instead spreads each row over a warp as the search does,
-// 32 (query, row) pairs at a time, and adds the partials in a transposed
-// butterfly (entry_tiles.cuh): the same sums.
+// The distance is the search kernel's, bit for bit, on the FP32 rows (partial
+// p sums dims p, p+32, ... with fused multiply-adds, the 32 partials meet in
+// the xor butterfly): the warp takes one query and eight rows at a time, or
+// four queries and eight rows (entry_rows.cuh).  The entry rows are copied
+// once into a contiguous block.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -24,290 +19,13 @@
 #include <vector>
 
 #include "entry_choice.cuh"
+#include "entry_rows.cuh"
 #include "entry_tiles.cuh"
 #include "internal.h"
 #include "song_gb300.h"
 
 namespace song {
 namespace {
-
-// One warp serves QB queries; lane e takes entries e, e+32, ... and reads
-// each entry row once, in 16-byte pieces, for all QB queries.  Rows and the
-// staged queries are zero-padded to dpad (a multiple of 4) floats: a padded
-// element adds fma(0, 0, t) = t, leaving every partial sum exactly as the
-// search leaves it.  Each lane keeps its NS nearest entries per query in a
-// sorted register list; the warp then merges the lists, ns rounds of an xor
-// argmin, into starts[q*ns ..], ascending by (distance, id).
-template <int METRIC, int QB, int NS>
-__global__ void __launch_bounds__(256) nearest_entry_kernel(const float *queries, int nq, int qstride, int dim,
-                                                            int dpad,
-                                                            const float *entry_rows, const uint32_t *entry_ids,
-                                                            int n_entries, int ns, uint32_t *starts) {
-  extern __shared__ float4 qs4[];  // (blockDim / 32) * QB query rows of dpad floats
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int q0 = (blockIdx.x * (blockDim.x >> 5) + wib) * QB;
-  if (q0 >= nq) return;  // whole warps leave together
-  const int d4 = dpad >> 2;
-  float *qw = reinterpret_cast<float *>(qs4) + static_cast<size_t>(wib) * QB * dpad;
-  for (int b = 0; b < QB; ++b)
-    for (int j = lane; j < dpad; j += 32)
-      qw[b * dpad + j] = (q0 + b < nq && j < dim) ? queries[static_cast<size_t>(q0 + b) * qstride + j] : 0.0f;
-  __syncwarp();
-  const float4 *q4 = reinterpret_cast<const float4 *>(qw);
-  float bd[QB][NS];
-  uint32_t bi[QB][NS];
-#pragma unroll
-  for (int b = 0; b < QB; ++b)
-#pragma unroll
-    for (int m = 0; m < NS; ++m) {
-      bd[b][m] = __int_as_float(0x7f800000);  // +inf
-      bi[b][m] = 0xffffffffu;
-    }
-  for (int e = lane; e < n_entries; e += 32) {
-    const float4 *x4 = reinterpret_cast<const float4 *>(entry_rows + static_cast<size_t>(e) * dpad);
-    float t[QB][32], l[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      l[i] = 0.0f;
-#pragma unroll
-      for (int b = 0; b < QB; ++b) t[b][i] = 0.0f;
-    }
-    for (int c0 = 0; c0 < d4; c0 += 8) {  // 32 dimensions: partial 4i + c takes dimension 4 (c0 + i) + c
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (c0 + i < d4) {
-          const float4 xv = __ldg(x4 + c0 + i);
-          const float xs[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-          for (int b = 0; b < QB; ++b) {
-            const float4 qv = q4[b * d4 + c0 + i];
-            const float qq[4] = {qv.x, qv.y, qv.z, qv.w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              if (METRIC == SONG_METRIC_L2) {
-                const float d = __fsub_rn(qq[c], xs[c]);
-                t[b][4 * i + c] = __fmaf_rn(d, d, t[b][4 * i + c]);
-              } else {
-                t[b][4 * i + c] = __fmaf_rn(qq[c], xs[c], t[b][4 * i + c]);
-              }
-            }
-          }
-          if (METRIC == SONG_METRIC_COS) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) l[4 * i + c] = __fmaf_rn(xs[c], xs[c], l[4 * i + c]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-      for (int i = 0; i < off; ++i) {
-#pragma unroll
-        for (int b = 0; b < QB; ++b) t[b][i] = __fadd_rn(t[b][i], t[b][i + off]);
-        if (METRIC == SONG_METRIC_COS) l[i] = __fadd_rn(l[i], l[i + off]);
-      }
-    }
-    const uint32_t id = entry_ids[e];
-#pragma unroll
-    for (int b = 0; b < QB; ++b) {
-      float d;
-      if (METRIC == SONG_METRIC_L2) {
-        d = t[b][0];
-      } else if (METRIC == SONG_METRIC_IP) {
-        d = -t[b][0];
-      } else if (l[0] != 0.0f) {
-        const float sign = t[b][0] < 0.0f ? 1.0f : -1.0f;
-        d = __fdiv_rn(__fmul_rn(__fmul_rn(sign, t[b][0]), t[b][0]), l[0]);
-      } else {
-        d = 0.0f;
-      }
-      // sorted insertion, the last entry falls off (positions read before written)
-#pragma unroll
-      for (int m = NS - 1; m >= 0; --m) {
-        const bool above = m > 0 && closer(d, id, bd[b][m > 0 ? m - 1 : 0], bi[b][m > 0 ? m - 1 : 0]);
-        const bool here = closer(d, id, bd[b][m], bi[b][m]);
-        if (above) {
-          bd[b][m] = bd[b][m - (m > 0 ? 1 : 0)];
-          bi[b][m] = bi[b][m - (m > 0 ? 1 : 0)];
-        } else if (here) {
-          bd[b][m] = d;
-          bi[b][m] = id;
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int b = 0; b < QB; ++b) {
-    int h = 0;  // this lane's next unused list position
-    for (int r = 0; r < ns; ++r) {
-      float d = __int_as_float(0x7f800000);
-      uint32_t id = 0xffffffffu;
-#pragma unroll
-      for (int m = 0; m < NS; ++m)
-        if (m == h) {
-          d = bd[b][m];
-          id = bi[b][m];
-        }
-      float wd = d;
-      uint32_t wid = id;
-      for (int o = 16; o > 0; o >>= 1) {
-        const float od = __shfl_xor_sync(0xffffffffu, wd, o);
-        const uint32_t oid = __shfl_xor_sync(0xffffffffu, wid, o);
-        if (closer(od, oid, wd, wid)) {
-          wd = od;
-          wid = oid;
-        }
-      }
-      if (id == wid && id != 0xffffffffu) ++h;  // entry ids are distinct: one lane owns the winner
-      if (lane == 0 && q0 + b < nq) starts[static_cast<size_t>(q0 + b) * ns + r] = wid;
-    }
-  }
-}
-
-// The same choice with the entry rows staged through shared memory, for rows
-// of up to 1 KB: the block loads 32 entry rows at a time with coalesced
-// 16-byte loads into rows padded to an odd number of 16-byte units (so the
-// lanes' 16-byte reads of 32 different rows hit distinct banks), and every
-// warp of the block then scores them against its queries, lane e taking row
-// e of the tile.  Partial sums, order and merge are those of
-// nearest_entry_kernel.
-template <int METRIC, int QB, int NS>
-__global__ void __launch_bounds__(256) nearest_entry_tiled_kernel(const float *queries, int nq, int qstride, int dim,
-                                                            int dpad,
-                                                                  const float *entry_rows,
-                                                                  const uint32_t *entry_ids, int n_entries, int ns,
-                                                                  uint32_t *starts) {
-  extern __shared__ float4 sm4[];
-  constexpr int TILE = 32;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int q0 = (blockIdx.x * nwarps + wib) * QB;
-  const bool active = q0 < nq;  // warp-uniform; idle warps still help load tiles
-  const int d4 = dpad >> 2, rs4 = d4 + 1;
-  float4 *tile = sm4;
-  float *qw = reinterpret_cast<float *>(sm4 + TILE * rs4) + static_cast<size_t>(wib) * QB * dpad;
-  for (int b = 0; b < QB; ++b)
-    for (int j = lane; j < dpad; j += 32)
-      qw[b * dpad + j] = (q0 + b < nq && j < dim) ? queries[static_cast<size_t>(q0 + b) * qstride + j] : 0.0f;
-  const float4 *q4 = reinterpret_cast<const float4 *>(qw);
-  float bd[QB][NS];
-  uint32_t bi[QB][NS];
-#pragma unroll
-  for (int b = 0; b < QB; ++b)
-#pragma unroll
-    for (int m = 0; m < NS; ++m) {
-      bd[b][m] = __int_as_float(0x7f800000);
-      bi[b][m] = 0xffffffffu;
-    }
-  for (int t0 = 0; t0 < n_entries; t0 += TILE) {
-    const int rows = min(TILE, n_entries - t0);
-    __syncthreads();  // the previous tile is consumed (and, first time, the queries are staged)
-    for (int i = threadIdx.x; i < rows * d4; i += blockDim.x) {
-      const int r = i / d4, c = i - r * d4;
-      tile[r * rs4 + c] = __ldg(reinterpret_cast<const float4 *>(entry_rows + static_cast<size_t>(t0 + r) * dpad) + c);
-    }
-    __syncthreads();
-    if (!active || lane >= rows) continue;
-    const float4 *x4 = tile + lane * rs4;
-    float t[QB][32], l[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      l[i] = 0.0f;
-#pragma unroll
-      for (int b = 0; b < QB; ++b) t[b][i] = 0.0f;
-    }
-    for (int c0 = 0; c0 < d4; c0 += 8) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (c0 + i < d4) {
-          const float4 xv = x4[c0 + i];
-          const float xs[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-          for (int b = 0; b < QB; ++b) {
-            const float4 qv = q4[b * d4 + c0 + i];
-            const float qq[4] = {qv.x, qv.y, qv.z, qv.w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              if (METRIC == SONG_METRIC_L2) {
-                const float d = __fsub_rn(qq[c], xs[c]);
-                t[b][4 * i + c] = __fmaf_rn(d, d, t[b][4 * i + c]);
-              } else {
-                t[b][4 * i + c] = __fmaf_rn(qq[c], xs[c], t[b][4 * i + c]);
-              }
-            }
-          }
-          if (METRIC == SONG_METRIC_COS) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) l[4 * i + c] = __fmaf_rn(xs[c], xs[c], l[4 * i + c]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-      for (int i = 0; i < off; ++i) {
-#pragma unroll
-        for (int b = 0; b < QB; ++b) t[b][i] = __fadd_rn(t[b][i], t[b][i + off]);
-        if (METRIC == SONG_METRIC_COS) l[i] = __fadd_rn(l[i], l[i + off]);
-      }
-    }
-    const uint32_t id = entry_ids[t0 + lane];
-#pragma unroll
-    for (int b = 0; b < QB; ++b) {
-      float d;
-      if (METRIC == SONG_METRIC_L2) {
-        d = t[b][0];
-      } else if (METRIC == SONG_METRIC_IP) {
-        d = -t[b][0];
-      } else if (l[0] != 0.0f) {
-        const float sign = t[b][0] < 0.0f ? 1.0f : -1.0f;
-        d = __fdiv_rn(__fmul_rn(__fmul_rn(sign, t[b][0]), t[b][0]), l[0]);
-      } else {
-        d = 0.0f;
-      }
-#pragma unroll
-      for (int m = NS - 1; m >= 0; --m) {
-        const bool above = m > 0 && closer(d, id, bd[b][m > 0 ? m - 1 : 0], bi[b][m > 0 ? m - 1 : 0]);
-        const bool here = closer(d, id, bd[b][m], bi[b][m]);
-        if (above) {
-          bd[b][m] = bd[b][m - (m > 0 ? 1 : 0)];
-          bi[b][m] = bi[b][m - (m > 0 ? 1 : 0)];
-        } else if (here) {
-          bd[b][m] = d;
-          bi[b][m] = id;
-        }
-      }
-    }
-  }
-  if (!active) return;
-#pragma unroll
-  for (int b = 0; b < QB; ++b) {
-    int h = 0;
-    for (int r = 0; r < ns; ++r) {
-      float d = __int_as_float(0x7f800000);
-      uint32_t id = 0xffffffffu;
-#pragma unroll
-      for (int m = 0; m < NS; ++m)
-        if (m == h) {
-          d = bd[b][m];
-          id = bi[b][m];
-        }
-      float wd = d;
-      uint32_t wid = id;
-      for (int o = 16; o > 0; o >>= 1) {
-        const float od = __shfl_xor_sync(0xffffffffu, wd, o);
-        const uint32_t oid = __shfl_xor_sync(0xffffffffu, wid, o);
-        if (closer(od, oid, wd, wid)) {
-          wd = od;
-          wid = oid;
-        }
-      }
-      if (id == wid && id != 0xffffffffu) ++h;
-      if (lane == 0 && q0 + b < nq) starts[static_cast<size_t>(q0 + b) * ns + r] = wid;
-    }
-  }
-}
 
 // Gathers the FP32 rows of the entries into a contiguous block.
 __global__ void gather_entry_rows_kernel(const float *rows, uint32_t row_floats, const uint32_t *ids, int n,
@@ -320,54 +38,12 @@ __global__ void gather_entry_rows_kernel(const float *rows, uint32_t row_floats,
   }
 }
 
-// The ns nearest of n entry rows (ids) for each of nq query rows (stride
-// qstride floats), into out[q*ns ..].
-cudaError_t launch_nearest(const float *queries, int nq, int qstride, int dim, int dpad, int metric,
-                           const float *rows, const uint32_t *ids, int n, int ns, uint32_t *out, cudaStream_t s) {
-  // warps per block: up to 8, within the default 48 KB of shared memory;
-  // rows of up to 1 KB are staged through shared memory in 32-row tiles
-  const int qb = metric == SONG_METRIC_COS ? 1 : 2;
-  const int per_warp = static_cast<int>(sizeof(float)) * dpad * qb;
-  const int tile_bytes = 32 * (dpad / 4 + 1) * 16;
-  const bool tiled = dpad * 4 <= 1024 && tile_bytes + per_warp <= 48 * 1024;
-  const int avail = 48 * 1024 - (tiled ? tile_bytes : 0);
-  const int wpb = std::max(1, std::min(8, avail / per_warp));
-  const size_t smem = static_cast<size_t>(per_warp) * wpb + (tiled ? tile_bytes : 0);
-  const unsigned grid = static_cast<unsigned>((nq + wpb * qb - 1) / (wpb * qb));
-  const int NSel = ns <= 1 ? 1 : (ns <= 2 ? 2 : (ns <= 4 ? 4 : 8));
-#define SONG_ENTRY_LAUNCH(M, QB, NS)                                                                        \
-  do {                                                                                                   \
-    if (tiled)                                                                                           \
-      nearest_entry_tiled_kernel<M, QB, NS><<<grid, 32 * wpb, smem, s>>>(queries, nq, qstride, dim, dpad,  \
-                                                                         rows, ids, n, ns, out);         \
-    else                                                                                                 \
-      nearest_entry_kernel<M, QB, NS><<<grid, 32 * wpb, smem, s>>>(queries, nq, qstride, dim, dpad, rows, \
-                                                                   ids, n, ns, out);                     \
-  } while (0)
-#define SONG_ENTRY_BY_NS(M, QB)                 \
-  switch (NSel) {                               \
-    case 1: SONG_ENTRY_LAUNCH(M, QB, 1); break; \
-    case 2: SONG_ENTRY_LAUNCH(M, QB, 2); break; \
-    case 4: SONG_ENTRY_LAUNCH(M, QB, 4); break; \
-    default: SONG_ENTRY_LAUNCH(M, QB, 8); break; \
-  }
-  switch (metric) {
-    case SONG_METRIC_L2: SONG_ENTRY_BY_NS(SONG_METRIC_L2, 2); break;
-    case SONG_METRIC_IP: SONG_ENTRY_BY_NS(SONG_METRIC_IP, 2); break;
-    default: SONG_ENTRY_BY_NS(SONG_METRIC_COS, 1); break;
-  }
-#undef SONG_ENTRY_BY_NS
-#undef SONG_ENTRY_LAUNCH
-  return cudaGetLastError();
-}
-
 // ---------------------------------------------------------------------------
 // Two-level choice: the probes nearest coarse entries, then the ns nearest
-// entries of their clusters.  Both phases score warp tiles of 4 queries x 8
-// rows (entry_tiles.cuh: exact search distances) from shared memory.  The
-// second phase runs cluster by cluster: the probe lists are inverted into one
-// query list per cluster, and a block loads each cluster's rows once for all
-// queries probing it.  Each query's per-cluster best lists are then merged.
+// entries of their clusters.  The second phase runs cluster by cluster: the
+// probe lists are inverted into one query list per cluster, and four queries
+// share the cluster's rows.  Each query's per-cluster best lists are then
+// merged.  Small batches take both phases query by query.
 // ---------------------------------------------------------------------------
 
 // 16-byte global-to-shared copies that complete without holding registers
@@ -521,11 +197,12 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t s, uint32_t *w
 }
 
 // Exclusive scans of the per-cluster probe counts (one block): offs[0..n],
-// a copy of offs[0..n-1] as the scatter cursors, and task_offs[0..n] of the
-// clusters' warp tasks (one per 4 of its queries), the clusters taken in the
-// order `order` (task_offs[i] belongs to cluster order[i]).
+// a copy of offs[0..n-1] as the scatter cursors, and task_offs[c], the first
+// of cluster c's tasks (one per 4 of its queries) when the clusters are taken
+// in the order `order`; *n_tasks tasks in all.
 __global__ void __launch_bounds__(1024) cluster_scan_kernel(const uint32_t *count, int n, const uint32_t *order,
-                                                            uint32_t *offs, uint32_t *cursor, uint32_t *task_offs) {
+                                                            uint32_t *offs, uint32_t *cursor, uint32_t *task_offs,
+                                                            uint32_t *n_tasks) {
   __shared__ uint32_t warp_sum[32];
   const int per = (n + blockDim.x - 1) / blockDim.x;
   const int b = threadIdx.x * per, e = min(n, b + per);
@@ -541,171 +218,308 @@ __global__ void __launch_bounds__(1024) cluster_scan_kernel(const uint32_t *coun
     offs[i] = run;
     cursor[i] = run;
     run += count[i];
-    if (task_offs) task_offs[i] = trun;
-    trun += (count[order[i]] + 3u) / 4u;
+    const uint32_t c = order[i];
+    task_offs[c] = trun;
+    trun += (count[c] + 3u) / 4u;
   }
   if (threadIdx.x == 0) {
     offs[n] = total;
-    if (task_offs) task_offs[n] = ttotal;
+    *n_tasks = ttotal;
   }
 }
 
 // Inverts the probe lists: list[cursor[c]++] = q * probes + r for every
-// probe r of every query q that names cluster c.
-__global__ void cluster_scatter_kernel(const uint32_t *probe, int total, uint32_t *cursor, uint32_t *list) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
-    list[atomicAdd(cursor + probe[i], 1u)] = static_cast<uint32_t>(i);
-}
-
-// Two-level choice, second kernel: block c scores cluster c's entries
-// (rows row_offs[c] .. row_offs[c+1] of the cluster-ordered block) against
-// every query that probes it, 4 per warp at a time, and writes each
-// (query, probe) pair's NS nearest entries, ascending, to part_*.
-template <int METRIC, int NS>
-__global__ void __launch_bounds__(256) clusters_tiled_kernel(const float *queries, int dim, int dpad,
-                                                             const float *fine_rows, const uint32_t *fine_ids,
-                                                             const uint32_t *row_offs, const uint32_t *q_offs,
-                                                             const uint32_t *q_list, int probes, int tile_rows,
-                                                             int nbuf, float *part_d, uint32_t *part_i) {
-  extern __shared__ __align__(16) float smt[];
-  const int c = blockIdx.x;
-  const uint32_t a0 = q_offs[c], a1 = q_offs[c + 1];
-  if (a0 == a1) return;  // no query probes this cluster (uniform over the block)
-  const int r0 = static_cast<int>(row_offs[c]), r1 = static_cast<int>(row_offs[c + 1]);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int bq = 4 * (blockDim.x >> 5);  // queries per pass
-  float *qs = smt;
-  float *xb = smt + static_cast<size_t>(dpad) * bq;
-  const float *qw = qs + static_cast<size_t>(4 * warp) * dpad;
-  for (uint32_t qb = a0; qb < a1; qb += bq) {
-    const int nqb = static_cast<int>(min(static_cast<uint32_t>(bq), a1 - qb));
-    const bool busy = 4 * warp < nqb;  // warp-uniform
-    __syncthreads();  // the previous query tile is no longer read
-    for (int i = threadIdx.x; i < bq * dpad; i += blockDim.x) {
-      const int r = i / dpad, j = i - r * dpad;
-      float v = 0.0f;
-      if (r < nqb && j < dim) v = queries[static_cast<size_t>(q_list[qb + r] / probes) * dim + j];
-      qs[i] = v;
-    }
-    float bd[NS];
-    uint32_t bi[NS];
-#pragma unroll
-    for (int m = 0; m < NS; ++m) {
-      bd[m] = __int_as_float(0x7f800000);
-      bi[m] = 0xffffffffu;
-    }
-    stream_rows(fine_rows, dpad, r0, r1, tile_rows, nbuf, xb, [&](int first, int n, const float *cur) {
-      if (!busy) return;
-      for (int g = 0; g < n; g += 8) {
-        const float d = warp_tile_distance<METRIC>(qw, dpad, cur + static_cast<size_t>(g) * dpad, dpad, dpad, lane);
-        const int r = g + (lane & 7);
-        if (r < n) list_insert<NS>(bd, bi, d, fine_ids[first + r]);
-      }
-    });
-    const int slot = 4 * warp + (lane >> 3);
-    const uint32_t pair = slot < nqb ? q_list[qb + slot] : 0u;
-    int h = 0;
-#pragma unroll
-    for (int r = 0; r < NS; ++r) {
-      float wd;
-      uint32_t wid;
-      group8_take<NS>(bd, bi, h, wd, wid);
-      if ((lane & 7) == 0 && slot < nqb) {
-        part_d[static_cast<size_t>(pair) * NS + r] = wd;
-        part_i[static_cast<size_t>(pair) * NS + r] = wid;
-      }
-    }
+// probe r of every query q that names cluster c.  The first of each four
+// writes their task: (cluster, which four).
+__global__ void cluster_scatter_kernel(const uint32_t *probe, int total, const uint32_t *offs,
+                                       const uint32_t *task_offs, uint32_t *cursor, uint32_t *list, uint2 *tasks) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint32_t c = probe[i], at = atomicAdd(cursor + c, 1u), k = at - offs[c];
+    list[at] = static_cast<uint32_t>(i);
+    if ((k & 3u) == 0u) tasks[task_offs[c] + (k >> 2)] = make_uint2(c, k >> 2);
   }
 }
 
-// Two-level choice, second kernel for rows of up to WARP_TASK_DPAD floats:
-// warp tasks of (cluster, 4 of the queries that probe it), taken by
-// persistent warps (task_offs: the scan's per-cluster task offsets).  A warp
-// stages its 4 queries and streams the cluster's rows 8 at a time through a
-// double buffer of its own (cp.async; warp barriers only), scores them as a
-// warp tile, and writes each (query, probe) pair's NS nearest entries.
-constexpr int WARP_TASK_DPAD = 256;
-constexpr int WT_WARPS = 4;  // warps per block
-
-size_t warp_task_smem(int dpad) { return sizeof(float) * static_cast<size_t>(dpad) * (4 + 2 * 8) * WT_WARPS; }
-
+// Two-level choice, second kernel: tasks of (cluster, 4 of the queries that
+// probe it), taken by persistent blocks of `warps` warps.  The block stages
+// its 4 queries, its warps take the cluster's rows eight at a time in turn
+// (tile_distance), and the lists of all warps meet in shared memory: each
+// (query, probe) pair's NS nearest entries go to part_*.
+// What bounds it: FP32 instructions while there are many tasks (a third of
+// the issue slots at 10,000 queries; its rows' 282 MB come from DRAM once,
+// prefetched a pass ahead: 360 -> 348 us for the choice), else the rows'
+// latency, which four warps a task and 128 registers of loads in flight
+// shorten: a block per cluster with its rows staged in shared memory took
+// 2,150 us of the 960-d choice of 1000 queries, now 382 in all.
 template <int METRIC, int NS>
-__global__ void __launch_bounds__(WT_WARPS * 32) clusters_warp_kernel(const float *queries, int dim, int dpad,
-                                                                      const float *fine_rows,
-                                                                      const uint32_t *fine_ids,
-                                                                      const uint32_t *row_offs,
-                                                                      const uint32_t *q_offs, const uint32_t *q_list,
-                                                                      const uint32_t *task_offs,
-                                                                      const uint32_t *cl_order, int n_clusters,
-                                                                      int probes, float *part_d, uint32_t *part_i) {
+__global__ void __launch_bounds__(128, 4) clusters_rows_kernel(const float *queries, int dim, int dpad, int qs,
+                                                            const float *fine_rows, const uint32_t *fine_ids,
+                                                            const uint32_t *row_offs, const uint32_t *q_offs,
+                                                            const uint32_t *q_list, const uint2 *tasks,
+                                                            const uint32_t *n_tasks, int probes, float *part_d,
+                                                            uint32_t *part_i) {
   extern __shared__ __align__(16) float smt[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  float *qs = smt + static_cast<size_t>(wib) * dpad * (4 + 16);
-  float *xb = qs + static_cast<size_t>(4) * dpad;  // two buffers of 8 rows
-  const uint32_t total = task_offs[n_clusters];
-  const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-  const int d4 = dpad / 4;
-  for (uint32_t t = blockIdx.x * (blockDim.x >> 5) + wib; t < total; t += nwarps) {
-    // the cluster of task t: the last position with task_offs <= t
-    int lo = 0, hi = n_clusters - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (task_offs[mid] <= t) lo = mid;
-      else hi = mid - 1;
-    }
-    const int at = lo;
-    const int c = static_cast<int>(cl_order[at]);
-    const uint32_t qb = q_offs[c] + 4u * (t - task_offs[at]);
+  __shared__ float md[4][4][NS];
+  __shared__ uint32_t mi[4][4][NS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const uint32_t total = *n_tasks;
+  for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
+    const uint2 task = tasks[t];
+    const uint32_t c = task.x, qb = q_offs[c] + 4u * task.y;
     const int nqg = static_cast<int>(min(4u, q_offs[c + 1] - qb));
     const int r0 = static_cast<int>(row_offs[c]), r1 = static_cast<int>(row_offs[c + 1]);
-    __syncwarp();  // the previous task's buffers are no longer read
-    for (int i = lane; i < 4 * dpad; i += 32) {
-      const int a = i / dpad, j = i - a * dpad;
-      qs[i] = (a < nqg && j < dim) ? queries[static_cast<size_t>(q_list[qb + a] / probes) * dim + j] : 0.0f;
-    }
+    __syncthreads();  // the previous task's queries and lists are no longer read
+    stage_queries<4>(smt, qs, dim, nqg, threadIdx.x, blockDim.x, [&](int a) {
+      return queries + static_cast<size_t>(q_list[qb + a] / static_cast<uint32_t>(probes)) * dim;
+    });
+    __syncthreads();
     float bd[NS];
     uint32_t bi[NS];
-#pragma unroll
-    for (int m = 0; m < NS; ++m) {
-      bd[m] = __int_as_float(0x7f800000);
-      bi[m] = 0xffffffffu;
-    }
-    auto issue = [&](int first, float *buf) {
-      const int n4 = min(8, r1 - first) * d4;
-      const float4 *src = reinterpret_cast<const float4 *>(fine_rows + static_cast<size_t>(first) * dpad);
-      float4 *dst = reinterpret_cast<float4 *>(buf);
-      for (int i = lane; i < n4; i += 32) cp_async16(dst + i, src + i);
-      cp_async_commit();
-    };
-    issue(r0, xb);
-    for (int first = r0, k = 0; first < r1; first += 8, ++k) {
-      float *cur = xb + static_cast<size_t>(k & 1) * 8 * dpad;
-      if (first + 8 < r1) {
-        issue(first + 8, xb + static_cast<size_t>((k + 1) & 1) * 8 * dpad);
-      } else {
-        cp_async_commit();
+    clear_list<NS>(bd, bi);
+    for (int first = r0 + 8 * warp; first < r1; first += 8 * warps) {
+      // the rows of this warp's next pass start their way into L2: on a
+      // large base they come from DRAM (each cluster is read once)
+      const int ahead = first + 8 * warps;
+      if (ahead < r1) {
+        const char *nx = reinterpret_cast<const char *>(fine_rows + static_cast<size_t>(ahead) * dpad);
+        const int bytes = min(8, r1 - ahead) * dpad * 4;
+        for (int i = 128 * lane; i < bytes; i += 128 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + i));
       }
-      cp_async_wait<1>();
-      __syncwarp();  // every lane's copies (and the staged queries) are visible
-      const float d = warp_tile_distance<METRIC>(qs, dpad, cur, dpad, dpad, lane);
+      const float d = tile_distance<METRIC>(smt, qs, fine_rows + static_cast<size_t>(first) * dpad, r1 - 1 - first,
+                                            dpad, lane);
       const int r = first + (lane & 7);
-      if (r < r1) list_insert<NS>(bd, bi, d, fine_ids[r]);
-      __syncwarp();  // this buffer is refilled two rounds on
+      const uint32_t id = r < r1 ? __ldg(fine_ids + r) : 0xffffffffu;
+      if (r < r1 && closer(d, id, bd[NS - 1], bi[NS - 1])) list_insert<NS>(bd, bi, d, id);
     }
     const int a = lane >> 3;
     const uint32_t pair = a < nqg ? q_list[qb + a] : 0u;
+    const size_t at = static_cast<size_t>(pair) * NS;
     int h = 0;
+    __syncwarp();
 #pragma unroll
     for (int r = 0; r < NS; ++r) {
       float wd;
       uint32_t wid;
       group8_take<NS>(bd, bi, h, wd, wid);
-      if ((lane & 7) == 0 && a < nqg) {
-        part_d[static_cast<size_t>(pair) * NS + r] = wd;
-        part_i[static_cast<size_t>(pair) * NS + r] = wid;
+      if ((lane & 7) == 0) {
+        if (warps > 1) {
+          md[warp][a][r] = wd;
+          mi[warp][a][r] = wid;
+        } else if (a < nqg) {
+          part_d[at + r] = wd;
+          part_i[at + r] = wid;
+        }
+      }
+    }
+    if (warps == 1) continue;
+    __syncthreads();
+    if (warp == 0) {
+      const int i = lane & 7;  // lane l takes warp l & 7's list of query l / 8
+      clear_list<NS>(bd, bi);
+      if (i < warps) {
+#pragma unroll
+        for (int r = 0; r < NS; ++r) {
+          bd[r] = md[i][a][r];
+          bi[r] = mi[i][a][r];
+        }
+      }
+      h = 0;
+      __syncwarp();
+#pragma unroll
+      for (int r = 0; r < NS; ++r) {
+        float wd;
+        uint32_t wid;
+        group8_take<NS>(bd, bi, h, wd, wid);
+        if (i == 0 && a < nqg) {
+          part_d[at + r] = wd;
+          part_i[at + r] = wid;
+        }
       }
     }
   }
+}
+
+// Small batches: the whole two-level choice in two kernels, every head scored
+// exactly (the heads stay in L2, and a few hundred queries' exact scan takes
+// less than the tensor-core phase's three launches and the grouping by
+// cluster: one query of 1M x 128 takes 22 us for the choice, 90 there).
+// First (and for the flat choice, over all entries), block (x, y): rows
+// chunk * x .. against the NQ queries from NQ * y, eight warps; each query's
+// NP nearest of the chunk, by the rows' ids or positions (ids null), to
+// part_* (queries x chunks x NP).
+template <int METRIC, int NP, int NQ>
+__global__ void __launch_bounds__(256, 2) nearest_rows_kernel(const float *queries, int nq, int qstride, int dim,
+                                                              int dpad, int qs, const float *heads,
+                                                              const uint32_t *ids, int n_heads, int chunk,
+                                                              float *part_d, uint32_t *part_i) {
+  extern __shared__ __align__(16) float smt[];
+  __shared__ float md[8][4][NP];
+  __shared__ uint32_t mi[8][4][NP];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q0 = NQ * blockIdx.y, nqg = min(NQ, nq - q0);
+  stage_queries<NQ>(smt, qs, dim, nqg, threadIdx.x, blockDim.x,
+                    [&](int a) { return queries + static_cast<size_t>(q0 + a) * qstride; });
+  __syncthreads();
+  float bd[NP];
+  uint32_t bi[NP];
+  clear_list<NP>(bd, bi);
+  const int r0 = chunk * blockIdx.x, r1 = min(n_heads, r0 + chunk);
+  for (int first = r0 + 8 * warp; first < r1; first += 64) {
+    const float *row = heads + static_cast<size_t>(first) * dpad;
+    float d;
+    int r;
+    if (NQ == 1) {  // four lanes a row; the first of them keeps it
+      float one[1];
+      r = first + (lane >> 2);
+      rows8_distance<METRIC, 1>(row + static_cast<size_t>(min(lane >> 2, r1 - 1 - first)) * dpad, smt, qs, dpad, one,
+                                lane);
+      d = one[0];
+      if ((lane & 3) != 0) r = r1;
+    } else {
+      d = tile_distance<METRIC>(smt, qs, row, r1 - 1 - first, dpad, lane);
+      r = first + (lane & 7);
+    }
+    const uint32_t name = ids && r < r1 ? __ldg(ids + r) : static_cast<uint32_t>(r);
+    if (r < r1 && closer(d, name, bd[NP - 1], bi[NP - 1])) list_insert<NP>(bd, bi, d, name);
+  }
+  // NQ = 1: one list over the warp; else query l >> 3's over eight lanes
+  const int a = NQ == 1 ? 0 : lane >> 3;
+  int h = 0;
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < NP; ++r) {
+    float wd;
+    uint32_t wid;
+    if (NQ == 1) warp_list_take<NP>(bd, bi, h, wd, wid);
+    else group8_take<NP>(bd, bi, h, wd, wid);
+    if ((lane & 7) == 0) {
+      md[warp][a][r] = wd;
+      mi[warp][a][r] = wid;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int q = lane >> 3;  // lane l takes warp l & 7's list of query l >> 3
+    clear_list<NP>(bd, bi);
+    if (q < NQ) {
+#pragma unroll
+      for (int r = 0; r < NP; ++r) {
+        bd[r] = md[lane & 7][q][r];
+        bi[r] = mi[lane & 7][q][r];
+      }
+    }
+    h = 0;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < NP; ++r) {
+      float wd;
+      uint32_t wid;
+      group8_take<NP>(bd, bi, h, wd, wid);
+      if ((lane & 7) == 0 && q < nqg) {
+        const size_t at = (static_cast<size_t>(q0 + q) * gridDim.x + blockIdx.x) * NP + r;
+        part_d[at] = wd;
+        part_i[at] = wid;
+      }
+    }
+  }
+}
+
+// The flat choice's end: a warp per query merges the chunks' lists.
+template <int N>
+__global__ void __launch_bounds__(256) merge_lists_kernel(const float *part_d, const uint32_t *part_i, int nq,
+                                                          int chunks, int ns, uint32_t *out) {
+  const int lane = threadIdx.x & 31, q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q >= nq) return;  // whole warps
+  float bd[N];
+  uint32_t bi[N];
+  clear_list<N>(bd, bi);
+  const size_t base = static_cast<size_t>(q) * chunks * N;
+  for (int i = lane; i < chunks * N; i += 32) list_insert<N>(bd, bi, part_d[base + i], part_i[base + i]);
+  int h = 0;
+  __syncwarp();
+  for (int r = 0; r < ns; ++r) {
+    float wd;
+    uint32_t wid;
+    warp_list_take<N>(bd, bi, h, wd, wid);
+    // no finite distance (a query that is not finite): vertex 0
+    if (lane == 0) out[static_cast<size_t>(q) * ns + r] = wid == 0xffffffffu ? 0u : wid;
+  }
+}
+
+// The N smallest of the block's lists (16 warps), ascending, to out(r, d, id)
+// on one lane of warp 0; ends with the lists no longer read.
+template <int N, class Out>
+__device__ __forceinline__ void block_lists(float (&bd)[N], uint32_t (&bi)[N], int n, float (*md)[8],
+                                            uint32_t (*mi)[8], int warp, int lane, Out out) {
+  int h = 0;
+  for (int r = 0; r < n; ++r) {
+    float wd;
+    uint32_t wid;
+    warp_list_take<N>(bd, bi, h, wd, wid);
+    if (lane == 0) {
+      md[warp][r] = wd;
+      mi[warp][r] = wid;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    clear_list<N>(bd, bi);
+#pragma unroll
+    for (int r = 0; r < N; ++r)
+      if (lane < 16 && r < n) {
+        bd[r] = md[lane][r];
+        bi[r] = mi[lane][r];
+      }
+    h = 0;
+    for (int r = 0; r < n; ++r) {
+      float wd;
+      uint32_t wid;
+      warp_list_take<N>(bd, bi, h, wd, wid);
+      if (lane == 0) out(r, wid);
+    }
+  }
+  __syncthreads();
+}
+
+// Then a block of 16 warps per query: its probed clusters from the chunks'
+// lists, and its ns nearest entries over those clusters' rows, the warps
+// taking eight rows in turn.
+template <int METRIC, int NP, int NS>
+__global__ void __launch_bounds__(512) query_starts_kernel(const float *queries, int dim, int dpad, int qs,
+                                                           const float *part_d, const uint32_t *part_i, int chunks,
+                                                           int n_heads, int probes, const float *fine_rows,
+                                                           const uint32_t *fine_ids, const uint32_t *row_offs, int ns,
+                                                           uint32_t *starts) {
+  extern __shared__ __align__(16) float smt[];
+  __shared__ float md[16][8];
+  __shared__ uint32_t mi[16][8];
+  __shared__ uint32_t probe[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t q = blockIdx.x;
+  stage_queries<1>(smt, qs, dim, 1, threadIdx.x, blockDim.x, [&](int) { return queries + q * dim; });
+  {
+    float bd[NP];
+    uint32_t bi[NP];
+    clear_list<NP>(bd, bi);
+    const size_t base = q * chunks * NP;
+    for (int i = threadIdx.x; i < chunks * NP; i += blockDim.x)
+      list_insert<NP>(bd, bi, part_d[base + i], part_i[base + i]);
+    // (a query that is not finite has no nearest head: cluster 0)
+    block_lists<NP>(bd, bi, probes, md, mi, warp, lane,
+                    [&](int r, uint32_t id) { probe[r] = id < static_cast<uint32_t>(n_heads) ? id : 0u; });
+  }
+  float bd[NS];
+  uint32_t bi[NS];
+  clear_list<NS>(bd, bi);
+  int turn = warp;  // passes until this warp's next one
+  for (int i = 0; i < probes; ++i) {
+    const int r0 = static_cast<int>(row_offs[probe[i]]), r1 = static_cast<int>(row_offs[probe[i] + 1]);
+    scan_rows<METRIC, NS>(fine_rows, dpad, r0 + 8 * turn, 128, r1, smt, qs, bd, bi, lane,
+                             [&](int row) { return __ldg(fine_ids + row); });
+    turn = (turn + 15 * ((r1 - r0 + 7) / 8)) & 15;
+  }
+  block_lists<NS>(bd, bi, ns, md, mi, warp, lane,
+                  [&](int r, uint32_t id) { starts[q * ns + r] = id == 0xffffffffu ? 0u : id; });
 }
 
 // Each query's ns nearest over its probes' lists, ascending by (distance, id).
@@ -724,7 +538,8 @@ __global__ void merge_starts_kernel(const float *part_d, const uint32_t *part_i,
     for (int i = 0; i < probes * NS; ++i) list_insert<NS>(bd, bi, part_d[base + i], part_i[base + i]);
 #pragma unroll
     for (int m = 0; m < NS; ++m)
-      if (m < ns) starts[static_cast<size_t>(q) * ns + m] = bi[m];
+      if (m < ns)  // no finite distance (a query that is not finite): vertex 0
+        starts[static_cast<size_t>(q) * ns + m] = bi[m] == 0xffffffffu ? 0u : bi[m];
   }
 }
 
@@ -734,10 +549,146 @@ cudaError_t allow_smem(K kern, size_t bytes) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
 }
 
+// Work area of the choice, grown to `words`.
+cudaError_t entry_work(song_index *ix, size_t words) {
+  if (words <= ix->cap_entry_work) return cudaSuccess;
+  cudaFree(ix->d_entry_work);
+  ix->d_entry_work = nullptr;
+  ix->cap_entry_work = 0;
+  cudaError_t e = song::dev_malloc(&ix->d_entry_work, sizeof(uint32_t) * words);
+  if (e == cudaSuccess) ix->cap_entry_work = words;
+  return e;
+}
+
+// Template arguments for run-time list lengths 1, 2, 4 or 8.
+#define SONG_BY_LEN(n, CALL)  \
+  switch (n) {                \
+    case 1: CALL(1); break;   \
+    case 2: CALL(2); break;   \
+    case 4: CALL(4); break;   \
+    default: CALL(8); break;  \
+  }
+
+// Batches that take the two-kernel choice: up to 512 queries, and up to 2^28
+// query x head x dimension products (1M x 128, 4096 heads: 68 against 96 us at
+// 257 queries, 112 against 109 at 512; 960-d rows, 1024 heads: 230 against
+// 323 at 257, 355 against 349 at 600); with few short heads, 2^22 products
+// (15k x 16, 128 heads: 44 against 94 us at 1000 queries).
+bool small_batch(int nq, int coarse, int dpad) {
+  const double work = static_cast<double>(nq) * coarse * dpad;
+  return (nq <= 512 && work <= 268435456.0) || work <= 4194304.0;
+}
+
+// The NP nearest of n rows for each of nq queries, chunk by chunk: *chunks
+// lists a query in the work area.
+template <int METRIC, int NP>
+cudaError_t launch_nearest_rows(song_index *ix, const float *queries, int nq, int qstride, const float *rows,
+                                const uint32_t *ids, int n, int *chunks, float **part_d, uint32_t **part_i,
+                                cudaStream_t s) {
+  const int dim = ix->dx.dim, dpad = static_cast<int>(ix->dx.f32_row_bytes / 4), qs = (dpad + 31) & ~31;
+  // one query a block row while there are few, four afterwards; chunks of 64
+  // rows (one pass a warp) until the grid fills the GPU some times over
+  const int nqb = nq <= 4 ? 1 : 4;
+  const long long groups = (nq + nqb - 1) / nqb;
+  int chunk = 64;
+  while (chunk < n && groups * (n / chunk) > 2048) chunk *= 2;
+  *chunks = (n + chunk - 1) / chunk;
+  const size_t lists = static_cast<size_t>(nq) * *chunks * NP;
+  cudaError_t e = entry_work(ix, 2 * lists);
+  if (e != cudaSuccess) return e;
+  *part_d = reinterpret_cast<float *>(ix->d_entry_work);
+  *part_i = ix->d_entry_work + lists;
+  auto k = nqb == 1 ? nearest_rows_kernel<METRIC, NP, 1> : nearest_rows_kernel<METRIC, NP, 4>;
+  const size_t smem = sizeof(float) * nqb * qs;
+  if ((e = allow_smem(k, smem)) != cudaSuccess) return e;
+  // at most 65,535 block rows a launch
+  for (int q0 = 0; q0 < nq; q0 += 65535 * nqb) {
+    const int m = std::min(nq - q0, 65535 * nqb);
+    const size_t at = static_cast<size_t>(q0) * *chunks * NP;
+    k<<<dim3(*chunks, (m + nqb - 1) / nqb), 256, smem, s>>>(queries + static_cast<size_t>(q0) * qstride, m, qstride,
+                                                           dim, dpad, qs, rows, ids, n, chunk, *part_d + at,
+                                                           *part_i + at);
+  }
+  return cudaGetLastError();
+}
+
+// The ns nearest of n rows (ids) for each of nq queries (qstride floats
+// apart), into out[q * ns ..]: the flat choice.  4096 entries of 256 floats:
+// 1.19 ms for 10,000 queries (3.15 with a thread per distance), 18 us for one
+// (773: one warp then took all the entries).
+template <int METRIC, int N>
+cudaError_t launch_flat(song_index *ix, const float *queries, int nq, int qstride, const float *rows,
+                        const uint32_t *ids, int n, int ns, uint32_t *out, cudaStream_t s) {
+  int chunks = 0;
+  float *part_d = nullptr;
+  uint32_t *part_i = nullptr;
+  cudaError_t e = launch_nearest_rows<METRIC, N>(ix, queries, nq, qstride, rows, ids, n, &chunks, &part_d, &part_i, s);
+  if (e != cudaSuccess) return e;
+  merge_lists_kernel<N><<<(nq + 7) / 8, 256, 0, s>>>(part_d, part_i, nq, chunks, ns, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_nearest(song_index *ix, const float *queries, int nq, int qstride, const float *rows,
+                           const uint32_t *ids, int n, int ns, uint32_t *out, cudaStream_t s) {
+  const int len = ns <= 1 ? 1 : (ns <= 2 ? 2 : (ns <= 4 ? 4 : 8));
+  cudaError_t e = cudaSuccess;
+#define SONG_FLAT_L2(N) e = launch_flat<SONG_METRIC_L2, N>(ix, queries, nq, qstride, rows, ids, n, ns, out, s)
+#define SONG_FLAT_IP(N) e = launch_flat<SONG_METRIC_IP, N>(ix, queries, nq, qstride, rows, ids, n, ns, out, s)
+#define SONG_FLAT_COS(N) e = launch_flat<SONG_METRIC_COS, N>(ix, queries, nq, qstride, rows, ids, n, ns, out, s)
+  switch (ix->dx.metric) {
+    case SONG_METRIC_L2: SONG_BY_LEN(len, SONG_FLAT_L2); break;
+    case SONG_METRIC_IP: SONG_BY_LEN(len, SONG_FLAT_IP); break;
+    default: SONG_BY_LEN(len, SONG_FLAT_COS); break;
+  }
+#undef SONG_FLAT_L2
+#undef SONG_FLAT_IP
+#undef SONG_FLAT_COS
+  return e;
+}
+
+template <int METRIC, int NP>
+cudaError_t launch_small(song_index *ix, const float *queries, int nq, int ns, uint32_t *out, cudaStream_t s) {
+  const int dim = ix->dx.dim, dpad = static_cast<int>(ix->dx.f32_row_bytes / 4), qs = (dpad + 31) & ~31;
+  const int n = ix->n_coarse;
+  int chunks = 0;
+  float *part_d = nullptr;
+  uint32_t *part_i = nullptr;
+  cudaError_t e = launch_nearest_rows<METRIC, NP>(ix, queries, nq, dim, ix->d_coarse_rows, nullptr, n, &chunks,
+                                                  &part_d, &part_i, s);
+  if (e != cudaSuccess) return e;
+#define SONG_STARTS(NS)                                                                                       \
+  do {                                                                                                        \
+    auto k = query_starts_kernel<METRIC, NP, NS>;                                                             \
+    if ((e = allow_smem(k, sizeof(float) * qs)) != cudaSuccess) return e;                                     \
+    k<<<nq, 512, sizeof(float) * qs, s>>>(queries, dim, dpad, qs, part_d, part_i, chunks, n, ix->n_probes,    \
+                                          ix->d_entry_rows, ix->d_entry_ids, ix->d_offsets, ns, out);         \
+  } while (0)
+  SONG_BY_LEN(ns <= 1 ? 1 : (ns <= 2 ? 2 : (ns <= 4 ? 4 : 8)), SONG_STARTS);
+#undef SONG_STARTS
+  return cudaGetLastError();
+}
+
+template <int METRIC>
+cudaError_t launch_small_by_probes(song_index *ix, const float *queries, int nq, uint32_t *out, cudaStream_t s) {
+  const int np = ix->n_probes;
+  cudaError_t e = cudaSuccess;
+#define SONG_SMALL(NP) e = launch_small<METRIC, NP>(ix, queries, nq, ix->n_starts, out, s)
+  SONG_BY_LEN(np <= 1 ? 1 : (np <= 2 ? 2 : (np <= 4 ? 4 : 8)), SONG_SMALL);
+#undef SONG_SMALL
+  return e;
+}
+
 // The two-level choice on stream s.  `out` holds nq * (ns + probes) words:
 // the starts, then the probed clusters.
 cudaError_t launch_2level(song_index *ix, const float *queries, int nq, uint32_t *out, cudaStream_t s) {
-  const int dim = ix->dx.dim, dpad = static_cast<int>(ix->dx.f32_row_bytes / 4);
+  if (!ix->head_stats_on && small_batch(nq, ix->n_coarse, static_cast<int>(ix->dx.f32_row_bytes / 4))) {
+    switch (ix->dx.metric) {
+      case SONG_METRIC_L2: return launch_small_by_probes<SONG_METRIC_L2>(ix, queries, nq, out, s);
+      case SONG_METRIC_IP: return launch_small_by_probes<SONG_METRIC_IP>(ix, queries, nq, out, s);
+      default: return launch_small_by_probes<SONG_METRIC_COS>(ix, queries, nq, out, s);
+    }
+  }
+  const int dim = ix->dx.dim, dpad = static_cast<int>(ix->dx.f32_row_bytes / 4), qs = (dpad + 31) & ~31;
   const int ns = ix->n_starts, np = ix->n_probes, coarse = ix->n_coarse;
   const TileShape ts = tile_shape(dpad);
   const size_t smem = ts.smem(dpad);
@@ -745,24 +696,25 @@ cudaError_t launch_2level(song_index *ix, const float *queries, int nq, uint32_t
   const int NSel = ns <= 1 ? 1 : (ns <= 2 ? 2 : (ns <= 4 ? 4 : 8));
   const int NPsel = np <= 1 ? 1 : (np <= 2 ? 2 : (np <= 4 ? 4 : 8));
   uint32_t *probes = out + static_cast<size_t>(nq) * ns;
-  // work area: cursors, offsets, inverted lists, per-(query, probe) lists
+  // work area: tasks (at most one per pair), cursors, offsets, the tasks'
+  // offsets, inverted lists, per-(query, probe) lists
   const size_t pairs = static_cast<size_t>(nq) * np;
-  const size_t need = static_cast<size_t>(coarse) * 3 + 2 + pairs + 2 * pairs * NSel;
-  if (need > ix->cap_entry_work) {
-    cudaFree(ix->d_entry_work);
-    ix->d_entry_work = nullptr;
-    ix->cap_entry_work = 0;
-    cudaError_t e = song::dev_malloc(&ix->d_entry_work, sizeof(uint32_t) * need);
-    if (e != cudaSuccess) return e;
-    ix->cap_entry_work = need;
-  }
-  uint32_t *cursor = ix->d_entry_work;
+  cudaError_t e = entry_work(ix, 2 * pairs + static_cast<size_t>(coarse) * 3 + 2 + pairs + 2 * pairs * NSel);
+  if (e != cudaSuccess) return e;
+  uint2 *tasks = reinterpret_cast<uint2 *>(ix->d_entry_work);
+  uint32_t *cursor = ix->d_entry_work + 2 * pairs;
   uint32_t *q_offs = cursor + coarse;
-  uint32_t *q_list = q_offs + coarse + 1;
+  uint32_t *task_offs = q_offs + coarse + 1;
+  uint32_t *n_tasks = task_offs + coarse;
+  uint32_t *q_list = n_tasks + 1;
   float *part_d = reinterpret_cast<float *>(q_list + pairs);
   uint32_t *part_i = q_list + pairs + pairs * NSel;
-  uint32_t *task_offs = part_i + pairs * NSel;  // coarse + 1
-  cudaError_t e = cudaMemsetAsync(ix->d_cl_count, 0, sizeof(uint32_t) * coarse, s);
+  // warps a task: four share a task's rows while there are few tasks, two
+  // from 32768 pairs on (10,000 queries, 4 probes: 348 us for the whole choice
+  // with two, 367 with four, 360 with one; 2501 queries of 256-d rows 313 us
+  // with one, 187 with four)
+  const int tw = pairs >= 32768 ? 2 : 4;
+  e = cudaMemsetAsync(ix->d_cl_count, 0, sizeof(uint32_t) * coarse, s);
   if (e != cudaSuccess) return e;
   const unsigned grid_q = static_cast<unsigned>((nq + bq - 1) / bq);
 #define SONG_HEADS(M, NP)                                                                                \
@@ -774,62 +726,50 @@ cudaError_t launch_2level(song_index *ix, const float *queries, int nq, uint32_t
   } while (0)
 #define SONG_CLUSTERS(M, NS)                                                                             \
   do {                                                                                                   \
-    if (dpad <= WARP_TASK_DPAD) {                                                                        \
-      auto w_ = clusters_warp_kernel<M, NS>;                                                             \
-      const size_t wsm = warp_task_smem(dpad);                                                           \
-      if ((e = allow_smem(w_, wsm)) != cudaSuccess) return e;                                            \
-      int per_sm = 0, sms = 0, dev = 0;                                                                  \
-      cudaGetDevice(&dev);                                                                               \
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);                                 \
-      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, w_, WT_WARPS * 32, wsm)) != cudaSuccess) \
-        return e;                                                                                        \
-      w_<<<std::max(1, per_sm) * sms, WT_WARPS * 32, wsm, s>>>(queries, dim, dpad, ix->d_entry_rows,    \
-                                                             ix->d_entry_ids, ix->d_offsets, q_offs, q_list, \
-                                                             task_offs, ix->d_cl_order, coarse, np, part_d,   \
-                                                             part_i);                                   \
-      merge_starts_kernel<NS><<<(nq + 255) / 256, 256, 0, s>>>(part_d, part_i, nq, np, ns, out);         \
-      break;                                                                                             \
-    }                                                                                                    \
-    auto k_ = clusters_tiled_kernel<M, NS>;                                                              \
-    if ((e = allow_smem(k_, smem)) != cudaSuccess) return e;                                             \
-    k_<<<coarse, ts.warps * 32, smem, s>>>(queries, dim, dpad, ix->d_entry_rows, ix->d_entry_ids,         \
-                                           ix->d_offsets, q_offs, q_list, np, ts.rows, ts.nbuf, part_d,  \
-                                           part_i);                                                      \
+    auto k_ = clusters_rows_kernel<M, NS>;                                                               \
+    const size_t qsm = sizeof(float) * 4 * qs;                                                           \
+    if ((e = allow_smem(k_, qsm)) != cudaSuccess) return e;                                              \
+    int per_sm = 0, sms = 0, dev = 0;                                                                    \
+    cudaGetDevice(&dev);                                                                                 \
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);                                   \
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_, 32 * tw, qsm)) != cudaSuccess)   \
+      return e;                                                                                          \
+    const size_t cap = static_cast<size_t>(std::max(1, per_sm)) * sms;                                   \
+    k_<<<static_cast<unsigned>(std::min(cap, pairs)), 32 * tw, qsm, s>>>(                                \
+        queries, dim, dpad, qs, ix->d_entry_rows, ix->d_entry_ids, ix->d_offsets, q_offs, q_list, tasks, \
+        n_tasks, np, part_d, part_i);                                                                    \
     merge_starts_kernel<NS><<<(nq + 255) / 256, 256, 0, s>>>(part_d, part_i, nq, np, ns, out);           \
   } while (0)
-#define SONG_HEADS_BY_NP(M)               \
-  switch (NPsel) {                        \
-    case 1: SONG_HEADS(M, 1); break;      \
-    case 2: SONG_HEADS(M, 2); break;      \
-    case 4: SONG_HEADS(M, 4); break;      \
-    default: SONG_HEADS(M, 8); break;     \
-  }
-#define SONG_CLUSTERS_BY_NS(M)            \
-  switch (NSel) {                         \
-    case 1: SONG_CLUSTERS(M, 1); break;   \
-    case 2: SONG_CLUSTERS(M, 2); break;   \
-    case 4: SONG_CLUSTERS(M, 4); break;   \
-    default: SONG_CLUSTERS(M, 8); break;  \
-  }
+#define SONG_HEADS_L2(NP) SONG_HEADS(SONG_METRIC_L2, NP)
+#define SONG_HEADS_IP(NP) SONG_HEADS(SONG_METRIC_IP, NP)
+#define SONG_HEADS_COS(NP) SONG_HEADS(SONG_METRIC_COS, NP)
+#define SONG_CLUSTERS_L2(NS) SONG_CLUSTERS(SONG_METRIC_L2, NS)
+#define SONG_CLUSTERS_IP(NS) SONG_CLUSTERS(SONG_METRIC_IP, NS)
+#define SONG_CLUSTERS_COS(NS) SONG_CLUSTERS(SONG_METRIC_COS, NS)
   if (heads_mma_usable(ix, queries, np)) {  // tensor-core scores, exact re-scoring of a shortlist
     if ((e = launch_heads_mma(ix, queries, nq, np, probes, s)) != cudaSuccess) return e;
   } else {
     switch (ix->dx.metric) {
-      case SONG_METRIC_L2: SONG_HEADS_BY_NP(SONG_METRIC_L2); break;
-      case SONG_METRIC_IP: SONG_HEADS_BY_NP(SONG_METRIC_IP); break;
-      default: SONG_HEADS_BY_NP(SONG_METRIC_COS); break;
+      case SONG_METRIC_L2: SONG_BY_LEN(NPsel, SONG_HEADS_L2); break;
+      case SONG_METRIC_IP: SONG_BY_LEN(NPsel, SONG_HEADS_IP); break;
+      default: SONG_BY_LEN(NPsel, SONG_HEADS_COS); break;
     }
   }
-  cluster_scan_kernel<<<1, 1024, 0, s>>>(ix->d_cl_count, coarse, ix->d_cl_order, q_offs, cursor, task_offs);
+  cluster_scan_kernel<<<1, 1024, 0, s>>>(ix->d_cl_count, coarse, ix->d_cl_order, q_offs, cursor, task_offs,
+                                         n_tasks);
   cluster_scatter_kernel<<<static_cast<unsigned>(std::min<size_t>((pairs + 255) / 256, 4096)), 256, 0, s>>>(
-      probes, static_cast<int>(pairs), cursor, q_list);
+      probes, static_cast<int>(pairs), q_offs, task_offs, cursor, q_list, tasks);
   switch (ix->dx.metric) {
-    case SONG_METRIC_L2: SONG_CLUSTERS_BY_NS(SONG_METRIC_L2); break;
-    case SONG_METRIC_IP: SONG_CLUSTERS_BY_NS(SONG_METRIC_IP); break;
-    default: SONG_CLUSTERS_BY_NS(SONG_METRIC_COS); break;
+    case SONG_METRIC_L2: SONG_BY_LEN(NSel, SONG_CLUSTERS_L2); break;
+    case SONG_METRIC_IP: SONG_BY_LEN(NSel, SONG_CLUSTERS_IP); break;
+    default: SONG_BY_LEN(NSel, SONG_CLUSTERS_COS); break;
   }
-#undef SONG_CLUSTERS_BY_NS
-#undef SONG_HEADS_BY_NP
+#undef SONG_CLUSTERS_L2
+#undef SONG_CLUSTERS_IP
+#undef SONG_CLUSTERS_COS
+#undef SONG_HEADS_L2
+#undef SONG_HEADS_IP
+#undef SONG_HEADS_COS
 #undef SONG_CLUSTERS
 #undef SONG_HEADS
   return cudaGetLastError();
@@ -880,11 +820,10 @@ int prepare_starts(song_index *ix, SearchCall &c, cudaStream_t s) {
     if (e != cudaSuccess) return fail(SONG_ERR_OOM, "entry starts: %s", cudaGetErrorString(e));
     ix->cap_starts = need;
   }
-  const int dim = ix->dx.dim, dpad = static_cast<int>(ix->dx.f32_row_bytes / 4);
   const cudaError_t le =
       ix->n_coarse > 0 ? launch_2level(ix, c.queries, c.nq, ix->d_starts, s)
-                       : launch_nearest(c.queries, c.nq, dim, dim, dpad, ix->dx.metric, ix->d_entry_rows,
-                                        ix->d_entry_ids, ix->n_entries, ix->n_starts, ix->d_starts, s);
+                       : launch_nearest(ix, c.queries, c.nq, ix->dx.dim, ix->d_entry_rows, ix->d_entry_ids,
+                                        ix->n_entries, ix->n_starts, ix->d_starts, s);
   if (le != cudaSuccess) return fail(SONG_ERR_CUDA, "entry launch: %s", cudaGetErrorString(le));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(SONG_ERR_CUDA, "entry launch: %s", cudaGetErrorString(e));
@@ -954,7 +893,7 @@ extern "C" int song_index_set_entries_2level(song_index *ix, const uint64_t *ids
   if (probes < 1 || probes > SONG_MAX_STARTS || probes > coarse)
     return fail(SONG_ERR_ARG, "probes must be 1..min(%d, coarse)", SONG_MAX_STARTS);
   if (starts < 1 || starts > probes) return fail(SONG_ERR_ARG, "starts must be 1..probes");
-  const int dim = ix->dx.dim, dpad = static_cast<int>(ix->dx.f32_row_bytes / 4);
+  const int dpad = static_cast<int>(ix->dx.f32_row_bytes / 4);
   // the smallest block shape (one warp, 4 queries, one tile of 8 rows) fits
   // a block's shared memory
   auto fits = [](int dp) { return TileShape{1, 8, 1}.smem(dp) <= 227u * 1024u; };
@@ -992,8 +931,8 @@ extern "C" int song_index_set_entries_2level(song_index *ix, const uint64_t *ids
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && count > coarse)
-    e = launch_nearest(d_rows + static_cast<size_t>(coarse) * dpad, count - coarse, dpad, dim, dpad, ix->dx.metric,
-                       d_rows, d_ids, coarse, 1, d_assign, ix->stream);
+    e = launch_nearest(ix, d_rows + static_cast<size_t>(coarse) * dpad, count - coarse, dpad, d_rows, d_ids, coarse, 1,
+                       d_assign, ix->stream);
   if (e == cudaSuccess && count > coarse)
     e = cudaMemcpyAsync(assign.data(), d_assign, sizeof(uint32_t) * (count - coarse), cudaMemcpyDeviceToHost,
                         ix->stream);

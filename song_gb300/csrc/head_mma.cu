@@ -38,6 +38,7 @@
 #include <cstring>
 
 #include "device_common.cuh"
+#include "entry_rows.cuh"
 #include "internal.h"
 #include "song_gb300.h"
 
@@ -209,53 +210,6 @@ __device__ __forceinline__ void warp_take(const float (&bd)[N], const uint32_t (
     }
   }
   if (id == wid && d == wd && id != 0xffffffffu) ++h;
-}
-
-// Exact search distance (lane-strided FMA chain over dims, xor butterfly) of
-// the query to R head rows at once (R = 8 or 32): row r is rows + idx(r) *
-// dpad; lane l returns row l / (32 / R)'s distance.  Products taken two rows
-// at a time through the paired FP32 instructions (the scalar roundings, in
-// the scalar order); the R rows meet in one transposed butterfly.
-template <int METRIC, int R, class Idx>
-__device__ __forceinline__ float rows_distance(const float *qv, int dim, const float *rows, int dpad, Idx idx,
-                                               int lane) {
-  constexpr bool COS = METRIC == SONG_METRIC_COS;
-  constexpr int P = R / 2;
-  uint64_t acc[P], ln[P];
-#pragma unroll
-  for (int p = 0; p < P; ++p) acc[p] = ln[p] = 0ull;
-  for (int j = lane; j < dim; j += 32) {
-    const float qj = qv[j];
-    const uint64_t qq = f2_pack(qj, qj);
-#pragma unroll
-    for (int p = 0; p < P; ++p) {
-      const float x0 = __ldg(rows + static_cast<size_t>(idx(2 * p)) * dpad + j);
-      const float x1 = __ldg(rows + static_cast<size_t>(idx(2 * p + 1)) * dpad + j);
-      const uint64_t xx = f2_pack(x0, x1);
-      if (METRIC == SONG_METRIC_L2) {
-        const uint64_t df = f2_sub(qq, xx);
-        acc[p] = f2_fma(df, df, acc[p]);
-      } else {
-        acc[p] = f2_fma(qq, xx, acc[p]);
-        if (COS) ln[p] = f2_fma(xx, xx, ln[p]);
-      }
-    }
-  }
-  float v[R];
-#pragma unroll
-  for (int p = 0; p < P; ++p) f2_unpack(acc[p], v[2 * p], v[2 * p + 1]);
-  const float t = butterfly_rows<R>(v, lane);
-  if (METRIC == SONG_METRIC_L2) return t;
-  if (METRIC == SONG_METRIC_IP) return -t;
-  float lv[R];
-#pragma unroll
-  for (int p = 0; p < P; ++p) f2_unpack(ln[p], lv[2 * p], lv[2 * p + 1]);
-  const float len = butterfly_rows<R>(lv, lane);
-  if (len != 0.0f) {
-    const float sign = t < 0.0f ? 1.0f : -1.0f;
-    return __fdiv_rn(__fmul_rn(__fmul_rn(sign, t), t), len);
-  }
-  return 0.0f;
 }
 
 // ---- step 1: tensor-core scores, intervals in the epilogue ------------------
@@ -457,16 +411,20 @@ __global__ void __launch_bounds__(128, 1)
 // rows x tiles x NP.  stats (or null): [0] queries, [1] heads re-scored, [2]
 // full scans.
 template <int METRIC, int NP>
-__global__ void __launch_bounds__(HM_SEL_WARPS * 32)
+__global__ void __launch_bounds__(HM_SEL_WARPS * 32, 3)
     head_select_kernel(const float *queries, int dim, int q_row0, int rows, const uint16_t *lo16, int ld,
                        const float *tile_hi, int tiles, const float *heads, int dpad, int n_heads, int probes,
                        uint32_t *probe_out, uint32_t *cl_count, unsigned long long *stats) {
   __shared__ uint32_t cand[HM_SEL_WARPS][HM_CAP];
+  extern __shared__ __align__(16) float staged[];  // a query per warp, zero-padded to qs floats
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = blockIdx.x * HM_SEL_WARPS + w;
+  const int r = blockIdx.x * (blockDim.x >> 5) + w;
   if (r >= rows) return;  // whole warp
   const int q = q_row0 + r;
-  const float *qv = queries + static_cast<size_t>(q) * dim;
+  const int qs = (dpad + 31) & ~31;
+  float *qv = staged + static_cast<size_t>(w) * qs;
+  for (int j = lane; j < qs; j += 32) qv[j] = j < dim ? __ldg(queries + static_cast<size_t>(q) * dim + j) : 0.0f;
+  __syncwarp();
 
   // U = the probes-th smallest upper bound over all heads: the tiles' lists
   // hold every head's bound that can be among them
@@ -529,36 +487,16 @@ __global__ void __launch_bounds__(HM_SEL_WARPS * 32)
   // finite, e.g. after a timed-out score kernel: scan everything then too)
   const bool full_scan = count > HM_CAP || count < probes;
   const int total = full_scan ? n_heads : count;
-  // 32 rows per pass, the last few (the common shortlist of a handful of
-  // heads) 8 at a time: a pass reads every one of its rows
-  for (int g = 0; g < total;) {
-    const int left = total - g;
-    if (left > 8) {
-      const int n = min(32, left);
-      float d;
-      if (full_scan) {
-        d = rows_distance<METRIC, 32>(qv, dim, heads, dpad, [&](int i) { return min(g + i, n_heads - 1); }, lane);
-      } else {
-        const uint32_t *cl = cand[w] + g;
-        d = rows_distance<METRIC, 32>(qv, dim, heads, dpad, [&](int i) { return cl[min(i, n - 1)]; }, lane);
-      }
-      if (lane < n) best_insert<NP>(bd, bi, d, full_scan ? static_cast<uint32_t>(g + lane) : cand[w][g + lane]);
-      g += n;
-    } else {
-      const int n = left;
-      float d;
-      if (full_scan) {
-        d = rows_distance<METRIC, 8>(qv, dim, heads, dpad, [&](int i) { return min(g + i, n_heads - 1); }, lane);
-      } else {
-        const uint32_t *cl = cand[w] + g;
-        d = rows_distance<METRIC, 8>(qv, dim, heads, dpad, [&](int i) { return cl[min(i, n - 1)]; }, lane);
-      }
-      const int row = lane >> 2;  // lane l holds row l / 4
-      if ((lane & 3) == 0 && row < n)
-        best_insert<NP>(bd, bi, d, full_scan ? static_cast<uint32_t>(g + row) : cand[w][g + row]);
-      g += n;
-    }
+  // eight rows a pass, four lanes a row (the common shortlist is a handful);
+  // the first lane of a row keeps it
+  for (int g = 0; g < total; g += 8) {
+    const int i = min(g + (lane >> 2), total - 1);
+    const uint32_t head = full_scan ? static_cast<uint32_t>(i) : cand[w][i];
+    float d[1];
+    rows8_distance<METRIC, 1>(heads + static_cast<size_t>(head) * dpad, qv, qs, dpad, d, lane);
+    if (g + (lane >> 2) < total && (lane & 3) == 0) best_insert<NP>(bd, bi, d[0], head);
   }
+  __syncwarp();
   int hp = 0;
   for (int k = 0; k < probes; ++k) {
     float wd;
@@ -631,7 +569,13 @@ cudaError_t launch_chunk(const CUtensorMap &tq, const CUtensorMap &th, HeadScore
   const int tiles = (a.n_heads + HM_B - 1) / HM_B;
   kern<<<dim3((a.rows + HM_B - 1) / HM_B, tiles), 128, HM_SMEM, s>>>(tq, th, a);
   const int dpad = static_cast<int>(ix->dx.f32_row_bytes / 4);
-  head_select_kernel<METRIC, NP><<<(a.rows + HM_SEL_WARPS - 1) / HM_SEL_WARPS, HM_SEL_WARPS * 32, 0, s>>>(
+  // fewer warps a block for wide queries, so that the staged queries fit
+  const int qbytes = 4 * ((dpad + 31) & ~31);
+  const int sw = std::max(1, std::min(HM_SEL_WARPS, 32 * 1024 / qbytes));
+  auto select = head_select_kernel<METRIC, NP>;
+  e = cudaFuncSetAttribute(select, cudaFuncAttributeMaxDynamicSharedMemorySize, sw * qbytes);
+  if (e != cudaSuccess) return e;
+  select<<<(a.rows + sw - 1) / sw, sw * 32, static_cast<size_t>(sw) * qbytes, s>>>(
       queries, ix->dx.dim, a.q_row0, a.rows, a.lo16, a.ld, a.tile_hi, tiles, ix->d_coarse_rows, dpad, ix->n_coarse,
       np, probe_out, ix->d_cl_count, ix->head_stats_on ? ix->d_head_stats : nullptr);
   return cudaGetLastError();
