@@ -569,14 +569,15 @@ cudaError_t entry_work(song_index *ix, size_t words) {
     default: CALL(8); break;  \
   }
 
-// Batches that take the two-kernel choice: up to 512 queries, and up to 2^28
-// query x head x dimension products (1M x 128, 4096 heads: 68 against 96 us at
-// 257 queries, 112 against 109 at 512; 960-d rows, 1024 heads: 230 against
-// 323 at 257, 355 against 349 at 600); with few short heads, 2^22 products
-// (15k x 16, 128 heads: 44 against 94 us at 1000 queries).
+// Batches that take the two-kernel choice: up to 512 queries (1M x 128, 4096
+// heads: 68 against 96 us at 257 queries, 112 against 109 at 512; 960-d rows,
+// 1024 heads: 230 against 323 at 257, 355 against 349 at 600; 256-d rows, 126
+// against 128 at 500), within 2^29 query x head x dimension products; with few
+// short heads, 2^22 products (15k x 16, 128 heads: 44 against 94 us at 1000
+// queries).
 bool small_batch(int nq, int coarse, int dpad) {
   const double work = static_cast<double>(nq) * coarse * dpad;
-  return (nq <= 512 && work <= 268435456.0) || work <= 4194304.0;
+  return (nq <= 512 && work <= 536870912.0) || work <= 4194304.0;
 }
 
 // The NP nearest of n rows for each of nq queries, chunk by chunk: *chunks

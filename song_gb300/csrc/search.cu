@@ -88,6 +88,28 @@ int get_shape(const void *fn, uint32_t warp_bytes, uint32_t extra, int *wpb, int
   return 0;
 }
 
+int get_team_shape(const void *fn, uint32_t bytes, int *grid_cap) {
+  std::lock_guard<std::mutex> lk(g_shape_mu);
+  int dev = 0;
+  cudaGetDevice(&dev);
+  for (const Shape &s : g_shapes)
+    if (s.fn == fn && s.dev == dev && s.warp_bytes == bytes && s.extra == 0) {
+      *grid_cap = s.blocks_per_sm * s.sms;
+      return 0;
+    }
+  int sms = 0, optin = 0, per_sm = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (bytes <= static_cast<uint32_t>(optin)) {
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * TEAM_WARPS, bytes);
+    if (e != cudaSuccess) return e;
+  }
+  g_shapes.push_back(Shape{fn, dev, bytes, 0, TEAM_WARPS, per_sm, sms});
+  *grid_cap = per_sm * sms;
+  return 0;
+}
+
 // What a warp may need, as the interface states it: two staging chunks of
 // the rows beside the query and the 8*pq-slot hash.  The kernel needs less,
 // at every size that this admits.

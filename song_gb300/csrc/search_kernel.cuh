@@ -20,7 +20,8 @@
 //  * each hop's unvisited neighbour rows are read straight from global memory
 //    into registers, eight rows at a time, four lanes a row (gather_rows);
 //  * one hop's visited-hash calls run one lane each (visited_update);
-//  * the next hop's adjacency row is loaded as soon as the next pop is known.
+//  * the next hop's adjacency row is loaded as soon as the next pop is known;
+//  * batches that fit the GPU a block per query get one (Team).
 //
 // Template parameters: METRIC (0 L2, 1 IP, 2 COS), STORAGE (0 F32, 1 BF16,
 // 2 FP8-E4M3 with a per-row scale, 3 256-bit codes), S (register queue
@@ -120,57 +121,65 @@ struct Code8 {
   uint32_t w[8];
 };
 
-// Distances of candidates 0..m-1 (candidate c's id in lane c) in lane c;
-// qv: the query, zero-padded to a multiple of 32 floats.  `width` elements a
-// row (zero-padded to the 16-byte load; a padded element adds fma(0, 0, t)).
+// One pass: the distance of the row of vertex `id` (the same in a row's four
+// lanes), in those lanes.  qv: the query, zero-padded to a multiple of 32
+// floats.  `width` elements a row (zero-padded to the 16-byte load; a padded
+// element adds fma(0, 0, t)).
 template <int METRIC, int STORAGE>
-__device__ __forceinline__ float gather_rows(const uint8_t *rows, uint32_t rb, uint32_t scale_off, int width,
-                                             const float *qv, int m, uint32_t cid, int lane) {
+__device__ __forceinline__ float rows_pass(const uint8_t *rows, uint32_t rb, uint32_t scale_off, int width,
+                                           const float *qv, uint32_t id, int lane) {
   using Read = RowRead<STORAGE>;
   const int g = lane & 3;
   const ulonglong2 *q2 = reinterpret_cast<const ulonglong2 *>(qv) + (Read::HALVES ? g : 2 * g);
   constexpr int QB = Read::HALVES ? 4 : 1;  // the second half's offset in 16-byte units
+  const uint8_t *row = rows + static_cast<uint64_t>(id) * rb;
+  const float scale = STORAGE == 2 ? __ldg(reinterpret_cast<const float *>(row + scale_off)) : 1.0f;
+  uint64_t acc[4], len[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[i] = len[i] = 0ull;
+  auto add = [&](const Read &r, int j) {
+    uint64_t x[4];
+    r.get(x, scale);
+    const ulonglong2 qa = q2[j >> 2], qb = q2[(j >> 2) + QB];
+    const uint64_t q[4] = {qa.x, qa.y, qb.x, qb.y};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (METRIC == 0) {
+        const uint64_t d = f2_sub(q[i], x[i]);
+        acc[i] = f2_fma(d, d, acc[i]);
+      } else {
+        acc[i] = f2_fma(q[i], x[i], acc[i]);
+        if (METRIC == 2) len[i] = f2_fma(x[i], x[i], len[i]);
+      }
+    }
+  };
+  int j = 0;
+  constexpr int U = STORAGE == 0 ? 4 : 8;  // 32-dimension steps in flight: 16 (FP8) to 32 registers
+  for (; j + 32 * U <= width; j += 32 * U) {
+    Read r[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i) r[i].load_full(row, j + 32 * i, g);
+#pragma unroll
+    for (int i = 0; i < U; ++i) add(r[i], j + 32 * i);
+  }
+  for (; j < width; j += 32) {
+    Read r;
+    r.load(row, j, g, width);
+    add(r, j);
+  }
+  const float t = row_butterfly<Read::HALVES>(acc, lane);
+  const float ln = METRIC == 2 ? row_butterfly<Read::HALVES>(len, lane) : 0.0f;
+  return finish_distance<METRIC>(t, ln);
+}
+
+// Distances of candidates 0..m-1 (candidate c's id in lane c) in lane c.
+template <int METRIC, int STORAGE>
+__device__ __forceinline__ float gather_rows(const uint8_t *rows, uint32_t rb, uint32_t scale_off, int width,
+                                             const float *qv, int m, uint32_t cid, int lane) {
   float out = 0.0f;
   for (int first = 0; first < m; first += 8) {
     const uint32_t id = __shfl_sync(FULL, cid, min(first + (lane >> 2), m - 1));
-    const uint8_t *row = rows + static_cast<uint64_t>(id) * rb;
-    const float scale = STORAGE == 2 ? __ldg(reinterpret_cast<const float *>(row + scale_off)) : 1.0f;
-    uint64_t acc[4], len[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i] = len[i] = 0ull;
-    auto add = [&](const Read &r, int j) {
-      uint64_t x[4];
-      r.get(x, scale);
-      const ulonglong2 qa = q2[j >> 2], qb = q2[(j >> 2) + QB];
-      const uint64_t q[4] = {qa.x, qa.y, qb.x, qb.y};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (METRIC == 0) {
-          const uint64_t d = f2_sub(q[i], x[i]);
-          acc[i] = f2_fma(d, d, acc[i]);
-        } else {
-          acc[i] = f2_fma(q[i], x[i], acc[i]);
-          if (METRIC == 2) len[i] = f2_fma(x[i], x[i], len[i]);
-        }
-      }
-    };
-    int j = 0;
-    constexpr int U = STORAGE == 0 ? 4 : 8;  // 32-dimension steps in flight: 16 (FP8) to 32 registers
-    for (; j + 32 * U <= width; j += 32 * U) {
-      Read r[U];
-#pragma unroll
-      for (int i = 0; i < U; ++i) r[i].load_full(row, j + 32 * i, g);
-#pragma unroll
-      for (int i = 0; i < U; ++i) add(r[i], j + 32 * i);
-    }
-    for (; j < width; j += 32) {
-      Read r;
-      r.load(row, j, g, width);
-      add(r, j);
-    }
-    const float t = row_butterfly<Read::HALVES>(acc, lane);
-    const float ln = METRIC == 2 ? row_butterfly<Read::HALVES>(len, lane) : 0.0f;
-    const float d = finish_distance<METRIC>(t, ln);
+    const float d = rows_pass<METRIC, STORAGE>(rows, rb, scale_off, width, qv, id, lane);
     const float mine = __shfl_sync(FULL, d, ((lane - first) & 7) * 4);
     if (lane >= first && lane < first + 8) out = mine;
   }
@@ -303,6 +312,88 @@ struct WarpCtx {
   }
 };
 
+// Small batches leave most of the GPU idle, and a query's time is the latency
+// of one warp's hops.  There a query gets a block of TEAM_WARPS warps: warp 0
+// runs the search, the others wait for its commands at a named barrier --
+// take your eight of a hop's candidates (the passes of one gather then run
+// side by side), or fetch into L2 the rows that the next vertex's neighbours
+// name (they arrive while warp 0 takes in this hop's candidates).  Search
+// alone, 1M x 128 from entry points: one query at pq 100 375 -> 307 us, 300 at
+// pq 43 257 -> 174; 300 of 60k x 960 at pq 75 652 -> 338; 15k x 16, whose rows
+// never leave L2, within 3 % either way.
+constexpr int TEAM_WARPS = 4;
+constexpr uint32_t TEAM_BYTES = 256;  // commands and distances
+
+struct Team {
+  int32_t *cmd;   // two slots of (command, argument), used in turn
+  float *dist;    // distances of one gather
+  int turn;
+  static constexpr int STOP = 0, PREFETCH = -1;  // > 0: gather that many
+
+  __device__ __forceinline__ void init(uint8_t *mem) {
+    cmd = reinterpret_cast<int32_t *>(mem);
+    dist = reinterpret_cast<float *>(mem + 128);
+    turn = 0;
+  }
+  static __device__ __forceinline__ void barrier() {
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * TEAM_WARPS) : "memory");
+  }
+  // Warp 0: hands out a command.
+  __device__ __forceinline__ void call(int c, int arg, int lane) {
+    if (lane == 0) {
+      cmd[2 * turn] = c;
+      cmd[2 * turn + 1] = arg;
+    }
+    __syncwarp();
+    barrier();
+    turn ^= 1;
+  }
+  // The others: waits for a command.
+  __device__ __forceinline__ int next(int *arg) {
+    barrier();
+    const int c = cmd[2 * turn];
+    *arg = cmd[2 * turn + 1];
+    turn ^= 1;
+    return c;
+  }
+};
+
+// Warp `wib`'s share of a gather: candidates 8 wib .. of the m listed in cbuf.
+template <int METRIC, int STORAGE>
+__device__ __forceinline__ void team_pass(const Params &p, const WarpCtx &w, const Team &t, int m, int wib, int lane) {
+  const int c = 8 * wib + (lane >> 2);
+  if (8 * wib >= m) return;  // whole warp
+  const float d = rows_pass<METRIC, STORAGE>(p.rows, p.row_bytes, p.scale_off, p.width, w.qv, w.cbuf[min(c, m - 1)],
+                                             lane);
+  if ((lane & 3) == 0 && c < m) t.dist[c] = d;
+}
+
+template <int METRIC, int STORAGE>
+__device__ __forceinline__ void team_help(const Params &p, const WarpCtx &w, Team t, int wib, int lane) {
+  const VisitedHash vh = VisitedOf<false>::make(w.tab, p.pq);
+  for (;;) {
+    int arg;
+    const int c = t.next(&arg);
+    if (c == Team::STOP) return;
+    if (c > 0) {
+      team_pass<METRIC, STORAGE>(p, w, t, c, wib, lane);
+      Team::barrier();
+      continue;
+    }
+    // the visited table may be changing under this look: it only decides what
+    // is worth fetching
+    const uint32_t *adj = p.adj + (static_cast<uint64_t>(static_cast<uint32_t>(arg)) << p.shift);
+    const uint32_t a = lane < (1 << p.shift) ? __ldg(adj + lane) : 0u;
+    const int deg = static_cast<int>(__shfl_sync(FULL, a, 0));
+    if (lane >= 1 && lane <= deg && !vh.test(a)) {
+      const uint8_t *row = p.rows + static_cast<uint64_t>(a) * p.row_bytes;
+      for (uint32_t b = 128u * (wib - 1); b < p.row_bytes; b += 128u * (TEAM_WARPS - 1))
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(row + b));
+    }
+    __syncwarp();
+  }
+}
+
 struct QueryStats {
   int hops, evals, version;
 };
@@ -348,10 +439,10 @@ __device__ __forceinline__ void select_insert(Queue &Q, VH &vh, int m, uint64_t 
 // (LEARNED) receives the per-hop features or is null.  False if a bulk copy
 // never completed.  MULTI: the reference's N_MULTIPROBE / FINISH_CNT knobs
 // (p.probes, p.finish_cnt) as run-time values.
-template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false>
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false, bool TEAM = false>
 __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const float *qsrc, const uint32_t *starts,
                                           int ns, int pq, int k, uint64_t *o, float *trace, QueryStats &st,
-                                          int lane, const uint32_t *qcode = nullptr) {
+                                          int lane, const uint32_t *qcode = nullptr, Team *team = nullptr) {
   Code8 qc;
 #pragma unroll
   for (int i = 0; i < 8; ++i) qc.w[i] = STORAGE == 3 ? qcode[i] : 0u;
@@ -555,7 +646,17 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
     const uint32_t cid = lane < m ? w.cbuf[lane] : 0u;
     const int chome = lane < m ? w.chome[lane] : 0;
     // :237-287 distances.
-    cd = gather_distances<METRIC, STORAGE>(p, w.qv, m, cid, lane, qc);
+    bool shared = false;
+    if constexpr (TEAM) {
+      shared = m > 8;
+      if (shared) {
+        team->call(m, 0, lane);
+        team_pass<METRIC, STORAGE>(p, w, *team, m, 0, lane);
+        Team::barrier();
+        cd = lane < m ? team->dist[lane] : 0.0f;
+      }
+    }
+    if (!shared) cd = gather_distances<METRIC, STORAGE>(p, w.qv, m, cid, lane, qc);
     evals += m;
     // The next vertex popped is the smaller of the queue head and the best
     // candidate (the select-insert rule can only reject candidates above a
@@ -567,6 +668,7 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
     if (nk != ~0ull) {
       next_id = key_id(nk);
       a_next = adjacency(next_id);
+      if constexpr (TEAM) team->call(Team::PREFETCH, static_cast<int>(next_id), lane);
     }
     select_insert(Q, vh, m, ck, chome, pq, qn, lane);
     if constexpr (LEARNED) {
@@ -704,6 +806,38 @@ __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, MinBlocks<S>::value)
   }
 }
 
+// The search with a block per query (Team).
+template <int METRIC, int STORAGE, int S>
+__global__ void __launch_bounds__(TEAM_WARPS * 32, S > 16 ? 2 : 4) search_team_kernel(const Params p) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  WarpCtx w;
+  w.init(smem_raw, p, 32, wib == 0 ? lane : 1);  // lane 0 of warp 0 sets the barrier up
+  w.wmlp = nullptr;
+  Team team;
+  team.init(smem_raw + p.warp_bytes);
+  if (wib > 0) {
+    team_help<METRIC, STORAGE>(p, w, team, wib, lane);
+    return;
+  }
+  for (int qid = blockIdx.x; qid < p.nq; qid += gridDim.x) {
+    QueryStats st;
+    if (!run_query<METRIC, STORAGE, S, false, false, true>(
+            p, w, p.queries + static_cast<size_t>(qid) * p.dim,
+            p.starts ? p.starts + static_cast<size_t>(qid) * p.n_starts : nullptr, p.n_starts, p.pq, p.k,
+            p.out + static_cast<size_t>(qid) * p.k, nullptr, st, lane, nullptr, &team)) {
+      if (lane == 0) atomicOr(p.error, 1);
+      break;
+    }
+    if (lane == 0) {
+      if (p.hops) p.hops[qid] = st.hops;
+      if (p.evals) p.evals[qid] = st.evals;
+    }
+    __syncwarp();
+  }
+  team.call(Team::STOP, 0, lane);
+}
+
 // ---------------------------------------------------------------------------
 // Host-side launch helpers shared by the per-storage translation units.
 // ---------------------------------------------------------------------------
@@ -711,9 +845,22 @@ __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, MinBlocks<S>::value)
 // Launch shape per (kernel, bytes per block): warps per block in {4, 2, 1}
 // that keeps the most warps resident per SM (search.cu).
 int get_shape(const void *fn, uint32_t warp_bytes, uint32_t extra_bytes, int *wpb, int *grid_cap);
+// The same for blocks of a fixed size and footprint: how many fit on the GPU.
+int get_team_shape(const void *fn, uint32_t bytes, int *grid_cap);
 
 template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false>
 int launch_kernel(const Params &p, cudaStream_t stream) {
+  if constexpr (STORAGE != 3 && !LEARNED && !MULTI) {
+    // a block per query while all of them run at once
+    auto team = search_team_kernel<METRIC, STORAGE, S>;
+    const uint32_t bytes = p.warp_bytes + TEAM_BYTES;
+    int cap = 0;
+    int e = get_team_shape(reinterpret_cast<const void *>(team), bytes, &cap);
+    if (e == 0 && p.nq <= cap) {
+      team<<<p.nq, TEAM_WARPS * 32, bytes, stream>>>(p);
+      return cudaGetLastError();
+    }
+  }
   auto kern = search_kernel<METRIC, STORAGE, S, LEARNED, MULTI>;
   const uint32_t extra = LEARNED ? static_cast<uint32_t>(MLP_NPARAM * sizeof(__nv_bfloat16) + 64) : 0u;
   int wpb = 0, cap = 0;

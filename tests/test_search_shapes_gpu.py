@@ -2,7 +2,8 @@
 the ends of each queue segment and of the two queue kinds, row widths at the
 remainders of the gather (every format), and ids laid out so that the visited
 hash has long runs (consecutive ids hash to neighbouring slots) across its
-end.  Bit-exact against the oracle (ids, hops, evaluations)."""
+end.  Bit-exact against the oracle (ids, hops, evaluations), in a small batch
+(a block per query) and in one of some thousand queries (a warp per query)."""
 import numpy as np
 import pytest
 
@@ -33,6 +34,15 @@ def _ring_graph(song, data, metric, shift, seed):
     return g
 
 
+def _check(ix, q, pq, oracle_result, what):
+    o_ids, o_hops, o_evals, _ = oracle_result
+    for reps in (1, 100):
+        ids, hops, evals = ix.search(np.tile(q, (reps, 1)), pq, pq, stats=True)
+        assert np.array_equal(ids, np.tile(o_ids, (reps, 1))), (what, reps)
+        assert np.array_equal(hops, np.tile(o_hops, reps)), (what, reps)
+        assert np.array_equal(evals, np.tile(o_evals, reps)), (what, reps)
+
+
 PQS = [2, 3, 30, 31, 32, 62, 63, 64, 126, 127, 128, 254, 255, 256, 510, 511, 512, 1022, 1023]
 
 
@@ -44,10 +54,9 @@ def test_queue_bounds(song, oracle, metric, shift):
     ox = oracle.OracleIndex(data, g, shift, metric)
     with song.Index(g, data, shift, metric) as ix:
         for pq in PQS:
-            ids, hops, evals = ix.search(q, pq, pq, stats=True)
-            o_ids, o_hops, o_evals, _ = ox.kernel_search(q, pq, oracle.MODE_LEX)
-            assert np.array_equal(ids, o_ids), "pq %d" % pq
-            assert np.array_equal(hops, o_hops) and np.array_equal(evals, o_evals), "pq %d" % pq
+            want = ox.kernel_search(q, pq, oracle.MODE_LEX)
+            _check(ix, q, pq, want, pq)
+            o_ids = want[0]
             for k in (1, min(pq, 32), min(pq, 33)):
                 assert np.array_equal(ix.search(q, pq, k), o_ids[:, :k]), "pq %d k %d" % (pq, k)
 
@@ -60,8 +69,5 @@ def test_row_widths(song, oracle, dim):
         for storage in ("f32", "bf16", "fp8"):
             with song.Index(g, data, 5, metric, storage=storage) as ix:
                 ix.set_rerank(0)
-                ids, hops, evals = ix.search(q, 40, 40, stats=True)
                 ox = oracle.OracleIndex(song.dequantize_rows(ix.rows(), storage, dim), g, 5, metric)
-                o_ids, o_hops, o_evals, _ = ox.kernel_search(q, 40, oracle.MODE_LEX)
-                assert np.array_equal(ids, o_ids), (metric, storage)
-                assert np.array_equal(hops, o_hops) and np.array_equal(evals, o_evals), (metric, storage)
+                _check(ix, q, 40, ox.kernel_search(q, 40, oracle.MODE_LEX), (metric, storage))
