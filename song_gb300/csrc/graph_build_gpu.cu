@@ -22,12 +22,15 @@
 // could only ever be popped to end the search, which the next larger queue
 // entry (or an empty queue) does just the same.
 //
-// One lane per candidate computes its distance (the double sum must run in
-// dimension order); lane 0 keeps the two heaps.  Per warp: the result list
-// and the query row in shared memory, the visited set (open addressing,
-// insert-only, atomicCAS) and the queue heap in a device scratch region whose
-// size is checked; a search that would overflow it flags the batch, which the
-// host repeats with larger regions.
+// Two kernels do it.  beam_search_kernel (budgets up to BEAM_BUDGET) keeps
+// queue and result list as one sorted list and sums the distances of a row
+// over the whole warp, in integers where that is exact (below).  A batch it
+// cannot finish (more equal distances at the list's end than its list holds)
+// and larger budgets take build_search_kernel, which follows the CPU search
+// step by step: one lane per candidate, lane 0 keeping the two heaps, the
+// visited set and the queue heap in a device scratch region whose size is
+// checked; a search that would overflow it flags the batch, which the host
+// repeats with larger regions.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -291,6 +294,295 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) build_search_kernel(const Bu
   }
 }
 
+// ---------------------------------------------------------------------------
+// The search with one sorted list.
+//
+// The list holds queued and popped vertices together, ordered by (distance,
+// id), each with a flag.  The next pop is its first vertex not popped.  A
+// vertex with `budget` or more listed vertices strictly below it can be
+// dropped: those below it pop first, and the result list is then full with
+// a maximum below it, which is the stop rule.  So the list keeps its first
+// `budget` vertices and those at the distance of the last of them, the search
+// ends when all of them are popped, and they are the result list.
+//
+// Distances.  The CPU adds the products (floats) in double, in dimension
+// order.  A product is M * 2^(e - 150) with a 24-bit M; with E the largest e
+// of a row's products, M << (e - E + K) is an integer when no nonzero product
+// lies more than K binades below the largest, and with dim * 2^(24 + K) <=
+// 2^53 every partial sum, in any order, is such an integer that a double
+// holds exactly.  So the sum is the CPU's whatever the order: a warp takes a
+// row's dimensions side by side and adds in 64-bit integers (the GB300 adds
+// two FP64 lanes a clock per SM).  Rows that fail the test (a wide range of
+// products, infinities, NaNs, denormal products) are summed in dimension
+// order, one lane each.
+// ---------------------------------------------------------------------------
+
+constexpr int BEAM_CAP = 256;     // list places
+constexpr int BEAM_BUDGET = 192;  // largest budget
+constexpr int BEAM_VIS_LOG2 = 13; // visited slots in shared memory (a block per vertex)
+
+struct BeamList {
+  uint64_t d[BEAM_CAP];   // order-preserving bits of the distance
+  uint32_t w[BEAM_CAP];   // id << 1 | popped
+};
+
+__device__ __forceinline__ uint64_t ordered(double d) {
+  if (d == 0.0) d = 0.0;  // -0 and +0 compare equal
+  const uint64_t u = static_cast<uint64_t>(__double_as_longlong(d));
+  return (u >> 63) ? ~u : (u | (1ull << 63));
+}
+
+// A row's products summed as integers: the sum and the largest exponent, the
+// same in all lanes; false when the sum is not exact.  K: see above.
+__device__ __forceinline__ bool exact_sum(const float *row, const float *qv, int dim, int metric, int K, int lane,
+                                          int64_t &sum, int &emax) {
+  constexpr int R = 8;  // products kept in registers (rows of up to 256 floats are read once)
+  uint32_t b[R];
+  uint32_t top = 0u;
+  auto product = [&](int j) {
+    const float x = __ldg(row + j), q = qv[j];
+    if (metric == SONG_METRIC_L2) {
+      const float diff = __fsub_rn(x, q);
+      return __float_as_uint(__fmul_rn(diff, diff));
+    }
+    return __float_as_uint(__fmul_rn(x, q));
+  };
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int j = lane + 32 * r;
+    b[r] = j < dim ? product(j) : 0u;
+    top = max(top, b[r] & 0x7f800000u);
+  }
+  for (int j = lane + 32 * R; j < dim; j += 32) top = max(top, product(j) & 0x7f800000u);
+  emax = static_cast<int>(__reduce_max_sync(FULLM, top) >> 23);
+  const int base = emax - K;
+  bool ok = emax != 255;
+  int64_t s = 0;
+  auto take = [&](uint32_t bits) {
+    const int e = static_cast<int>((bits >> 23) & 255u);
+    const int sh = e - base;
+    const bool zero = (bits & 0x7fffffffu) == 0u;
+    ok = ok && (zero || (e > 0 && sh >= 0));
+    const int64_t m = zero ? 0 : static_cast<int64_t>((bits & 0x7fffffu) | 0x800000u) << max(sh, 0);
+    s += (bits & 0x80000000u) ? -m : m;
+  };
+#pragma unroll
+  for (int r = 0; r < R; ++r) take(b[r]);
+  for (int j = lane + 32 * R; j < dim; j += 32) take(product(j));
+  if (__any_sync(FULLM, !ok)) return false;
+  // |s| <= 2^48: two 24-bit parts, each part's warp sum within 32 bits
+  const int hi = __reduce_add_sync(FULLM, static_cast<int>(s >> 24));
+  const int lo = __reduce_add_sync(FULLM, static_cast<int>(s & 0xffffff));
+  sum = (static_cast<int64_t>(hi) << 24) + lo;
+  return true;
+}
+
+// W warps a vertex: 4, with the visited set in the block's shared memory, for
+// batches that fill the GPU that way at most once (what counts there is the
+// latency of one search); 1, with it in the scratch region, beyond.
+template <int W>
+__global__ void __launch_bounds__(BUILD_WARPS * 32) beam_search_kernel(const BuildArgs p, const int K) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int team = W == 1 ? wib : 0, rank = W == 1 ? 0 : wib;  // this vertex's slice, this warp's place in it
+  const size_t qbytes = (static_cast<size_t>(p.dim) * 4 + 15) & ~size_t(15);
+  const size_t slice = sizeof(BeamList) + 32 * 8 + 32 * 4 + 16 + qbytes;
+  unsigned char *mem = smem + slice * team;
+  BeamList &L = *reinterpret_cast<BeamList *>(mem);
+  double *cd = reinterpret_cast<double *>(mem + sizeof(BeamList));        // candidates' distances
+  uint32_t *cid = reinterpret_cast<uint32_t *>(cd + 32);                  // and ids
+  volatile int *ctl = reinterpret_cast<volatile int *>(cid + 32);         // candidates of the hop, -1: done
+  float *qv = reinterpret_cast<float *>(mem + sizeof(BeamList) + 32 * 8 + 32 * 4 + 16);
+  const uint64_t gw = static_cast<uint64_t>(blockIdx.x) * BUILD_WARPS + wib;
+  uint32_t *vis = W == 1 ? p.vis + gw * p.vis_cap : reinterpret_cast<uint32_t *>(smem + slice);
+  const uint32_t vis_cap = W == 1 ? p.vis_cap : 1u << BEAM_VIS_LOG2;
+  const int vis_log2 = W == 1 ? p.vis_log2 : BEAM_VIS_LOG2;
+  const uint32_t vis_limit = vis_cap - (vis_cap >> 2);  // fill at most 3/4
+  const uint32_t nslots = 1u << p.shift;
+  auto sync = [&] {
+    if (W == 1) __syncwarp();
+    else __syncthreads();
+  };
+
+  for (;;) {
+    uint32_t t = 0;
+    if (rank == 0 && lane == 0) t = atomicAdd(p.counter, 1u);
+    if (W == 1) {
+      t = __shfl_sync(FULLM, t, 0);
+    } else {
+      if (threadIdx.x == 0) ctl[1] = static_cast<int>(t);
+      __syncthreads();
+      t = static_cast<uint32_t>(ctl[1]);
+    }
+    if (t >= p.count) break;
+    const uint64_t v = p.first + t;
+    if (p.limit == 0) {  // the first vertex: nothing to search
+      if (rank == 0 && lane == 0) p.out_cnt[t] = 0;
+      sync();
+      continue;
+    }
+    for (uint32_t i = rank * 32 + lane; i < vis_cap; i += 32 * W) vis[i] = VIS_EMPTY;
+    const float *vrow = p.data + v * static_cast<uint64_t>(p.dim);
+    for (int i = rank * 32 + lane; i < p.dim; i += 32 * W) qv[i] = vrow[i];
+    const float lenv = p.norms ? p.norms[v] : 0.0f;
+    sync();
+    if (rank == 0 && lane == 0) {
+      vis_insert(vis, vis_cap, vis_log2, 0u);
+      cid[0] = 0u;
+      ctl[0] = 1;
+    }
+    sync();
+    int n = 0;             // listed vertices (rank 0)
+    uint32_t vis_n = 1;    // visited ones (rank 0)
+    bool overflow = false; // (rank 0)
+    for (;;) {
+      // distances of this hop's candidates, the warps taking them in turn
+      const int m = ctl[0];
+      if (m < 0) break;
+      int64_t sum = 0;
+      int emax = 0;
+      bool have = false, ok = false;
+      for (int c = rank; c < m; c += W) {
+        int64_t s = 0;
+        int e = 0;
+        const bool good =
+            exact_sum(p.data + static_cast<uint64_t>(cid[c]) * p.dim, qv, p.dim, p.metric, K, lane, s, e);
+        if (lane == c) {
+          sum = s;
+          emax = e;
+          ok = good;
+          have = true;
+        }
+      }
+      if (have) {
+        const uint32_t id = cid[lane];
+        double d;
+        if (ok) {
+          // 2^(emax - K - 150): the integers' unit
+          const double unit = __longlong_as_double(static_cast<int64_t>(emax - K - 150 + 1023) << 52);
+          d = __dmul_rn(static_cast<double>(sum), unit);
+          if (p.metric == SONG_METRIC_IP) d = __dsub_rn(0.0, d);
+          if (p.metric == SONG_METRIC_COS) {
+            const double sign = d < 0 ? 1.0 : -1.0;
+            d = __dmul_rn(sign, __ddiv_rn(__ddiv_rn(__dmul_rn(d, d), static_cast<double>(p.norms[id])),
+                                          static_cast<double>(lenv)));
+          }
+        } else {
+          d = cpu_distance(p, p.data + static_cast<uint64_t>(id) * p.dim, qv, p.norms ? p.norms[id] : 0.0f, lenv);
+        }
+        cd[lane] = d;
+      }
+      sync();
+      if (rank == 0) {
+        // the candidates into the list: each one's place is the number of
+        // listed vertices and of candidates below it
+        uint64_t key = ~0ull;
+        uint32_t id = 0xffffffffu;
+        bool in = lane < m;
+        if (in) {
+          key = ordered(cd[lane]);
+          id = cid[lane];
+          if (n >= p.budget && key > L.d[p.budget - 1]) in = false;
+        }
+        const bool bad = lane < m && isnan(cd[min(lane, 31)]);  // no order: for the step-by-step search
+        if (__any_sync(FULLM, bad)) overflow = true;
+        unsigned live = __ballot_sync(FULLM, in);
+        const int add = __popc(live);
+        if (n + add > BEAM_CAP) overflow = true;
+        if (add > 0 && !overflow) {
+          int lo = 0;
+          if (in) {
+            int hi = n;
+            while (lo < hi) {
+              const int mid = (lo + hi) >> 1;
+              const uint64_t x = L.d[mid];
+              if (x < key || (x == key && (L.w[mid] >> 1) < id)) lo = mid + 1;
+              else hi = mid;
+            }
+          }
+          uint64_t od[BEAM_CAP / 32];
+          uint32_t ow[BEAM_CAP / 32];
+          int up[BEAM_CAP / 32];
+#pragma unroll
+          for (int j = 0; j < BEAM_CAP / 32; ++j) {
+            od[j] = L.d[32 * j + lane];
+            ow[j] = L.w[32 * j + lane];
+            up[j] = 0;
+          }
+          int before = 0;
+          __syncwarp();
+          while (live) {
+            const int c = __ffs(live) - 1;
+            live &= live - 1u;
+            const uint64_t ok_ = __shfl_sync(FULLM, key, c);
+            const uint32_t oid = __shfl_sync(FULLM, id, c);
+            const int at = __shfl_sync(FULLM, lo, c);
+            before += (ok_ < key || (ok_ == key && oid < id)) ? 1 : 0;
+#pragma unroll
+            for (int j = 0; j < BEAM_CAP / 32; ++j) up[j] += at <= 32 * j + lane ? 1 : 0;
+          }
+#pragma unroll
+          for (int j = 0; j < BEAM_CAP / 32; ++j) {
+            const int i = 32 * j + lane;
+            if (i < n && up[j] > 0) {
+              L.d[i + up[j]] = od[j];
+              L.w[i + up[j]] = ow[j];
+            }
+          }
+          if (in) {
+            L.d[lo + before] = key;
+            L.w[lo + before] = id << 1;
+          }
+          n += add;
+          __syncwarp();
+          if (n > p.budget) {  // beyond the first `budget`, only their last one's equals stay
+            const uint64_t last = L.d[p.budget - 1];
+            int keep = p.budget;
+            for (int b = p.budget; b < n; b += 32)
+              keep += __popc(__ballot_sync(FULLM, b + lane < n && L.d[min(b + lane, BEAM_CAP - 1)] <= last));
+            n = keep;
+          }
+        }
+        // the next pop: the first listed vertex not popped
+        int at = -1;
+        for (int b = 0; b < n && at < 0; b += 32) {
+          const unsigned o = __ballot_sync(FULLM, b + lane < n && (L.w[min(b + lane, BEAM_CAP - 1)] & 1u) == 0u);
+          if (o) at = b + __ffs(o) - 1;
+        }
+        int next = -1;
+        if (at >= 0 && !overflow) {
+          const uint32_t now = L.w[at] >> 1;
+          __syncwarp();
+          if (lane == 0) L.w[at] |= 1u;
+          // graph.h:196-205: its unvisited neighbours
+          const uint32_t *row = p.adj + (static_cast<uint64_t>(now) << p.shift);
+          const uint32_t a = static_cast<uint32_t>(lane) < nslots ? __ldg(row + lane) : 0u;
+          const uint32_t deg = __shfl_sync(FULLM, a, 0);
+          const bool fresh = lane >= 1 && static_cast<uint32_t>(lane) <= deg && vis_insert(vis, vis_cap, vis_log2, a);
+          const unsigned fm = __ballot_sync(FULLM, fresh);
+          next = __popc(fm);
+          vis_n += next;
+          if (vis_n > vis_limit) overflow = true;
+          if (fresh) cid[__popc(fm & ((1u << lane) - 1u))] = a;
+        }
+        if (lane == 0) ctl[0] = overflow ? -1 : next;
+      }
+      sync();
+    }
+    if (rank == 0) {
+      if (overflow) {
+        if (lane == 0) atomicOr(p.error, vis_n > vis_limit ? (W == 1 ? 1 : 4) : 4);
+      } else {
+        // graph.h:207-215: the list in ascending order
+        const int num = min(min(n, p.budget), p.out_k);
+        for (int i = lane; i < num; i += 32) p.out[static_cast<uint64_t>(t) * p.out_k + i] = L.w[i] >> 1;
+        if (lane == 0) p.out_cnt[t] = min(n, p.budget);
+      }
+    }
+    sync();
+  }
+}
+
 // Squared norms of all rows, each a float sum in dimension order (data.h:50-62).
 __global__ void row_norms_kernel(const float *data, uint64_t n, int dim, float *out) {
   for (uint64_t r = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; r < n;
@@ -374,6 +666,31 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
   const uint64_t blocks = static_cast<uint64_t>(sms) * per_sm;
   const uint64_t warps = blocks * BUILD_WARPS;
 
+  // the one-list search: list, candidates and query per vertex, and with a
+  // block per vertex the visited set
+  const size_t beam_slice = sizeof(BeamList) + 32 * 8 + 32 * 4 + 16 + ((static_cast<size_t>(dim) * 4 + 15) & ~size_t(15));
+  const size_t beam_smem1 = beam_slice * BUILD_WARPS, beam_smem4 = beam_slice + (sizeof(uint32_t) << BEAM_VIS_LOG2);
+  int log2dim = 0;
+  while ((1ull << log2dim) < static_cast<uint64_t>(dim)) ++log2dim;
+  const int beam_k = 53 - 24 - log2dim;
+  int beam1 = 0, beam4 = 0;  // resident blocks per SM
+  const bool beam = budget <= BEAM_BUDGET && shift <= 5 && n < (1ull << 31) && beam_smem1 <= static_cast<size_t>(optin) &&
+                    beam_smem4 <= static_cast<size_t>(optin) && beam_k > 0;
+  if (beam) {
+    e = cudaFuncSetAttribute(beam_search_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(beam_smem1));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(beam_search_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(beam_smem4));
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&beam1, beam_search_kernel<1>, BUILD_WARPS * 32, beam_smem1);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&beam4, beam_search_kernel<4>, BUILD_WARPS * 32, beam_smem4);
+    if (e != cudaSuccess) return fail(SONG_ERR_CUDA, "graph build: %s", cudaGetErrorString(e));
+    beam1 = std::max(1, std::min(beam1, per_sm));  // (the scratch has room for per_sm blocks)
+    beam4 = std::max(1, beam4);
+  }
+
   cudaStream_t st;
   e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
   if (e != cudaSuccess) return fail(SONG_ERR_CUDA, "graph build: %s", cudaGetErrorString(e));
@@ -438,6 +755,7 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
   while (a < n) {
     const uint64_t bs = batch_div == 0 ? 1 : std::max<uint64_t>(1, a / static_cast<uint64_t>(batch_div));
     const uint64_t end = std::min<uint64_t>(n, a + bs);
+    bool one_list = beam;
     for (int attempt = 0;; ++attempt) {
       BuildArgs p;
       p.data = static_cast<const float *>(d_data.p);
@@ -461,8 +779,15 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
       p.counter = static_cast<uint32_t *>(d_ctl.p);
       p.error = static_cast<int32_t *>(d_ctl.p) + 1;
       SONG_GB_CK(cudaMemsetAsync(d_ctl.p, 0, 8, st));
-      const uint64_t grid = std::min<uint64_t>(blocks, (end - a + BUILD_WARPS - 1) / BUILD_WARPS);
-      build_search_kernel<<<static_cast<unsigned>(grid), BUILD_WARPS * 32, smem, st>>>(p);
+      const uint64_t count = end - a, grid = std::min<uint64_t>(blocks, (count + BUILD_WARPS - 1) / BUILD_WARPS);
+      const uint64_t fit4 = static_cast<uint64_t>(sms) * beam4, fit1 = static_cast<uint64_t>(sms) * beam1;
+      if (one_list && count <= fit4)
+        beam_search_kernel<4><<<static_cast<unsigned>(count), BUILD_WARPS * 32, beam_smem4, st>>>(p, beam_k);
+      else if (one_list)
+        beam_search_kernel<1><<<static_cast<unsigned>(std::min<uint64_t>(fit1, grid)), BUILD_WARPS * 32, beam_smem1, st>>>(
+            p, beam_k);
+      else
+        build_search_kernel<<<static_cast<unsigned>(grid), BUILD_WARPS * 32, smem, st>>>(p);
       SONG_GB_CK(cudaGetLastError());
       SONG_GB_CK(cudaMemcpyAsync(h_err32, p.error, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
       SONG_GB_CK(cudaMemcpyAsync(h_cnt32, d_cnt.p, sizeof(int32_t) * (end - a), cudaMemcpyDeviceToHost, st));
@@ -470,7 +795,11 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
                                  cudaMemcpyDeviceToHost, st));
       SONG_GB_CK(cudaStreamSynchronize(st));
       if (*h_err32 == 0) break;
-      if (attempt >= 6) return fail(SONG_ERR_OOM, "graph build: search scratch still too small after growing");
+      if (*h_err32 & 4) {  // for the step-by-step search
+        one_list = false;
+        continue;
+      }
+      if (attempt >= 7) return fail(SONG_ERR_OOM, "graph build: search scratch still too small after growing");
       if (*h_err32 & 1) ++vis_log2;
       if (*h_err32 & 2) ++q_log2;
       rc = alloc_scratch();
