@@ -358,25 +358,27 @@ struct Team {
   }
 };
 
-// Warp `wib`'s share of a gather: candidates 8 wib .. of the m listed in cbuf.
+// Warp `wib`'s share of a gather: candidates 8 wib .. of the m listed from
+// cbuf[at] on.
 template <int METRIC, int STORAGE>
-__device__ __forceinline__ void team_pass(const Params &p, const WarpCtx &w, const Team &t, int m, int wib, int lane) {
+__device__ __forceinline__ void team_pass(const Params &p, const WarpCtx &w, const Team &t, int m, int at, int wib,
+                                          int lane) {
   const int c = 8 * wib + (lane >> 2);
   if (8 * wib >= m) return;  // whole warp
-  const float d = rows_pass<METRIC, STORAGE>(p.rows, p.row_bytes, p.scale_off, p.width, w.qv, w.cbuf[min(c, m - 1)],
-                                             lane);
+  const float d = rows_pass<METRIC, STORAGE>(p.rows, p.row_bytes, p.scale_off, p.width, w.qv,
+                                             w.cbuf[at + min(c, m - 1)], lane);
   if ((lane & 3) == 0 && c < m) t.dist[c] = d;
 }
 
-template <int METRIC, int STORAGE>
+template <int METRIC, int STORAGE, bool LEARNED>
 __device__ __forceinline__ void team_help(const Params &p, const WarpCtx &w, Team t, int wib, int lane) {
-  const VisitedHash vh = VisitedOf<false>::make(w.tab, p.pq);
+  const auto vh = VisitedOf<LEARNED>::make(w.tab, p.pq);
   for (;;) {
     int arg;
     const int c = t.next(&arg);
     if (c == Team::STOP) return;
     if (c > 0) {
-      team_pass<METRIC, STORAGE>(p, w, t, c, wib, lane);
+      team_pass<METRIC, STORAGE>(p, w, t, c, arg, wib, lane);
       Team::barrier();
       continue;
     }
@@ -518,20 +520,45 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
       if (tn < pq) ++tn;
       else vh.del(key_id(ev), lane);
       if (tn == pq) tmax = TS.max();
+      return;
+    }
+    visited_refresh(vh, now_id, now_home, lane);
+    if (tn < pq) {
+      ++tn;
+      T.append(now, pq, lane);
+      if (tn == pq) tmax = T.max();
+    } else if (now < tmax) {
+      vh.del(key_id(tmax), lane);
+      T.replace(tmax, now, lane);
+      tmax = T.max();
     } else {
-      visited_refresh(vh, now_id, now_home, lane);
-      if (tn < pq) {
-        ++tn;
-        T.append(now, pq, lane);
-        if (tn == pq) tmax = T.max();
-      } else if (now < tmax) {
-        vh.del(key_id(tmax), lane);
-        T.replace(tmax, now, lane);
-        tmax = T.max();
-      } else {
-        vh.del(now_id, lane);
+      vh.del(now_id, lane);
+    }
+  };
+
+  // Distances of the m candidates listed from cbuf[at] on (cid in lane c),
+  // the block's other warps helping when there is one (Team).
+  auto gather = [&](int m, uint32_t cid, int at) {
+    if constexpr (TEAM) {
+      if (m > 8) {
+        team->call(m, at, lane);
+        team_pass<METRIC, STORAGE>(p, w, *team, m, at, 0, lane);
+        Team::barrier();
+        return lane < m ? team->dist[lane] : 0.0f;
       }
     }
+    // The rows past the first pass start their way into L2 (rows of 512 bytes
+    // and more: 1M x 128, 10,000 queries at pq 43 1193 -> 1161 us, at pq 100
+    // from vertex 0 4.61 -> 4.41 ms; no gain on shorter ones, and the learned
+    // kernels lose registers to it: 959 -> 1025 us).
+    if constexpr (!LEARNED && !TEAM && STORAGE <= 1) {
+      if (lane >= 8 && lane < m && p.row_bytes >= 512) {
+        const uint8_t *row = p.rows + static_cast<uint64_t>(cid) * p.row_bytes;
+        for (uint32_t b = 0; b < p.row_bytes; b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + b));
+      }
+      __syncwarp();
+    }
+    return gather_distances<METRIC, STORAGE>(p, w.qv, m, cid, lane, qc);
   };
 
   int finished = 0;  // MULTI: finish tests that held (finished[cid], :190-192)
@@ -579,7 +606,7 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
         const int mr = min(32, m - r0);
         const uint32_t cid = lane < mr ? w.cbuf[r0 + lane] : 0u;
         const int chome = lane < mr ? w.chome[r0 + lane] : 0;
-        cd = gather_distances<METRIC, STORAGE>(p, w.qv, mr, cid, lane, qc);
+        cd = gather(mr, cid, r0);
         evals += mr;
         const uint64_t ck = lane < mr ? make_key(cd, cid) : ~0ull;
         if (p.double_check) {
@@ -608,6 +635,7 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
       if (qn > 0) {
         next_id = key_id(Q.min());
         a_next = adjacency(next_id);
+        if constexpr (TEAM) team->call(Team::PREFETCH, static_cast<int>(next_id), lane);
       }
       continue;
     }
@@ -629,8 +657,9 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
       last_change = hops;
     }
     list_insert(now, now_id, vh.slot(now_id));
-    if constexpr (LEARNED)
+    if constexpr (LEARNED) {
       if (enters && tn >= k) kth_key = TS.at(TS.start + k - 1);
+    }
     // :211-224 neighbours not in the visited hash, in row order.
     const int deg = static_cast<int>(__shfl_sync(FULL, a, 0));
     const int ahome = vh.slot(a);
@@ -646,17 +675,7 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
     const uint32_t cid = lane < m ? w.cbuf[lane] : 0u;
     const int chome = lane < m ? w.chome[lane] : 0;
     // :237-287 distances.
-    bool shared = false;
-    if constexpr (TEAM) {
-      shared = m > 8;
-      if (shared) {
-        team->call(m, 0, lane);
-        team_pass<METRIC, STORAGE>(p, w, *team, m, 0, lane);
-        Team::barrier();
-        cd = lane < m ? team->dist[lane] : 0.0f;
-      }
-    }
-    if (!shared) cd = gather_distances<METRIC, STORAGE>(p, w.qv, m, cid, lane, qc);
+    cd = gather(m, cid, 0);
     evals += m;
     // The next vertex popped is the smaller of the queue head and the best
     // candidate (the select-insert rule can only reject candidates above a
@@ -759,6 +778,39 @@ struct MinBlocks {
   static constexpr int value = S > 16 ? 2 : (S > 4 ? 4 : 5);
 };
 
+// Query qid of the launch; false if a bulk copy never completed.
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI, bool TEAM>
+__device__ __forceinline__ bool search_one(const Params &p, WarpCtx &w, uint32_t qid, int lane, Team *team) {
+  float *trace = nullptr;
+  if (LEARNED && p.trace) trace = p.trace + static_cast<size_t>(qid) * p.trace_hops * TRACE_FIELDS;
+  QueryStats st;
+  if (!run_query<METRIC, STORAGE, S, LEARNED, MULTI, TEAM>(
+          p, w, p.queries + static_cast<size_t>(qid) * p.dim,
+          p.starts ? p.starts + static_cast<size_t>(qid) * p.n_starts : nullptr, p.n_starts, p.pq, p.k,
+          p.out + static_cast<size_t>(qid) * p.k, trace, st, lane,
+          STORAGE == 3 ? p.qcodes + static_cast<size_t>(qid) * 8 : nullptr, team)) {
+    if (lane == 0) atomicOr(p.error, 1);
+    return false;
+  }
+  if (lane == 0) {
+    if (p.hops) p.hops[qid] = st.hops;
+    if (p.evals) p.evals[qid] = st.evals;
+    if (LEARNED && p.trace_final) {
+      p.trace_final[2 * qid] = st.version;
+      p.trace_final[2 * qid + 1] = min(st.hops, p.trace_hops);
+    }
+  }
+  __syncwarp();
+  return true;
+}
+
+// The early-exit network's weights into the block's shared memory.
+__device__ __forceinline__ void load_mlp(const Params &p, __nv_bfloat16 *wmlp) {
+  if (p.mlp)
+    for (int i = threadIdx.x; i < MLP_NPARAM; i += blockDim.x) wmlp[i] = p.mlp[i];
+  __syncthreads();
+}
+
 template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false>
 __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, MinBlocks<S>::value)
     search_kernel(const Params p) {
@@ -770,71 +822,35 @@ __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, MinBlocks<S>::value)
   w.init(smem_raw + static_cast<size_t>(wib) * p.warp_bytes, p, (MULTI ? MAX_PROBES : 1) * 32, lane);
   __nv_bfloat16 *wmlp = reinterpret_cast<__nv_bfloat16 *>(smem_raw + static_cast<size_t>(nwarps) * p.warp_bytes);
   w.wmlp = wmlp;
-  if (LEARNED) {
-    if (p.mlp)
-      for (int i = threadIdx.x; i < MLP_NPARAM; i += blockDim.x) wmlp[i] = p.mlp[i];
-    __syncthreads();
-  }
+  if (LEARNED) load_mlp(p, wmlp);
 
   for (;;) {
     uint32_t qid = 0;
     if (lane == 0) qid = atomicAdd(p.counter, 1u);
     qid = __shfl_sync(FULL, qid, 0);
     if (qid >= static_cast<uint32_t>(p.nq)) break;
-    float *trace = nullptr;
-    if (LEARNED && p.trace) trace = p.trace + static_cast<size_t>(qid) * p.trace_hops * TRACE_FIELDS;
-    QueryStats st;
-    if (!run_query<METRIC, STORAGE, S, LEARNED, MULTI>(p, w, p.queries + static_cast<size_t>(qid) * p.dim,
-                                                   p.starts ? p.starts + static_cast<size_t>(qid) * p.n_starts
-                                                            : nullptr,
-                                                   p.n_starts, p.pq,
-                                                   p.k, p.out + static_cast<size_t>(qid) * p.k, trace, st,
-                                                   lane, STORAGE == 3 ? p.qcodes + static_cast<size_t>(qid) * 8
-                                                                      : nullptr)) {
-      if (lane == 0) atomicOr(p.error, 1);
-      return;
-    }
-    if (lane == 0) {
-      if (p.hops) p.hops[qid] = st.hops;
-      if (p.evals) p.evals[qid] = st.evals;
-      if (LEARNED && p.trace_final) {
-        p.trace_final[2 * qid] = st.version;
-        p.trace_final[2 * qid + 1] = min(st.hops, p.trace_hops);
-      }
-    }
-    __syncwarp();
+    if (!search_one<METRIC, STORAGE, S, LEARNED, MULTI, false>(p, w, qid, lane, nullptr)) return;
   }
 }
 
 // The search with a block per query (Team).
-template <int METRIC, int STORAGE, int S>
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI>
 __global__ void __launch_bounds__(TEAM_WARPS * 32, S > 16 ? 2 : 4) search_team_kernel(const Params p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   WarpCtx w;
-  w.init(smem_raw, p, 32, wib == 0 ? lane : 1);  // lane 0 of warp 0 sets the barrier up
-  w.wmlp = nullptr;
+  w.init(smem_raw, p, (MULTI ? MAX_PROBES : 1) * 32, wib == 0 ? lane : 1);  // lane 0 of warp 0 sets the barrier up
   Team team;
   team.init(smem_raw + p.warp_bytes);
+  __nv_bfloat16 *wmlp = reinterpret_cast<__nv_bfloat16 *>(smem_raw + p.warp_bytes + TEAM_BYTES);
+  w.wmlp = wmlp;
+  if (LEARNED) load_mlp(p, wmlp);
   if (wib > 0) {
-    team_help<METRIC, STORAGE>(p, w, team, wib, lane);
+    team_help<METRIC, STORAGE, LEARNED>(p, w, team, wib, lane);
     return;
   }
-  for (int qid = blockIdx.x; qid < p.nq; qid += gridDim.x) {
-    QueryStats st;
-    if (!run_query<METRIC, STORAGE, S, false, false, true>(
-            p, w, p.queries + static_cast<size_t>(qid) * p.dim,
-            p.starts ? p.starts + static_cast<size_t>(qid) * p.n_starts : nullptr, p.n_starts, p.pq, p.k,
-            p.out + static_cast<size_t>(qid) * p.k, nullptr, st, lane, nullptr, &team)) {
-      if (lane == 0) atomicOr(p.error, 1);
-      break;
-    }
-    if (lane == 0) {
-      if (p.hops) p.hops[qid] = st.hops;
-      if (p.evals) p.evals[qid] = st.evals;
-    }
-    __syncwarp();
-  }
+  for (uint32_t qid = blockIdx.x; qid < static_cast<uint32_t>(p.nq); qid += gridDim.x)
+    if (!search_one<METRIC, STORAGE, S, LEARNED, MULTI, true>(p, w, qid, lane, &team)) break;
   team.call(Team::STOP, 0, lane);
 }
 
@@ -850,10 +866,11 @@ int get_team_shape(const void *fn, uint32_t bytes, int *grid_cap);
 
 template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false>
 int launch_kernel(const Params &p, cudaStream_t stream) {
-  if constexpr (STORAGE != 3 && !LEARNED && !MULTI) {
+  const uint32_t extra = LEARNED ? static_cast<uint32_t>(MLP_NPARAM * sizeof(__nv_bfloat16) + 64) : 0u;
+  if constexpr (STORAGE != 3) {
     // a block per query while all of them run at once
-    auto team = search_team_kernel<METRIC, STORAGE, S>;
-    const uint32_t bytes = p.warp_bytes + TEAM_BYTES;
+    auto team = search_team_kernel<METRIC, STORAGE, S, LEARNED, MULTI>;
+    const uint32_t bytes = p.warp_bytes + TEAM_BYTES + extra;
     int cap = 0;
     int e = get_team_shape(reinterpret_cast<const void *>(team), bytes, &cap);
     if (e == 0 && p.nq <= cap) {
@@ -862,7 +879,6 @@ int launch_kernel(const Params &p, cudaStream_t stream) {
     }
   }
   auto kern = search_kernel<METRIC, STORAGE, S, LEARNED, MULTI>;
-  const uint32_t extra = LEARNED ? static_cast<uint32_t>(MLP_NPARAM * sizeof(__nv_bfloat16) + 64) : 0u;
   int wpb = 0, cap = 0;
   int e = get_shape(reinterpret_cast<const void *>(kern), p.warp_bytes, extra, &wpb, &cap);
   if (e != 0) return e;

@@ -71,3 +71,21 @@ def test_row_widths(song, oracle, dim):
                 ix.set_rerank(0)
                 ox = oracle.OracleIndex(song.dequantize_rows(ix.rows(), storage, dim), g, 5, metric)
                 _check(ix, q, 40, ox.kernel_search(q, 40, oracle.MODE_LEX), (metric, storage))
+
+
+@pytest.mark.parametrize("pq", [10, 40, 100, 200, 300, 600])
+def test_multi_probe_and_learned_batches(song, oracle, pq):
+    """The multi-probe and the learned kernels with a block and with a warp
+    per query (the latter with an exit that never fires: the exact visited
+    set's search)."""
+    data, q = _clustered(2500, 16, seed=7)
+    g = _ring_graph(song, data, 0, 5, seed=7)
+    ox = oracle.OracleIndex(data, g, 5, 0)
+    with song.Index(g, data, 5, 0) as ix:
+        for probes, cnt, dc in ((4, 1, False), (2, 2, True)):
+            ix.set_multiprobe(probes, cnt, dc)
+            want = ox.kernel_search(q, pq, oracle.MODE_LEX, probes=probes, finish_cnt=cnt, double_check=dc)
+            _check(ix, q, pq, want, (probes, cnt, dc))
+        ix.set_multiprobe()
+        ix.set_hop_limit(1 << 30)
+        _check(ix, q, pq, ox.kernel_search(q, pq, oracle.MODE_LEX_EXACT), "learned")
