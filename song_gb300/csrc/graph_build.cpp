@@ -33,9 +33,14 @@
 // This file must be compiled without floating-point contraction.
 #include <algorithm>
 #include <atomic>
+#include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <functional>
+#include <mutex>
+#include <system_error>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include "graph_build.h"
@@ -43,7 +48,79 @@
 
 namespace {
 
+// Worker threads that live as long as their builder: a build applies hundreds
+// of batches of a fraction of a millisecond, and starting 15 threads for each
+// took longer than the work.  A worker looks for the next call for about
+// 0.3 ms before it sleeps.
+class Pool {
+ public:
+  ~Pool() {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      stop_ = true;
+    }
+    cv_.notify_all();
+    for (auto &t : threads_) t.join();
+  }
+
+  // Runs fn on nt threads (this one among them) and returns when all are done.
+  void run(int nt, const std::function<void()> &fn) {
+    try {
+      while (static_cast<int>(threads_.size()) < nt - 1) {
+        const int i = static_cast<int>(threads_.size());
+        threads_.emplace_back([this, i] { loop(i); });
+      }
+    } catch (const std::system_error &) {  // with the threads there are
+    }
+    const uint64_t want = static_cast<uint64_t>(std::max(0, std::min<int>(nt - 1, static_cast<int>(threads_.size()))));
+    if (want == 0) {
+      fn();
+      return;
+    }
+    job_ = &fn;
+    left_.store(want, std::memory_order_relaxed);
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      state_.store((((state_.load() >> 16) + 1) << 16) | want);  // the call's number, its workers
+    }
+    cv_.notify_all();
+    fn();
+    while (left_.load(std::memory_order_acquire) > 0) std::this_thread::yield();
+  }
+
+ private:
+  void loop(int me) {
+    uint64_t seen = 0;
+    for (;;) {
+      uint64_t s = state_.load(std::memory_order_acquire);
+      for (int i = 0; s == seen && i < 1000 && !stop_; ++i) {
+        std::this_thread::yield();
+        s = state_.load(std::memory_order_acquire);
+      }
+      if (s == seen) {
+        std::unique_lock<std::mutex> lk(mu_);
+        cv_.wait(lk, [&] { return stop_ || state_.load() != seen; });
+        s = state_.load();
+      }
+      if (s == seen) return;  // stopping
+      seen = s;
+      if (static_cast<uint64_t>(me) < (s & 0xffffu)) {
+        (*job_)();
+        left_.fetch_sub(1, std::memory_order_release);
+      }
+    }
+  }
+
+  std::vector<std::thread> threads_;
+  std::mutex mu_;
+  std::condition_variable cv_;
+  std::atomic<uint64_t> state_{0}, left_{0};
+  std::atomic<bool> stop_{false};
+  const std::function<void()> *job_ = nullptr;
+};
+
 struct Builder {
+  Pool pool;
   const float *data;
   uint64_t n;
   int dim, metric, shift, search_degree, fixed_degree, budget;
@@ -137,61 +214,75 @@ struct Builder {
     }
   }
 
-  // Edges of the new vertices a..e-1 (nb(v): its search result, ascending),
-  // row-parallel over nthreads; the rows changed are appended to *touched.
-  template <class NB>
-  void apply_batch(uint64_t a, uint64_t e, NB nb, int nthreads, std::vector<uint64_t> *touched) {
+  // Edges of the new vertices a..e-1 (nb(v): its search result, ascending,
+  // and its length), row-parallel over nthreads; done(i, row) once the i-th
+  // changed row is final (the new rows, then the others).  Returns their
+  // number.
+  template <class NB, class Done>
+  uint64_t apply_batch(uint64_t a, uint64_t e, NB nb, int nthreads, Done done) {
+    // one 64-bit word per (target row, new vertex) where both fit 32 bits
+    return n <= (1ull << 32) ? apply_sorted<Packed>(a, e, nb, nthreads, done)
+                             : apply_sorted<Wide>(a, e, nb, nthreads, done);
+  }
+
+  struct Packed {
+    uint64_t k;
+    Packed(uint64_t target, uint64_t v) : k((target << 32) | v) {}
+    uint64_t target() const { return k >> 32; }
+    uint64_t vertex() const { return k & 0xffffffffu; }
+    bool operator<(const Packed &o) const { return k < o.k; }
+  };
+  struct Wide {
+    uint64_t t, v;
+    Wide(uint64_t target, uint64_t vertex) : t(target), v(vertex) {}
+    uint64_t target() const { return t; }
+    uint64_t vertex() const { return v; }
+    bool operator<(const Wide &o) const { return t < o.t || (t == o.t && v < o.v); }
+  };
+
+  template <class Upd, class NB, class Done>
+  uint64_t apply_sorted(uint64_t a, uint64_t e, NB nb, int nthreads, Done done) {
     const uint64_t m = e - a;
-    std::vector<std::pair<uint64_t, uint64_t>> upd;  // (target row, new vertex)
+    std::vector<Upd> upd;
+    upd.reserve(static_cast<size_t>(m) * search_degree);
     for (uint64_t v = a; v < e; ++v) {
-      const uint64_t *ids;
-      int cnt;
-      nb(v, &ids, &cnt);
-      const int num = std::min<int>(search_degree, cnt);
-      for (int i = 0; i < num; ++i) upd.push_back({ids[i], v});
+      const auto r = nb(v);
+      const int num = std::min<int>(search_degree, r.second);
+      for (int i = 0; i < num; ++i) upd.emplace_back(r.first[i], v);
     }
     std::sort(upd.begin(), upd.end());
     std::vector<size_t> starts;  // one group per distinct target row
     for (size_t i = 0; i < upd.size(); ++i)
-      if (i == 0 || upd[i].first != upd[i - 1].first) starts.push_back(i);
+      if (i == 0 || upd[i].target() != upd[i - 1].target()) starts.push_back(i);
     starts.push_back(upd.size());
     const size_t groups = starts.size() - 1;
     auto own = [&](uint64_t v) {
-      const uint64_t *ids;
-      int cnt;
-      nb(v, &ids, &cnt);
-      const int num = std::min<int>(search_degree, cnt);
+      const auto r = nb(v);
+      const int num = std::min<int>(search_degree, r.second);
       size_t off = (size_t)v << shift;
       edges[off] = (uint64_t)num;
-      for (int i = 0; i < num; ++i) edges[off + i + 1] = ids[i];
+      for (int i = 0; i < num; ++i) edges[off + i + 1] = r.first[i];
       rank_edges(off);
     };
     auto rev = [&](size_t g) {
-      for (size_t i = starts[g]; i < starts[g + 1]; ++i) add_edge(upd[i].first, upd[i].second);
+      for (size_t i = starts[g]; i < starts[g + 1]; ++i) add_edge(upd[i].target(), upd[i].vertex());
     };
     const uint64_t work = m + groups;
-    int nt = (int)std::min<uint64_t>((uint64_t)std::max(1, nthreads), work / 16 + 1);
-    if (nt <= 1) {
-      for (uint64_t v = a; v < e; ++v) own(v);
-      for (size_t g = 0; g < groups; ++g) rev(g);
-    } else {
-      std::atomic<uint64_t> next(0);
-      auto worker = [&]() {
-        for (;;) {
-          uint64_t i = next.fetch_add(1);
-          if (i >= work) break;
+    const int nt = (int)std::min<uint64_t>((uint64_t)std::max(1, nthreads), work / 16 + 1);
+    std::atomic<uint64_t> next(0);
+    pool.run(nt, [&]() {
+      constexpr uint64_t STEP = 4;  // items a thread takes at a time
+      for (;;) {
+        const uint64_t first = next.fetch_add(STEP);
+        if (first >= work) break;
+        for (uint64_t i = first; i < std::min(work, first + STEP); ++i) {
           if (i < m) own(a + i);
           else rev((size_t)(i - m));
+          done(i, i < m ? a + i : upd[starts[i - m]].target());
         }
-      };
-      std::vector<std::thread> th;
-      for (int t = 0; t < nt; ++t) th.emplace_back(worker);
-      for (auto &x : th) x.join();
-    }
-    if (touched) {
-      for (uint64_t v = a; v < e; ++v) touched->push_back(v);
-      for (size_t g = 0; g < groups; ++g) touched->push_back(upd[starts[g]].first);
-    }
+      }
+    });
+    return work;
   }
 
   void apply(uint64_t v, const std::vector<uint64_t> &nb) {
@@ -315,24 +406,21 @@ extern "C" int song_graph_build(const float *data, uint64_t n, int dim, int metr
       res.assign(e - a, std::vector<uint64_t>());
       std::atomic<uint64_t> next(a);
       int nt = (int)std::min<uint64_t>((uint64_t)nthreads, e - a);
-      auto work = [&](int tid) {
+      std::atomic<int> ids(0);
+      b.pool.run(nt, [&]() {
+        const int tid = ids.fetch_add(1);
         for (;;) {
           uint64_t v = next.fetch_add(1);
           if (v >= e) break;
           searchers[tid].search(b.row(v), a, budget, res[v - a]);
         }
-      };
-      if (nt <= 1) {
-        work(0);
-      } else {
-        std::vector<std::thread> th;
-        for (int t = 0; t < nt; ++t) th.emplace_back(work, t);
-        for (auto &x : th) x.join();
-      }
-      b.apply_batch(a, e, [&](uint64_t v, const uint64_t **ids, int *cnt) {
-        *ids = res[v - a].data();
-        *cnt = (int)res[v - a].size();
-      }, nthreads, nullptr);
+      });
+      b.apply_batch(
+          a, e,
+          [&](uint64_t v) {
+            return std::pair<const uint64_t *, int>(res[v - a].data(), (int)res[v - a].size());
+          },
+          nthreads, [](uint64_t, uint64_t) {});
       a = e;
     }
   }
@@ -375,14 +463,21 @@ GraphBuilder *graph_builder_create(const float *data, uint64_t n, int dim, int m
 
 void graph_builder_free(GraphBuilder *g) { delete g; }
 
-void graph_builder_apply(GraphBuilder *g, uint64_t a, uint64_t e, const uint32_t *ids, const int32_t *cnt,
-                         int ld, int nthreads, std::vector<uint64_t> *touched) {
-  std::vector<uint64_t> wide((size_t)(e - a) * (size_t)ld);
-  for (size_t i = 0; i < wide.size(); ++i) wide[i] = ids[i];
-  g->b.apply_batch(a, e, [&](uint64_t v, const uint64_t **p, int *c) {
-    *p = wide.data() + (size_t)(v - a) * (size_t)ld;
-    *c = cnt[v - a];
-  }, nthreads, touched);
+uint64_t graph_builder_apply(GraphBuilder *g, uint64_t a, uint64_t e, const uint32_t *ids, const int32_t *cnt,
+                             int ld, int nthreads, uint32_t *rows, uint64_t *row_ids) {
+  Builder &b = g->b;
+  const uint64_t w = 1ull << b.shift;
+  return b.apply_batch(
+      a, e,
+      [&](uint64_t v) {
+        return std::pair<const uint32_t *, int>(ids + (size_t)(v - a) * (size_t)ld, cnt[v - a]);
+      },
+      nthreads,
+      [&](uint64_t i, uint64_t row) {
+        const uint64_t *src = b.edges.data() + (row << b.shift);
+        for (uint64_t j = 0; j < w; ++j) rows[i * w + j] = static_cast<uint32_t>(src[j]);
+        row_ids[i] = row;
+      });
 }
 
 const uint64_t *graph_builder_edges(const GraphBuilder *g) { return g->b.edges.data(); }

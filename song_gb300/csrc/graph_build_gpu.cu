@@ -731,25 +731,25 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
                                               static_cast<float *>(d_norms.p));
     SONG_GB_CK(cudaGetLastError());
   }
-  int vis_log2 = 13, q_log2 = 12;  // grown when a batch overflows
-  auto alloc_scratch = [&]() -> int {
+  // scratch of the searches that keep their sets in device memory, allocated
+  // when the first such batch comes; grown when a batch overflows
+  int vis_log2 = 13, q_log2 = 12;
+  auto alloc_scratch = [&](bool queue) -> int {
     if (d_vis.p) cudaFree(d_vis.p);
     if (d_q.p) cudaFree(d_q.p);
     d_vis.p = d_q.p = nullptr;
     cudaError_t e1 = song::dev_malloc(&d_vis.p, sizeof(uint32_t) * (warps << vis_log2));
-    if (e1 == cudaSuccess) e1 = song::dev_malloc(&d_q.p, sizeof(QE) * (warps << q_log2));
+    if (e1 == cudaSuccess && queue) e1 = song::dev_malloc(&d_q.p, sizeof(QE) * (warps << q_log2));
     if (e1 != cudaSuccess)
       return fail(e1 == cudaErrorMemoryAllocation ? SONG_ERR_OOM : SONG_ERR_CUDA, "graph build: scratch: %s",
                   cudaGetErrorString(e1));
     return SONG_OK;
   };
-  int rc = alloc_scratch();
-  if (rc != SONG_OK) return rc;
+  int rc = SONG_OK;
 
   uint32_t *h_out32 = static_cast<uint32_t *>(h_out.p);
   int32_t *h_cnt32 = static_cast<int32_t *>(h_cnt.p);
   int32_t *h_err32 = static_cast<int32_t *>(h_err.p);
-  std::vector<uint64_t> touched;
   const uint64_t *edges = graph_builder_edges(gb);
   uint64_t a = 0;
   while (a < n) {
@@ -757,6 +757,11 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
     const uint64_t end = std::min<uint64_t>(n, a + bs);
     bool one_list = beam;
     for (int attempt = 0;; ++attempt) {
+      const uint64_t count = end - a, grid = std::min<uint64_t>(blocks, (count + BUILD_WARPS - 1) / BUILD_WARPS);
+      const uint64_t fit4 = static_cast<uint64_t>(sms) * beam4, fit1 = static_cast<uint64_t>(sms) * beam1;
+      const bool block_each = one_list && count <= fit4;
+      if ((!block_each && !d_vis.p) || (!one_list && !d_q.p))
+        if ((rc = alloc_scratch(!one_list)) != SONG_OK) return rc;
       BuildArgs p;
       p.data = static_cast<const float *>(d_data.p);
       p.norms = static_cast<const float *>(d_norms.p);
@@ -779,9 +784,7 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
       p.counter = static_cast<uint32_t *>(d_ctl.p);
       p.error = static_cast<int32_t *>(d_ctl.p) + 1;
       SONG_GB_CK(cudaMemsetAsync(d_ctl.p, 0, 8, st));
-      const uint64_t count = end - a, grid = std::min<uint64_t>(blocks, (count + BUILD_WARPS - 1) / BUILD_WARPS);
-      const uint64_t fit4 = static_cast<uint64_t>(sms) * beam4, fit1 = static_cast<uint64_t>(sms) * beam1;
-      if (one_list && count <= fit4)
+      if (block_each)
         beam_search_kernel<4><<<static_cast<unsigned>(count), BUILD_WARPS * 32, beam_smem4, st>>>(p, beam_k);
       else if (one_list)
         beam_search_kernel<1><<<static_cast<unsigned>(std::min<uint64_t>(fit1, grid)), BUILD_WARPS * 32, beam_smem1, st>>>(
@@ -802,20 +805,13 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
       if (attempt >= 7) return fail(SONG_ERR_OOM, "graph build: search scratch still too small after growing");
       if (*h_err32 & 1) ++vis_log2;
       if (*h_err32 & 2) ++q_log2;
-      rc = alloc_scratch();
+      rc = alloc_scratch(d_q.p != nullptr);
       if (rc != SONG_OK) return rc;
     }
-    touched.clear();
-    graph_builder_apply(gb, a, end, h_out32, h_cnt32, search_degree, nthreads, &touched);
-    // upload the changed rows
+    // the edges, and the changed rows straight into the upload buffer: <= (end - a) * (search_degree + 1) <= rows_cap
     uint32_t *hr = static_cast<uint32_t *>(h_rows.p);
     uint64_t *hi = static_cast<uint64_t *>(h_ids.p);
-    const uint64_t nt = touched.size();  // <= (end - a) * (search_degree + 1) <= rows_cap
-    for (uint64_t i = 0; i < nt; ++i) {
-      const uint64_t *src = edges + (touched[i] << shift);
-      for (uint32_t j = 0; j < w; ++j) hr[i * w + j] = static_cast<uint32_t>(src[j]);
-      hi[i] = touched[i];
-    }
+    const uint64_t nt = graph_builder_apply(gb, a, end, h_out32, h_cnt32, search_degree, nthreads, hr, hi);
     SONG_GB_CK(cudaMemcpyAsync(d_rows.p, hr, sizeof(uint32_t) * nt * w, cudaMemcpyHostToDevice, st));
     SONG_GB_CK(cudaMemcpyAsync(d_ids.p, hi, sizeof(uint64_t) * nt, cudaMemcpyHostToDevice, st));
     const uint64_t blocks_s = std::min<uint64_t>(4096, (nt * w + 255) / 256);
