@@ -132,7 +132,7 @@ int song_graph_build(const float *data, uint64_t n, int dim, int metric, int shi
                      uint64_t *graph_out);
 
 /* The same construction with each batch's searches (graph.h:169-216) on GPU
- * `device`, one warp per new vertex, and the edge updates on nthreads host
+ * `device`, a warp or a block per new vertex, and the edge updates on nthreads host
  * threads: graph_out equals song_graph_build's for the same arguments, bit
  * for bit.  budget <= 1024, n < 2^32 - 1. */
 int song_graph_build_gpu(const float *data, uint64_t n, int dim, int metric, int shift,
@@ -319,10 +319,11 @@ int song_search_noalloc(song_index *index, const float *queries, int nq, int pq,
 
 /* Test hooks for the failure paths (no counterpart in the reference).
  * song_debug_fail_alloc(n): the n-th next device allocation of the library
- * fails as out of memory (0: none).  song_debug_set_wait: the search kernel's
- * bounded waits give up after wait_limit polls (default 2^24), and every
- * batch of row copies expects extra_tx bytes (a multiple of 16) that no copy
- * delivers -- a wait that cannot complete; the call then returns
+ * fails as out of memory (0: none).  song_debug_set_wait: the kernels'
+ * bounded waits give up after wait_limit polls (default 2^24), and the copies
+ * that they wait for (a query's first adjacency row, the head phase's tiles)
+ * expect extra_tx bytes (a multiple of 16) that no copy delivers -- a wait
+ * that cannot complete; the call then returns
  * SONG_ERR_TIMEOUT and the index stays usable.  song_debug_server_hold(1):
  * admitted requests are kept from the kernel until song_debug_server_hold(0). */
 int song_debug_fail_alloc(int n);

@@ -1,5 +1,6 @@
 // entry_tiles.cuh -- exact search distances of a warp tile of 4 queries x 8
-// rows (32 pairs), for the two-level entry choice (entries.cu).
+// rows (32 pairs), for the head phase of rows that the tensor cores' form does
+// not take (entries.cu: heads_tiled_kernel).
 //
 // The search distance of a query q to a row x is fixed by the search kernel's
 // arithmetic (warp_astar_accelerator.h:237-287 with nvcc's FMA contraction):

@@ -72,7 +72,9 @@ class Pool {
       }
     } catch (const std::system_error &) {  // with the threads there are
     }
-    const uint64_t want = static_cast<uint64_t>(std::max(0, std::min<int>(nt - 1, static_cast<int>(threads_.size()))));
+    // (the state word holds their number in 16 bits)
+    const uint64_t want = static_cast<uint64_t>(
+        std::max(0, std::min(std::min(nt - 1, static_cast<int>(threads_.size())), 0xffff)));
     if (want == 0) {
       fn();
       return;
@@ -84,8 +86,13 @@ class Pool {
       state_.store((((state_.load() >> 16) + 1) << 16) | want);  // the call's number, its workers
     }
     cv_.notify_all();
+    struct Join {  // also when fn throws here: the workers use the caller's frame
+      std::atomic<uint64_t> &left;
+      ~Join() {
+        while (left.load(std::memory_order_acquire) > 0) std::this_thread::yield();
+      }
+    } join{left_};
     fn();
-    while (left_.load(std::memory_order_acquire) > 0) std::this_thread::yield();
   }
 
  private:

@@ -3,8 +3,8 @@
 // The builder (graph_build.cpp) inserts vertices in batches; every new vertex
 // runs the reference's CPU best-first search (graph.h:169-216) with result
 // size `budget` against the graph as it stood before its batch.  This file
-// runs those searches on the GPU, one warp per new vertex, and leaves the edge
-// bookkeeping (graph.h:116-167) to graph_build.cpp.  The GPU search is the CPU
+// runs those searches on the GPU (a warp, or a block of four, per new vertex)
+// and leaves the edge bookkeeping (graph.h:116-167) to graph_build.cpp.  The GPU search is the CPU
 // search restated exactly, so the GPU builder writes the same graph as the CPU
 // builder with the same batch_div, bit for bit:
 //
