@@ -173,14 +173,15 @@ int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t strea
   p.probes = c.probes;
   p.finish_cnt = c.finish_cnt;
   p.double_check = c.double_check;
-  if (multi) return launch_multi(p, ix.metric, S, stream);
+  const bool lng = ix.row_bytes >= LONG_ROW;
+  if (multi) return (lng ? launch_multi_long : launch_multi)(p, ix.metric, S, stream);
   if (learned) {
     if (ix.storage >= 2) return -1;
-    return launch_learned(p, ix.storage, ix.metric, S, stream);
+    return (lng ? launch_learned_long : launch_learned)(p, ix.storage, ix.metric, S, stream);
   }
   switch (ix.storage) {
-    case 0: return launch_f32(p, ix.metric, S, stream);
-    case 1: return launch_bf16(p, ix.metric, S, stream);
+    case 0: return (lng ? launch_f32_long : launch_f32)(p, ix.metric, S, stream);
+    case 1: return (lng ? launch_bf16_long : launch_bf16)(p, ix.metric, S, stream);
     case 2: return launch_fp8(p, ix.metric, S, stream);
     case 3: return c.qcodes ? launch_bits(p, ix.metric, S, stream) : -1;  // query codes come from the caller's path
     default: return -1;

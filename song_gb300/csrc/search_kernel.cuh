@@ -26,7 +26,8 @@
 // Template parameters: METRIC (0 L2, 1 IP, 2 COS), STORAGE (0 F32, 1 BF16,
 // 2 FP8-E4M3 with a per-row scale, 3 256-bit codes), S (register queue
 // segment, capacity 32*S >= pq+1), LEARNED (per-hop features: trace capture
-// and/or the early-exit network), MULTI (the multi-probe knobs).
+// and/or the early-exit network), MULTI (the multi-probe knobs), LONG (rows of
+// LONG_ROW bytes and more).
 //
 // What bounds it: instructions, in full batches and for a single query alike
 // (about six cycles each on a dependent path).  A hop of the headline search
@@ -121,11 +122,18 @@ struct Code8 {
   uint32_t w[8];
 };
 
+// 32-dimension steps of a row whose loads are in flight together: 16 (FP8) to
+// 32 registers a lane, 64 for long FP32 rows.
+template <int STORAGE, bool LONG>
+constexpr int row_steps() {
+  return STORAGE == 0 && !LONG ? 4 : 8;
+}
+
 // One pass: the distance of the row of vertex `id` (the same in a row's four
 // lanes), in those lanes.  qv: the query, zero-padded to a multiple of 32
 // floats.  `width` elements a row (zero-padded to the 16-byte load; a padded
 // element adds fma(0, 0, t)).
-template <int METRIC, int STORAGE>
+template <int METRIC, int STORAGE, bool LONG>
 __device__ __forceinline__ float rows_pass(const uint8_t *rows, uint32_t rb, uint32_t scale_off, int width,
                                            const float *qv, uint32_t id, int lane) {
   using Read = RowRead<STORAGE>;
@@ -154,7 +162,7 @@ __device__ __forceinline__ float rows_pass(const uint8_t *rows, uint32_t rb, uin
     }
   };
   int j = 0;
-  constexpr int U = STORAGE == 0 ? 4 : 8;  // 32-dimension steps in flight: 16 (FP8) to 32 registers
+  constexpr int U = row_steps<STORAGE, LONG>();
   for (; j + 32 * U <= width; j += 32 * U) {
     Read r[U];
 #pragma unroll
@@ -173,13 +181,13 @@ __device__ __forceinline__ float rows_pass(const uint8_t *rows, uint32_t rb, uin
 }
 
 // Distances of candidates 0..m-1 (candidate c's id in lane c) in lane c.
-template <int METRIC, int STORAGE>
+template <int METRIC, int STORAGE, bool LONG = false>
 __device__ __forceinline__ float gather_rows(const uint8_t *rows, uint32_t rb, uint32_t scale_off, int width,
                                              const float *qv, int m, uint32_t cid, int lane) {
   float out = 0.0f;
   for (int first = 0; first < m; first += 8) {
     const uint32_t id = __shfl_sync(FULL, cid, min(first + (lane >> 2), m - 1));
-    const float d = rows_pass<METRIC, STORAGE>(rows, rb, scale_off, width, qv, id, lane);
+    const float d = rows_pass<METRIC, STORAGE, LONG>(rows, rb, scale_off, width, qv, id, lane);
     const float mine = __shfl_sync(FULL, d, ((lane - first) & 7) * 4);
     if (lane >= first && lane < first + 8) out = mine;
   }
@@ -187,7 +195,7 @@ __device__ __forceinline__ float gather_rows(const uint8_t *rows, uint32_t rb, u
 }
 
 // The index's stored rows.
-template <int METRIC, int STORAGE>
+template <int METRIC, int STORAGE, bool LONG>
 __device__ __forceinline__ float gather_distances(const Params &p, const float *qv, int m, uint32_t cid, int lane,
                                                   const Code8 &qc) {
   if constexpr (STORAGE == 3) {
@@ -204,7 +212,7 @@ __device__ __forceinline__ float gather_distances(const Params &p, const float *
     }
     return out;
   } else {
-    return gather_rows<METRIC, STORAGE>(p.rows, p.row_bytes, p.scale_off, p.width, qv, m, cid, lane);
+    return gather_rows<METRIC, STORAGE, LONG>(p.rows, p.row_bytes, p.scale_off, p.width, qv, m, cid, lane);
   }
 }
 
@@ -360,17 +368,17 @@ struct Team {
 
 // Warp `wib`'s share of a gather: candidates 8 wib .. of the m listed from
 // cbuf[at] on.
-template <int METRIC, int STORAGE>
+template <int METRIC, int STORAGE, bool LONG>
 __device__ __forceinline__ void team_pass(const Params &p, const WarpCtx &w, const Team &t, int m, int at, int wib,
                                           int lane) {
   const int c = 8 * wib + (lane >> 2);
   if (8 * wib >= m) return;  // whole warp
-  const float d = rows_pass<METRIC, STORAGE>(p.rows, p.row_bytes, p.scale_off, p.width, w.qv,
+  const float d = rows_pass<METRIC, STORAGE, LONG>(p.rows, p.row_bytes, p.scale_off, p.width, w.qv,
                                              w.cbuf[at + min(c, m - 1)], lane);
   if ((lane & 3) == 0 && c < m) t.dist[c] = d;
 }
 
-template <int METRIC, int STORAGE, bool LEARNED>
+template <int METRIC, int STORAGE, bool LEARNED, bool LONG>
 __device__ __forceinline__ void team_help(const Params &p, const WarpCtx &w, Team t, int wib, int lane) {
   const auto vh = VisitedOf<LEARNED>::make(w.tab, p.pq);
   for (;;) {
@@ -378,7 +386,7 @@ __device__ __forceinline__ void team_help(const Params &p, const WarpCtx &w, Tea
     const int c = t.next(&arg);
     if (c == Team::STOP) return;
     if (c > 0) {
-      team_pass<METRIC, STORAGE>(p, w, t, c, arg, wib, lane);
+      team_pass<METRIC, STORAGE, LONG>(p, w, t, c, arg, wib, lane);
       Team::barrier();
       continue;
     }
@@ -441,7 +449,7 @@ __device__ __forceinline__ void select_insert(Queue &Q, VH &vh, int m, uint64_t 
 // (LEARNED) receives the per-hop features or is null.  False if a bulk copy
 // never completed.  MULTI: the reference's N_MULTIPROBE / FINISH_CNT knobs
 // (p.probes, p.finish_cnt) as run-time values.
-template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false, bool TEAM = false>
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false, bool TEAM = false, bool LONG = false>
 __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const float *qsrc, const uint32_t *starts,
                                           int ns, int pq, int k, uint64_t *o, float *trace, QueryStats &st,
                                           int lane, const uint32_t *qcode = nullptr, Team *team = nullptr) {
@@ -475,7 +483,7 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
   vh.clear(lane);
 
   // warp_astar_accelerator.h:115-176: distances to the starts, queue = {starts}.
-  float cd = gather_distances<METRIC, STORAGE>(p, w.qv, ns, sid, lane, qc);
+  float cd = gather_distances<METRIC, STORAGE, LONG>(p, w.qv, ns, sid, lane, qc);
   const float d0 = __shfl_sync(FULL, cd, 0);
   uint32_t a_next;
   if (bulk) {
@@ -542,23 +550,27 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
     if constexpr (TEAM) {
       if (m > 8) {
         team->call(m, at, lane);
-        team_pass<METRIC, STORAGE>(p, w, *team, m, at, 0, lane);
+        team_pass<METRIC, STORAGE, LONG>(p, w, *team, m, at, 0, lane);
         Team::barrier();
         return lane < m ? team->dist[lane] : 0.0f;
       }
     }
-    // The rows past the first pass start their way into L2 (rows of 512 bytes
-    // and more: 1M x 128, 10,000 queries at pq 43 1193 -> 1161 us, at pq 100
-    // from vertex 0 4.61 -> 4.41 ms; no gain on shorter ones, and the learned
-    // kernels lose registers to it: 959 -> 1025 us).
-    if constexpr (!LEARNED && !TEAM && STORAGE <= 1) {
-      if (lane >= 8 && lane < m && p.row_bytes >= 512) {
+    // What the first pass does not load at once starts its way into L2: the
+    // rows past it (512-byte rows: 1M x 128, 10,000 queries at pq 43 1193 ->
+    // 1161 us, at pq 100 from vertex 0 4.61 -> 4.41 ms; no gain on shorter
+    // ones, and the learned and multi-probe kernels lose registers to it: 959
+    // -> 1025 us), and of long rows, in every kernel, also the first eight's ends
+    // (1000 queries of 960-d rows with the exit network 2853 -> 2421 us).
+    if constexpr (!TEAM && STORAGE <= 1 && (LONG || (!LEARNED && !MULTI))) {
+      constexpr uint32_t first = 32u * row_steps<STORAGE, LONG>() * (STORAGE == 0 ? 4u : 2u);
+      if (lane < m && (LONG || (lane >= 8 && p.row_bytes >= 512))) {
         const uint8_t *row = p.rows + static_cast<uint64_t>(cid) * p.row_bytes;
-        for (uint32_t b = 0; b < p.row_bytes; b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + b));
+        for (uint32_t b = LONG && lane < 8 ? first : 0u; b < p.row_bytes; b += 128)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(row + b));
       }
       __syncwarp();
     }
-    return gather_distances<METRIC, STORAGE>(p, w.qv, m, cid, lane, qc);
+    return gather_distances<METRIC, STORAGE, LONG>(p, w.qv, m, cid, lane, qc);
   };
 
   int finished = 0;  // MULTI: finish tests that held (finished[cid], :190-192)
@@ -767,24 +779,33 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
   return true;
 }
 
-// Resident blocks of four warps asked for: 5 while the queues are small (S <=
-// 4: 96 registers; 6 blocks, at 80, cost 25 % of a
-// small batch's time, 1000 queries of 1M x 128 from entry points at pq 43 287
-// -> 362 us, for 1 % of a full one's), 4 for the wider register queue of S = 8
-// and the lists of S = 16, 2 beyond, where shared memory holds eight warps at
-// most.
-template <int S>
+// Resident blocks of four warps asked for.  Short rows: 5 while the queues are
+// small (S <= 4: 96 registers; 6 blocks, at 80, cost 25 % of a small batch's
+// time, 1000 queries of 1M x 128 from entry points at pq 43 287 -> 362 us, for
+// 1 % of a full one's), 4 for the wider register queue of S = 8 and the lists
+// of S = 16, 2 beyond, where shared memory holds eight warps at most.  The
+// multi-probe kernels, whose double check is one long chain, take 6 (10,000
+// queries of 1M x 128, two probes: 1489 us with 5, 1414 with 6), the learned
+// ones on BF16 rows 4 (their decoding spills at 96 registers: 1765 us with 5,
+// 1511 with 4).  LONG rows (1 KB and more): 3, for the 64 registers that a
+// pass's loads take: 10,000 queries of 256-d rows from vertex 0 at pq 75 3.13
+// ms with 5 blocks and half the loads in flight, 2.53 with 4, 2.78 with 3; 1000
+// of 960-d rows 2.51, 2.33 and 1.70; 10,000 of 128-d rows at pq 43 1.16 with 5
+// blocks, 1.50 with 3.
+constexpr uint32_t LONG_ROW = 1024;
+
+template <int STORAGE, int S, bool LEARNED, bool MULTI, bool LONG>
 struct MinBlocks {
-  static constexpr int value = S > 16 ? 2 : (S > 4 ? 4 : 5);
+  static constexpr int value = S > 16 ? 2 : LONG ? 3 : S > 4 ? 4 : MULTI ? 6 : LEARNED && STORAGE == 1 ? 4 : 5;
 };
 
 // Query qid of the launch; false if a bulk copy never completed.
-template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI, bool TEAM>
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI, bool TEAM, bool LONG>
 __device__ __forceinline__ bool search_one(const Params &p, WarpCtx &w, uint32_t qid, int lane, Team *team) {
   float *trace = nullptr;
   if (LEARNED && p.trace) trace = p.trace + static_cast<size_t>(qid) * p.trace_hops * TRACE_FIELDS;
   QueryStats st;
-  if (!run_query<METRIC, STORAGE, S, LEARNED, MULTI, TEAM>(
+  if (!run_query<METRIC, STORAGE, S, LEARNED, MULTI, TEAM, LONG>(
           p, w, p.queries + static_cast<size_t>(qid) * p.dim,
           p.starts ? p.starts + static_cast<size_t>(qid) * p.n_starts : nullptr, p.n_starts, p.pq, p.k,
           p.out + static_cast<size_t>(qid) * p.k, trace, st, lane,
@@ -811,8 +832,8 @@ __device__ __forceinline__ void load_mlp(const Params &p, __nv_bfloat16 *wmlp) {
   __syncthreads();
 }
 
-template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false>
-__global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, MinBlocks<S>::value)
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI, bool LONG>
+__global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, MinBlocks<STORAGE, S, LEARNED, MULTI, LONG>::value)
     search_kernel(const Params p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int lane = threadIdx.x & 31;
@@ -829,12 +850,12 @@ __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, MinBlocks<S>::value)
     if (lane == 0) qid = atomicAdd(p.counter, 1u);
     qid = __shfl_sync(FULL, qid, 0);
     if (qid >= static_cast<uint32_t>(p.nq)) break;
-    if (!search_one<METRIC, STORAGE, S, LEARNED, MULTI, false>(p, w, qid, lane, nullptr)) return;
+    if (!search_one<METRIC, STORAGE, S, LEARNED, MULTI, false, LONG>(p, w, qid, lane, nullptr)) return;
   }
 }
 
 // The search with a block per query (Team).
-template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI>
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI, bool LONG>
 __global__ void __launch_bounds__(TEAM_WARPS * 32, S > 16 ? 2 : 4) search_team_kernel(const Params p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -846,11 +867,11 @@ __global__ void __launch_bounds__(TEAM_WARPS * 32, S > 16 ? 2 : 4) search_team_k
   w.wmlp = wmlp;
   if (LEARNED) load_mlp(p, wmlp);
   if (wib > 0) {
-    team_help<METRIC, STORAGE, LEARNED>(p, w, team, wib, lane);
+    team_help<METRIC, STORAGE, LEARNED, LONG>(p, w, team, wib, lane);
     return;
   }
   for (uint32_t qid = blockIdx.x; qid < static_cast<uint32_t>(p.nq); qid += gridDim.x)
-    if (!search_one<METRIC, STORAGE, S, LEARNED, MULTI, true>(p, w, qid, lane, &team)) break;
+    if (!search_one<METRIC, STORAGE, S, LEARNED, MULTI, true, LONG>(p, w, qid, lane, &team)) break;
   team.call(Team::STOP, 0, lane);
 }
 
@@ -864,12 +885,12 @@ int get_shape(const void *fn, uint32_t warp_bytes, uint32_t extra_bytes, int *wp
 // The same for blocks of a fixed size and footprint: how many fit on the GPU.
 int get_team_shape(const void *fn, uint32_t bytes, int *grid_cap);
 
-template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI = false>
+template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI, bool LONG>
 int launch_kernel(const Params &p, cudaStream_t stream) {
   const uint32_t extra = LEARNED ? static_cast<uint32_t>(MLP_NPARAM * sizeof(__nv_bfloat16) + 64) : 0u;
   if constexpr (STORAGE != 3) {
     // a block per query while all of them run at once
-    auto team = search_team_kernel<METRIC, STORAGE, S, LEARNED, MULTI>;
+    auto team = search_team_kernel<METRIC, STORAGE, S, LEARNED, MULTI, LONG>;
     const uint32_t bytes = p.warp_bytes + TEAM_BYTES + extra;
     int cap = 0;
     int e = get_team_shape(reinterpret_cast<const void *>(team), bytes, &cap);
@@ -878,7 +899,7 @@ int launch_kernel(const Params &p, cudaStream_t stream) {
       return cudaGetLastError();
     }
   }
-  auto kern = search_kernel<METRIC, STORAGE, S, LEARNED, MULTI>;
+  auto kern = search_kernel<METRIC, STORAGE, S, LEARNED, MULTI, LONG>;
   int wpb = 0, cap = 0;
   int e = get_shape(reinterpret_cast<const void *>(kern), p.warp_bytes, extra, &wpb, &cap);
   if (e != 0) return e;
@@ -890,36 +911,41 @@ int launch_kernel(const Params &p, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-template <int STORAGE, int METRIC, bool LEARNED, bool MULTI = false>
+template <int STORAGE, int METRIC, bool LEARNED, bool MULTI, bool LONG>
 int launch_by_s(const Params &p, int S, cudaStream_t s) {
   switch (S) {
-    case 1: return launch_kernel<METRIC, STORAGE, 1, LEARNED, MULTI>(p, s);
-    case 2: return launch_kernel<METRIC, STORAGE, 2, LEARNED, MULTI>(p, s);
-    case 4: return launch_kernel<METRIC, STORAGE, 4, LEARNED, MULTI>(p, s);
-    case 8: return launch_kernel<METRIC, STORAGE, 8, LEARNED, MULTI>(p, s);
-    case 16: return launch_kernel<METRIC, STORAGE, 16, LEARNED, MULTI>(p, s);
-    case 32: return launch_kernel<METRIC, STORAGE, 32, LEARNED, MULTI>(p, s);
+    case 1: return launch_kernel<METRIC, STORAGE, 1, LEARNED, MULTI, LONG>(p, s);
+    case 2: return launch_kernel<METRIC, STORAGE, 2, LEARNED, MULTI, LONG>(p, s);
+    case 4: return launch_kernel<METRIC, STORAGE, 4, LEARNED, MULTI, LONG>(p, s);
+    case 8: return launch_kernel<METRIC, STORAGE, 8, LEARNED, MULTI, LONG>(p, s);
+    case 16: return launch_kernel<METRIC, STORAGE, 16, LEARNED, MULTI, LONG>(p, s);
+    case 32: return launch_kernel<METRIC, STORAGE, 32, LEARNED, MULTI, LONG>(p, s);
     default: return -1;
   }
 }
 
-template <int STORAGE, bool LEARNED, bool MULTI = false>
+template <int STORAGE, bool LEARNED, bool MULTI = false, bool LONG = false>
 int launch_storage(const Params &p, int metric, int S, cudaStream_t s) {
   switch (metric) {
-    case 0: return launch_by_s<STORAGE, 0, LEARNED, MULTI>(p, S, s);
-    case 1: return launch_by_s<STORAGE, 1, LEARNED, MULTI>(p, S, s);
-    case 2: return launch_by_s<STORAGE, 2, LEARNED, MULTI>(p, S, s);
+    case 0: return launch_by_s<STORAGE, 0, LEARNED, MULTI, LONG>(p, S, s);
+    case 1: return launch_by_s<STORAGE, 1, LEARNED, MULTI, LONG>(p, S, s);
+    case 2: return launch_by_s<STORAGE, 2, LEARNED, MULTI, LONG>(p, S, s);
     default: return -1;
   }
 }
 
 // One per translation unit (search_f32.cu, search_bf16.cu, search_fp8.cu,
-// search_bits.cu, search_learned.cu, search_multi.cu).
+// search_bits.cu, search_learned.cu, search_multi.cu, and search_*_long.cu for
+// rows of LONG_ROW bytes and more).
 int launch_f32(const Params &p, int metric, int S, cudaStream_t s);
 int launch_bf16(const Params &p, int metric, int S, cudaStream_t s);
 int launch_fp8(const Params &p, int metric, int S, cudaStream_t s);
 int launch_bits(const Params &p, int metric, int S, cudaStream_t s);
 int launch_learned(const Params &p, int storage, int metric, int S, cudaStream_t s);
 int launch_multi(const Params &p, int metric, int S, cudaStream_t s);
+int launch_f32_long(const Params &p, int metric, int S, cudaStream_t s);
+int launch_bf16_long(const Params &p, int metric, int S, cudaStream_t s);
+int launch_learned_long(const Params &p, int storage, int metric, int S, cudaStream_t s);
+int launch_multi_long(const Params &p, int metric, int S, cudaStream_t s);
 
 }  // namespace song

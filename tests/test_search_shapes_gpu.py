@@ -89,3 +89,24 @@ def test_multi_probe_and_learned_batches(song, oracle, pq):
         ix.set_multiprobe()
         ix.set_hop_limit(1 << 30)
         _check(ix, q, pq, ox.kernel_search(q, pq, oracle.MODE_LEX_EXACT), "learned")
+
+
+@pytest.mark.parametrize("dim", [252, 253, 256, 288, 508, 512, 516, 961])
+def test_long_rows(song, oracle, dim):
+    """Rows around 1 KB and longer, where another instance of each kernel
+    reads them: FP32 from 253 dimensions, BF16 from 505."""
+    data, q = _clustered(900, dim, seed=dim)
+    g = _ring_graph(song, data, 0, 4, seed=dim)
+    for storage in ("f32", "bf16"):
+        with song.Index(g, data, 4, 0, storage=storage) as ix:
+            ix.set_rerank(0)
+            ox = oracle.OracleIndex(song.dequantize_rows(ix.rows(), storage, dim), g, 4, 0)
+            for pq in (20, 140, 270, 520):
+                _check(ix, q, pq, ox.kernel_search(q, pq, oracle.MODE_LEX), (storage, pq))
+            if storage == "f32":
+                ix.set_multiprobe(2, 1, True)
+                want = ox.kernel_search(q, 50, oracle.MODE_LEX, probes=2, finish_cnt=1, double_check=True)
+                _check(ix, q, 50, want, "multi")
+                ix.set_multiprobe()
+            ix.set_hop_limit(1 << 30)
+            _check(ix, q, 50, ox.kernel_search(q, 50, oracle.MODE_LEX_EXACT), (storage, "learned"))
