@@ -31,7 +31,7 @@
 //
 // What bounds it: instructions, in full batches and for a single query alike
 // (about six cycles each on a dependent path).  A hop of the headline search
-// (1M x 128 L2, pq 43 from entry points, 21 candidates) takes 2,000 of them
+// (1M x 128 L2, pq 43 from entry points, 21 candidates) takes 1,790 of them
 // (2,650 before its rows were read directly and its hash calls made side by
 // side), one at pq 1000 from vertex 0 500 (5,900).
 #pragma once
@@ -791,12 +791,18 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
 // pass's loads take: 10,000 queries of 256-d rows from vertex 0 at pq 75 3.13
 // ms with 5 blocks and half the loads in flight, 2.53 with 4, 2.78 with 3; 1000
 // of 960-d rows 2.51, 2.33 and 1.70; 10,000 of 128-d rows at pq 43 1.16 with 5
-// blocks, 1.50 with 3.
+// blocks, 1.50 with 3.  Their multi-probe and learned kernels take 4 while pq <
+// 32, where loading is less of a hop (10,000 of 256-d rows at pq 30, four
+// probes: 3.22 ms with 3, 2.79 with 4; at pq 55 3.82 and 3.97).
 constexpr uint32_t LONG_ROW = 1024;
 
 template <int STORAGE, int S, bool LEARNED, bool MULTI, bool LONG>
 struct MinBlocks {
-  static constexpr int value = S > 16 ? 2 : LONG ? 3 : S > 4 ? 4 : MULTI ? 6 : LEARNED && STORAGE == 1 ? 4 : 5;
+  static constexpr int value = S > 16 ? 2
+                               : LONG ? (S == 1 && STORAGE == 0 && (MULTI || LEARNED) ? 4 : 3)
+                               : S > 4 ? 4
+                               : MULTI ? 6
+                               : LEARNED && STORAGE == 1 ? 4 : 5;
 };
 
 // Query qid of the launch; false if a bulk copy never completed.
