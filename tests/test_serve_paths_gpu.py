@@ -1,0 +1,41 @@
+"""The server's own path where it can part from the batched search's: the time
+of one request, which runs the same hops as one search."""
+import time
+
+import numpy as np
+import pytest
+
+from conftest import load_golden
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("name", ["l2_s5_d32", "cos_s4_d16"])
+def test_one_request_takes_about_one_search(song, name):
+    """One query through the server (a warp runs it, the host polls) against
+    one query through song_search (a block of four warps, two copies).  Both
+    make the same hops; a warp whose lanes go through them apart takes more
+    than four times as long.  3 lies between that and the 1.5 to be expected."""
+    from song_gb300.serve import Server
+    g = load_golden(name)
+    q = np.ascontiguousarray(g["queries"][:1])
+
+    def best(call, reps=60):
+        t = []
+        for _ in range(reps):
+            t0 = time.perf_counter()
+            call()
+            t.append(time.perf_counter() - t0)
+        return min(t[reps // 2:])
+
+    with song.Index(g["graph"], g["data"], int(g["shift"]), int(g["metric"])) as ix:
+        alone = best(lambda: ix.search(q, 100, 10))
+        with Server(ix, max_pq=100, max_k=10, slots=4, slot_queries=8, sm_fraction=0.25) as srv:
+            def request():
+                t = srv.submit(q, 100, 10)
+                while t not in srv.poll():
+                    pass
+                srv.result(t, 1, 10)
+            served = best(request)
+    print("\n[serve] one search %.0f us, one request %.0f us" % (1e6 * alone, 1e6 * served))
+    assert served < 3 * alone
