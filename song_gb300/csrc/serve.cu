@@ -96,7 +96,8 @@ __device__ __forceinline__ void serve_choose_starts(const Params &p, const float
     int h = 0;
     uint32_t mine = 0;
     for (int r = 0; r < p.n_probes; ++r) {
-      const uint32_t c = list_take<NL>(hd, hi, h);
+      uint32_t c = list_take<NL>(hd, hi, h);
+      if (c >= static_cast<uint32_t>(p.n_coarse)) c = 0u;  // no finite distance (a query that is not finite)
       if (lane == r) mine = c;
     }
     for (int r = 0; r < p.n_probes; ++r) {
@@ -118,7 +119,8 @@ __device__ __forceinline__ void serve_choose_starts(const Params &p, const float
   int h = 0;
   for (int r = 0; r < p.n_starts; ++r) {
     const uint32_t id = list_take<NL>(bd, bi, h);
-    if (lane == 0) out[r] = id;
+    // no finite distance (a query that is not finite): vertex 0
+    if (lane == 0) out[r] = id == 0xffffffffu ? 0u : id;
   }
   __syncwarp();
 }

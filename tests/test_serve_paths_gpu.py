@@ -1,5 +1,6 @@
 """The server's own path where it can part from the batched search's: the time
-of one request, which runs the same hops as one search."""
+of one request, which runs the same hops as one search, and the starts of a
+query that has no finite distance to any entry vertex."""
 import time
 
 import numpy as np
@@ -39,3 +40,29 @@ def test_one_request_takes_about_one_search(song, name):
             served = best(request)
     print("\n[serve] one search %.0f us, one request %.0f us" % (1e6 * alone, 1e6 * served))
     assert served < 3 * alone
+
+
+@pytest.mark.parametrize("kind", ["flat", "two_level"])
+@pytest.mark.parametrize("name", ["l2_s5_d32", "ip_s5_d24", "cos_s4_d16"])
+def test_queries_that_are_not_finite_start_at_vertex_0(song, name, kind):
+    """NaN has no nearest entry: the server and the search both start such a
+    query at vertex 0 (with one start: the search without entry points)."""
+    from song_gb300.serve import Server
+    g = load_golden(name)
+    q = np.ascontiguousarray(g["queries"][:6])
+    q[1, :] = np.nan
+    q[3, 2] = np.nan
+    q[4, 1] = np.inf
+    ent = np.random.default_rng(2).choice(len(g["data"]), 200, replace=False).astype(np.uint64)
+    with song.Index(g["graph"], g["data"], int(g["shift"]), int(g["metric"])) as ix:
+        plain = ix.search(q, 30, 10)
+        for starts in (1, 3):
+            ix.set_entries(ent, starts=starts, **(dict(coarse=12, probes=3) if kind == "two_level" else {}))
+            alone = ix.search(q, 30, 10)
+            with Server(ix, max_pq=40, max_k=10, slots=2, slot_queries=8, sm_fraction=0.25) as srv:
+                t = srv.submit(q, 30, 10)
+                srv.wait(t, 10_000)
+                assert np.array_equal(srv.result(t, len(q), 10), alone), starts
+            if starts == 1:
+                assert np.array_equal(alone[[1, 3]], plain[[1, 3]])
+            ix.set_entries(None)
