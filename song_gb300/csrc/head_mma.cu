@@ -34,6 +34,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cstdint>
 #include <cstring>
 
@@ -350,7 +351,8 @@ __global__ void __launch_bounds__(128, 1)
         } else {
           float lo = __int_as_float(0x7f800000), hi = lo;
           if (col0 + i < a.n_heads) head_interval<METRIC>(s, qn2, qn, hx2[32 * j + i], hx[32 * j + i], lo, hi);
-          o[i] = lo;
+          // a bound that is not a number (norms that overflow) bounds nothing: -inf
+          o[i] = fmaxf(lo, -__int_as_float(0x7f800000));
           // the tile's NP smallest upper bounds (values only)
           if (hi < best[NP - 1]) {
             float x = hi;
@@ -445,6 +447,9 @@ __global__ void __launch_bounds__(HM_SEL_WARPS * 32, 3)
       uint32_t wid;
       warp_take<NP>(hb, hid, hp, U, wid);
     }
+    // the places past the heads hold +inf: no shortlist takes them, also when
+    // no upper bound is finite (a query whose squared norm overflows)
+    U = fminf(U, FLT_MAX);
   }
   // the shortlist: every head whose lower bound is <= U, four 16-byte
   // groups of eight BF16 bounds per lane in flight
@@ -491,7 +496,8 @@ __global__ void __launch_bounds__(HM_SEL_WARPS * 32, 3)
   // the first lane of a row keeps it
   for (int g = 0; g < total; g += 8) {
     const int i = min(g + (lane >> 2), total - 1);
-    const uint32_t head = full_scan ? static_cast<uint32_t>(i) : cand[w][i];
+    // (bounds that a timed-out score kernel never wrote may name any place)
+    const uint32_t head = full_scan ? static_cast<uint32_t>(i) : min(cand[w][i], static_cast<uint32_t>(n_heads - 1));
     float d[1];
     rows8_distance<METRIC, 1>(heads + static_cast<size_t>(head) * dpad, qv, qs, dpad, d, lane);
     if (g + (lane >> 2) < total && (lane & 3) == 0) best_insert<NP>(bd, bi, d[0], head);
