@@ -327,6 +327,12 @@ int song_search_noalloc(song_index *index, const float *queries, int nq, int pq,
  * SONG_ERR_TIMEOUT and the index stays usable.  song_debug_server_hold(1):
  * admitted requests are kept from the kernel until song_debug_server_hold(0). */
 int song_debug_fail_alloc(int n);
+/* Shared memory of a search, on the host alone: *accepted_by, the bytes a warp
+ * by which song_search accepts the size (at most 227 KB), and *used, those of
+ * the kernel's smallest block (learned: the kernel of the early exit and of
+ * tracing; multi: the multi-probe kernel). */
+int song_debug_shared_bytes(int storage, int dim, int pq, int learned, int multi, uint32_t *accepted_by,
+                            uint32_t *used);
 int song_debug_set_wait(song_index *index, uint32_t wait_limit, uint32_t extra_tx);
 int song_debug_server_hold(song_server *server, int hold);
 

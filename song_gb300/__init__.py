@@ -49,7 +49,7 @@ EXPORTED = [
     "song_index_set_hash_planes",
     "song_server_set_idle_polls", "song_server_running", "song_server_wait", "song_debug_fail_alloc",
     "song_debug_set_wait", "song_debug_server_hold", "song_debug_head_path", "song_debug_head_stats",
-    "song_debug_head_scores",
+    "song_debug_head_scores", "song_debug_shared_bytes",
 ]
 MLP_PARAMS = 1281
 TRACE_FIELDS = 6
@@ -152,6 +152,8 @@ def load_library():
     L.song_server_running.argtypes = [P, ctypes.POINTER(i32)]
     L.song_server_wait.restype = i32
     L.song_server_wait.argtypes = [P, ctypes.c_uint64, i32]
+    L.song_debug_shared_bytes.restype = i32
+    L.song_debug_shared_bytes.argtypes = [i32, i32, i32, i32, i32, P, P]
     L.song_debug_fail_alloc.restype = i32
     L.song_debug_fail_alloc.argtypes = [i32]
     L.song_debug_set_wait.restype = i32
@@ -430,6 +432,15 @@ def hash_planes(dim, seed=123):
 def debug_fail_alloc(n):
     """Test hook: the n-th next device allocation of the library fails (0: none)."""
     _check(load_library().song_debug_fail_alloc(int(n)))
+
+
+def debug_shared_bytes(storage, dim, pq, learned=False, multi=False):
+    """(bytes by which a search of this size is accepted, bytes that the
+    kernel's smallest block takes)."""
+    a, b = ctypes.c_uint32(), ctypes.c_uint32()
+    _check(load_library().song_debug_shared_bytes(_storage(storage), int(dim), int(pq), int(bool(learned)),
+                                                  int(bool(multi)), ctypes.byref(a), ctypes.byref(b)))
+    return a.value, b.value
 
 
 def debug_fixhash(ids, pq):

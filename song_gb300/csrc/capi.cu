@@ -37,6 +37,25 @@ namespace {
 std::atomic<long long> g_fail_alloc{0};  // song_debug_fail_alloc: allocations left until one fails
 }  // namespace
 
+void set_row_layout(DeviceIndex &dx) {
+  const int dpad4 = (dx.dim + 3) / 4 * 4;
+  dx.f32_row_bytes = static_cast<uint32_t>(dpad4) * 4u;
+  if (dx.storage == SONG_STORAGE_F32) {
+    dx.dpad = dpad4;
+    dx.row_bytes = dx.f32_row_bytes;
+  } else if (dx.storage == SONG_STORAGE_BF16) {
+    dx.dpad = (dx.dim + 7) / 8 * 8;
+    dx.row_bytes = static_cast<uint32_t>(dx.dpad) * 2u;
+  } else if (dx.storage == SONG_STORAGE_BITS) {
+    dx.dpad = SONG_HASH_BITS / 32;  // code words
+    dx.row_bytes = SONG_HASH_BITS / 8;
+  } else {
+    dx.dpad = (dx.dim + 15) / 16 * 16;
+    dx.scale_off = static_cast<uint32_t>(dx.dpad);
+    dx.row_bytes = dx.scale_off + 16u;
+  }
+}
+
 cudaError_t dev_malloc(void **p, size_t bytes) {
   if (g_fail_alloc.load() > 0 && g_fail_alloc.fetch_sub(1) == 1) {
     *p = nullptr;
@@ -274,22 +293,7 @@ int song_index_create(const uint64_t *graph, const float *data, uint64_t n, int 
   dx.shift = shift;
   dx.metric = metric;
   dx.storage = storage;
-  const int dpad4 = (dim + 3) / 4 * 4;
-  dx.f32_row_bytes = static_cast<uint32_t>(dpad4) * 4u;
-  if (storage == SONG_STORAGE_F32) {
-    dx.dpad = dpad4;
-    dx.row_bytes = dx.f32_row_bytes;
-  } else if (storage == SONG_STORAGE_BF16) {
-    dx.dpad = (dim + 7) / 8 * 8;
-    dx.row_bytes = static_cast<uint32_t>(dx.dpad) * 2u;
-  } else if (storage == SONG_STORAGE_BITS) {
-    dx.dpad = SONG_HASH_BITS / 32;  // code words
-    dx.row_bytes = SONG_HASH_BITS / 8;
-  } else {
-    dx.dpad = (dim + 15) / 16 * 16;
-    dx.scale_off = static_cast<uint32_t>(dx.dpad);
-    dx.row_bytes = dx.scale_off + 16u;
-  }
+  song::set_row_layout(dx);
   auto bail = [&](int code) {
     release(ix);
     return code;
@@ -451,6 +455,21 @@ int song_debug_fail_alloc(int n) {
   g_last_error.clear();
   if (n < 0) return fail(SONG_ERR_ARG, "n must be >= 0");
   song::g_fail_alloc.store(n);
+  return SONG_OK;
+}
+
+int song_debug_shared_bytes(int storage, int dim, int pq, int learned, int multi, uint32_t *accepted_by,
+                            uint32_t *used) {
+  g_last_error.clear();
+  if (storage < SONG_STORAGE_F32 || storage > SONG_STORAGE_BITS || dim < 1 || dim > 65536 || pq < 2 ||
+      pq > SONG_MAX_PQ || !accepted_by || !used)
+    return fail(SONG_ERR_ARG, "bad arguments");
+  song::DeviceIndex dx;
+  dx.storage = storage;
+  dx.dim = dim;
+  song::set_row_layout(dx);
+  *accepted_by = song::search_warp_bytes(dx, pq, multi != 0);
+  *used = song::search_block_bytes(dx, pq, learned != 0, multi != 0);
   return SONG_OK;
 }
 

@@ -56,8 +56,13 @@ struct SearchCall {
 // -1 when the shape is unsupported; sets *smem_per_warp if non-null.
 int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t stream);
 
-// Shared-memory bytes one warp needs for (ix, pq).
+// dpad, row_bytes, scale_off and f32_row_bytes of dx.storage and dx.dim.
+void set_row_layout(DeviceIndex &dx);
+
+// Shared-memory bytes of a warp by which (ix, pq) is accepted, and those that
+// the kernel's smallest block takes.
 uint32_t search_warp_bytes(const DeviceIndex &ix, int pq, bool multi = false);
+uint32_t search_block_bytes(const DeviceIndex &ix, int pq, bool learned, bool multi);
 // Whether an index's knobs select the multi-probe kernel.
 inline bool multi_knobs(int probes, int finish_cnt, int double_check) {
   return probes > 1 || finish_cnt > 1 || double_check != 0;

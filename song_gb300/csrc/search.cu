@@ -110,14 +110,28 @@ int get_team_shape(const void *fn, uint32_t bytes, int *grid_cap) {
   return 0;
 }
 
-// What a warp may need, as the interface states it: two staging chunks of
-// the rows beside the query and the 8*pq-slot hash.  The kernel needs less,
-// at every size that this admits.
+// The accepted sizes, as the interface states them: two staging chunks of the
+// rows beside the query and the 8*pq-slot hash within a block's shared memory.
+// The kernel's own layout (warp_layout) has no staging, but the queue's ring,
+// the home slots and the sort's keys instead: more than this at small sizes,
+// which are far from the limit, and never above the limit where this is within
+// it (a CPU test goes through all storages, kernels and queue bounds).
 uint32_t search_warp_bytes(const DeviceIndex &ix, int pq, bool multi) {
   const uint32_t rows = ix.row_bytes <= 1024 ? (pq >= 512 ? 1u : 4u) : 2u;
   uint32_t off = align_up(2u * rows * ix.row_bytes, 16) + 16 + (multi ? MAX_PROBES : 1) * 32 * 4;
   off = align_up(off, 16) + align_up(static_cast<uint32_t>(ix.dim) * 4u, 16) + 4u * 8u * static_cast<uint32_t>(pq);
   return align_up(off, 128);
+}
+
+namespace {
+WarpLayout search_layout(const DeviceIndex &ix, int pq, bool learned, bool multi) {
+  return warp_layout(ix.dim, pq, queue_segment(pq), learned ? exact_cap(pq) : 8 * pq, (multi ? MAX_PROBES : 1) * 32,
+                     ix.storage == 3);
+}
+}  // namespace
+
+uint32_t search_block_bytes(const DeviceIndex &ix, int pq, bool learned, bool multi) {
+  return search_layout(ix, pq, learned, multi).warp_bytes + (learned ? MLP_BYTES : 0u);
 }
 
 int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t stream) {
@@ -126,7 +140,7 @@ int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t strea
   const bool multi = c.probes > 1 || c.finish_cnt > 1 || c.double_check;
   if (multi && (learned || ix.storage != 0 || c.probes > MAX_PROBES || c.finish_cnt < 1)) return -1;
   const int S = queue_segment(c.pq), cap = learned ? exact_cap(c.pq) : 8 * c.pq;
-  const WarpLayout L = warp_layout(ix.dim, c.pq, S, cap, (multi ? MAX_PROBES : 1) * 32);
+  const WarpLayout L = search_layout(ix, c.pq, learned, multi);
   Params p;
   p.rows = static_cast<const uint8_t *>(ix.rows);
   p.row_bytes = ix.row_bytes;
@@ -183,7 +197,9 @@ int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t strea
     case 0: return (lng ? launch_f32_long : launch_f32)(p, ix.metric, S, stream);
     case 1: return (lng ? launch_bf16_long : launch_bf16)(p, ix.metric, S, stream);
     case 2: return launch_fp8(p, ix.metric, S, stream);
-    case 3: return c.qcodes ? launch_bits(p, ix.metric, S, stream) : -1;  // query codes come from the caller's path
+    case 3:
+      if (!c.qcodes) return -1;  // they come from the caller's path
+      return (L.late ? launch_bits_wide : launch_bits)(p, ix.metric, S, stream);
     default: return -1;
   }
 }

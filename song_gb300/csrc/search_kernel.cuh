@@ -27,7 +27,8 @@
 // 2 FP8-E4M3 with a per-row scale, 3 256-bit codes), S (register queue
 // segment, capacity 32*S >= pq+1), LEARNED (per-hop features: trace capture
 // and/or the early-exit network), MULTI (the multi-probe knobs), LONG (rows of
-// LONG_ROW bytes and more).
+// LONG_ROW bytes and more; with codes, vectors too wide for WarpLayout's usual
+// order).
 //
 // What bounds it: instructions, in full batches and for a single query alike
 // (about six cycles each on a dependent path).  A hop of the headline search
@@ -41,6 +42,7 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -62,6 +64,7 @@ constexpr int MLP_B2 = MLP_W2 + MLP_H * MLP_H;   // [MLP_H]
 constexpr int MLP_W3 = MLP_B2 + MLP_H;           // [MLP_H]
 constexpr int MLP_B3 = MLP_W3 + MLP_H;           // [1]
 constexpr int MLP_NPARAM = MLP_B3 + 1;
+constexpr uint32_t MLP_BYTES = MLP_NPARAM * sizeof(__nv_bfloat16) + 64;  // a block's copy
 constexpr int TRACE_FIELDS = 6;  // 5 features + top-k version
 
 struct Params {
@@ -274,20 +277,37 @@ struct QueueOf {
 // Shared memory of one warp, in this order: the first adjacency row (bulk
 // copy), its barrier, the candidate ids and home slots, the query, the
 // queue's ring, and the visited hash, which the answer's sort reuses (8 bytes
-// for each of 32*S keys).
+// for each of 32*S keys).  Codes leave the FP32 query for the re-rank only:
+// where it does not fit beside the rest (50,000 floats and the ring of pq
+// 1000), it is staged once the search is done, over all but the barrier, after
+// the sort's keys (`late`: the LONG kernels of codes).  Not at every size: the
+// pointers it needs to the end cost spills (5000 queries of 15k x 16 at pq 100
+// 1440 -> 1500 us).
+constexpr uint32_t MAX_BLOCK_BYTES = 227u * 1024u;
+constexpr uint32_t LATE_ROW = 16;  // late: the row's place, after the barrier
 struct WarpLayout {
   uint32_t warp_bytes, off_mbar, off_cand, off_q, off_queue, off_hash;
+  bool late;
 };
-inline WarpLayout warp_layout(int dim, int pq, int S, int cap, int cands) {
+inline WarpLayout warp_layout(int dim, int pq, int S, int cap, int cands, bool codes) {
   auto up = [](uint32_t x, uint32_t a) { return (x + a - 1) / a * a; };
+  const uint32_t query = 4u * up(static_cast<uint32_t>(dim), 32), ring = S >= BUF_S ? BufQueue::bytes(pq) : 0u;
+  const uint32_t hash = 4u * static_cast<uint32_t>(cap), sort = 256u * static_cast<uint32_t>(S);
   WarpLayout L;
   L.off_mbar = 128;
   L.off_cand = L.off_mbar + 16;
   L.off_q = L.off_cand + 8u * static_cast<uint32_t>(cands);
-  L.off_queue = up(L.off_q + 4u * up(static_cast<uint32_t>(dim), 32), 16);
-  L.off_hash = up(L.off_queue + (S >= BUF_S ? BufQueue::bytes(pq) : 0u), 16);
-  const uint32_t hash = 4u * static_cast<uint32_t>(cap), sort = 256u * static_cast<uint32_t>(S);
-  L.warp_bytes = up(L.off_hash + (hash > sort ? hash : sort), 128);
+  L.off_queue = up(L.off_q + query, 16);
+  L.off_hash = up(L.off_queue + ring, 16);
+  L.warp_bytes = up(L.off_hash + std::max(hash, sort), 128);
+  L.late = codes && L.warp_bytes > MAX_BLOCK_BYTES;
+  if (L.late) {
+    L.off_mbar = 0;
+    L.off_queue = up(L.off_q, 16);
+    L.off_hash = up(L.off_queue + ring, 16);
+    L.off_q = LATE_ROW + sort;
+    L.warp_bytes = up(std::max(L.off_hash + hash, L.off_q + query), 128);
+  }
   return L;
 }
 
@@ -303,8 +323,8 @@ struct WarpCtx {
   const __nv_bfloat16 *wmlp;
   uint32_t ph;
 
-  __device__ __forceinline__ void init(uint8_t *ws, const Params &p, int cands, int lane) {
-    row = reinterpret_cast<uint32_t *>(ws);
+  __device__ __forceinline__ void init(uint8_t *ws, const Params &p, int cands, int lane, uint32_t row_at = 0) {
+    row = reinterpret_cast<uint32_t *>(ws + row_at);
     mbar = reinterpret_cast<uint64_t *>(ws + p.off_mbar);
     cbuf = reinterpret_cast<uint32_t *>(ws + p.off_cand);
     chome = reinterpret_cast<int32_t *>(cbuf + cands);
@@ -479,7 +499,11 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
       bulk_g2s(w.row, p.adj + (static_cast<uint64_t>(next_id) << p.shift), 4u << p.shift, w.mbar);
     }
   }
-  for (int j = lane; j < ((p.dim + 31) & ~31); j += 32) w.qv[j] = j < p.dim ? qsrc[j] : 0.0f;
+  auto stage_query = [&] {
+    for (int j = lane; j < ((p.dim + 31) & ~31); j += 32) w.qv[j] = j < p.dim ? qsrc[j] : 0.0f;
+  };
+  constexpr bool late = STORAGE == 3 && LONG;
+  if (!late) stage_query();
   vh.clear(lane);
 
   // warp_astar_accelerator.h:115-176: distances to the starts, queue = {starts}.
@@ -739,8 +763,9 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
   }
 
   // :331-335 the list's first k ids, ascending; slots past its length get
-  // UINT64_MAX.  The keys are sorted where the visited hash was.
-  uint64_t *keys = reinterpret_cast<uint64_t *>(w.tab);
+  // UINT64_MAX.  The keys are sorted where the visited hash was (late: from
+  // the adjacency row on).
+  uint64_t *keys = late ? reinterpret_cast<uint64_t *>(w.row) : reinterpret_cast<uint64_t *>(w.tab);
   int live = tn;  // keys that can be returned
   __syncwarp();
   if constexpr (LEARNED) {
@@ -757,6 +782,10 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
   if (STORAGE != 0 && p.rerank > 0) {
     // FP32 re-rank of the best `rerank` entries of the list, then the first k.
     const int R = min(max(p.rerank, k), tn);
+    if (late) {
+      stage_query();
+      __syncwarp();
+    }
     if (!LEARNED && R < tn) warp_sort_shared(keys, 32 * S, lane);
     for (int base = 0; base < R; base += 32) {
       const int cnt = min(32, R - base);
@@ -850,7 +879,8 @@ __global__ void __launch_bounds__(MAX_WARPS_PER_BLOCK * 32, MinBlocks<STORAGE, S
   const int wib = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
   WarpCtx w;
-  w.init(smem_raw + static_cast<size_t>(wib) * p.warp_bytes, p, (MULTI ? MAX_PROBES : 1) * 32, lane);
+  w.init(smem_raw + static_cast<size_t>(wib) * p.warp_bytes, p, (MULTI ? MAX_PROBES : 1) * 32, lane,
+         STORAGE == 3 && LONG ? LATE_ROW : 0u);
   __nv_bfloat16 *wmlp = reinterpret_cast<__nv_bfloat16 *>(smem_raw + static_cast<size_t>(nwarps) * p.warp_bytes);
   w.wmlp = wmlp;
   if (LEARNED) load_mlp(p, wmlp);
@@ -897,7 +927,7 @@ int get_team_shape(const void *fn, uint32_t bytes, int *grid_cap);
 
 template <int METRIC, int STORAGE, int S, bool LEARNED, bool MULTI, bool LONG>
 int launch_kernel(const Params &p, cudaStream_t stream) {
-  const uint32_t extra = LEARNED ? static_cast<uint32_t>(MLP_NPARAM * sizeof(__nv_bfloat16) + 64) : 0u;
+  const uint32_t extra = LEARNED ? MLP_BYTES : 0u;
   if constexpr (STORAGE != 3) {
     // a block per query while all of them run at once
     auto team = search_team_kernel<METRIC, STORAGE, S, LEARNED, MULTI, LONG>;
@@ -946,11 +976,13 @@ int launch_storage(const Params &p, int metric, int S, cudaStream_t s) {
 
 // One per translation unit (search_f32.cu, search_bf16.cu, search_fp8.cu,
 // search_bits.cu, search_learned.cu, search_multi.cu, and search_*_long.cu for
-// rows of LONG_ROW bytes and more).
+// rows of LONG_ROW bytes and more, search_bits_wide.cu for WarpLayout's late
+// query).
 int launch_f32(const Params &p, int metric, int S, cudaStream_t s);
 int launch_bf16(const Params &p, int metric, int S, cudaStream_t s);
 int launch_fp8(const Params &p, int metric, int S, cudaStream_t s);
 int launch_bits(const Params &p, int metric, int S, cudaStream_t s);
+int launch_bits_wide(const Params &p, int metric, int S, cudaStream_t s);
 int launch_learned(const Params &p, int storage, int metric, int S, cudaStream_t s);
 int launch_multi(const Params &p, int metric, int S, cudaStream_t s);
 int launch_f32_long(const Params &p, int metric, int S, cudaStream_t s);

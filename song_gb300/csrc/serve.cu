@@ -427,7 +427,7 @@ int song_server_create(song_index *ix, int max_pq, int max_k, int nslots, int sl
     ++ix->servers;
     s->holds_entries = true;
   }
-  const song::WarpLayout L = song::warp_layout(dim, max_pq, s->S, 8 * max_pq, 32);
+  const song::WarpLayout L = song::warp_layout(dim, max_pq, s->S, 8 * max_pq, 32, false);
   p.off_mbar = L.off_mbar;
   p.off_cand = L.off_cand;
   p.off_q = L.off_q;
@@ -436,7 +436,8 @@ int song_server_create(song_index *ix, int max_pq, int max_k, int nslots, int sl
   p.warp_bytes = L.warp_bytes;
   p.width = dx.dpad;
   // the interface's limit: two staging chunks of the rows beside the query
-  // and the hash (the kernel needs less)
+  // and the hash.  Near a block's shared memory the staging (16 bytes a
+  // dimension) is far above the ring and the sort that the layout has instead
   const uint32_t limit = song::align_up(2u * (dx.row_bytes <= 1024 ? 4u : 2u) * dx.row_bytes, 16) + 16 + 32 * 4 +
                          song::align_up(static_cast<uint32_t>(dim) * 4u, 16) + 32u * static_cast<uint32_t>(max_pq);
   if (song::align_up(limit, 128) > 227u * 1024u) {
