@@ -511,11 +511,7 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
   const float d0 = __shfl_sync(FULL, cd, 0);
   uint32_t a_next;
   if (bulk) {
-    // One decision for the warp: a lane that gives up alone would leave the
-    // others shuffling with a lane that is gone, and lanes that see the copy at
-    // different polls would go through the whole query apart (in the server one
-    // query of 15k x 16 took 1363 us that way, 299 so).
-    if (!__all_sync(FULL, mbar_wait(w.mbar, w.ph, p.wait_limit))) return false;
+    if (!mbar_wait_warp(w.mbar, w.ph, p.wait_limit)) return false;
     w.ph ^= 1u;
     a_next = lane < nslots ? w.row[lane] : 0u;
   } else {
