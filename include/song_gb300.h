@@ -340,11 +340,13 @@ int song_debug_server_hold(song_server *server, int hold);
  * By default it scores queries against the coarse entries with a TF32
  * tensor-core product and re-scores, with the search's exact arithmetic, the
  * shortlist whose error intervals reach the probes-th best -- the same
- * clusters as an exact scan.  song_debug_head_path(index, 0) switches to the
- * exact CUDA-core scan of every coarse entry (1: back); *prepared (may be
- * NULL) tells whether the tensor path exists for the index (it needs
- * dim % 4 == 0).  song_debug_head_stats(index, enable, stats): with enable,
- * later searches count [0] queries, [1] coarse entries re-scored exactly,
+ * clusters as an exact scan; small batches take a scan of their own.
+ * song_debug_head_path(index, 1) has every batch, whatever its size, take the
+ * tensor cores' phase, 0 the exact CUDA-core scan of every coarse entry, -1
+ * (the default) chooses by the batch; *prepared (may be NULL) tells whether the
+ * tensor path exists for the index (it needs dim % 4 == 0; without it, 1 is the
+ * scan too).  song_debug_head_stats(index, enable, stats): with enable,
+ * later searches' tensor-core phases count [0] queries, [1] coarse entries re-scored exactly,
  * [2] queries whose shortlist overflowed into a full scan; stats (3 values,
  * may be NULL) receives the counts since the previous call, which restart at
  * zero.  song_debug_head_scores: the tensor-core scores alone, d_scores[q*ld

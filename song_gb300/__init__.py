@@ -289,11 +289,13 @@ class Index:
         _check(load_library().song_index_set_hop_limit(self._h, int(max_hops)))
 
     def debug_head_path(self, use_tensor_cores=True):
-        """Head phase of the two-level entry choice: tensor-core shortlist
-        (default) or the exact CUDA-core scan; returns whether the tensor
-        path is prepared for this index."""
+        """Head phase of the two-level entry choice of every later batch,
+        whatever its size: tensor-core shortlist or the exact CUDA-core scan
+        (None: the default, by batch size); returns whether the tensor path is
+        prepared for this index."""
         prepared = ctypes.c_int(0)
-        _check(load_library().song_debug_head_path(self._h, int(bool(use_tensor_cores)), ctypes.byref(prepared)))
+        path = -1 if use_tensor_cores is None else int(bool(use_tensor_cores))
+        _check(load_library().song_debug_head_path(self._h, path, ctypes.byref(prepared)))
         return bool(prepared.value)
 
     def debug_head_stats(self, enable=True):

@@ -486,7 +486,7 @@ int song_debug_set_wait(song_index *ix, uint32_t wait_limit, uint32_t extra_tx) 
 int song_debug_head_path(song_index *ix, int use_tensor_cores, int *prepared) {
   g_last_error.clear();
   if (!ix) return fail(SONG_ERR_ARG, "null index");
-  ix->heads_mma_enabled = use_tensor_cores != 0;
+  ix->head_path = use_tensor_cores < 0 ? -1 : (use_tensor_cores != 0 ? 1 : 0);
   if (prepared) *prepared = ix->heads_mma ? 1 : 0;
   return SONG_OK;
 }

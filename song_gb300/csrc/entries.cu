@@ -682,7 +682,7 @@ cudaError_t launch_small_by_probes(song_index *ix, const float *queries, int nq,
 // The two-level choice on stream s.  `out` holds nq * (ns + probes) words:
 // the starts, then the probed clusters.
 cudaError_t launch_2level(song_index *ix, const float *queries, int nq, uint32_t *out, cudaStream_t s) {
-  if (!ix->head_stats_on && small_batch(nq, ix->n_coarse, static_cast<int>(ix->dx.f32_row_bytes / 4))) {
+  if (ix->head_path < 0 && small_batch(nq, ix->n_coarse, static_cast<int>(ix->dx.f32_row_bytes / 4))) {
     switch (ix->dx.metric) {
       case SONG_METRIC_L2: return launch_small_by_probes<SONG_METRIC_L2>(ix, queries, nq, out, s);
       case SONG_METRIC_IP: return launch_small_by_probes<SONG_METRIC_IP>(ix, queries, nq, out, s);

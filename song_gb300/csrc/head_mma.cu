@@ -609,7 +609,7 @@ bool heads_mma_prepare(song_index *ix, int coarse) {
 }
 
 bool heads_mma_usable(const song_index *ix, const float *queries, int np) {
-  return ix->heads_mma && ix->heads_mma_enabled && np <= 8 && (reinterpret_cast<uintptr_t>(queries) & 15u) == 0;
+  return ix->heads_mma && ix->head_path != 0 && np <= 8 && (reinterpret_cast<uintptr_t>(queries) & 15u) == 0;
 }
 
 cudaError_t launch_heads_mma(song_index *ix, const float *queries, int nq, int np, uint32_t *probe_out,

@@ -167,7 +167,7 @@ struct song_index {
   // rows (a CUtensorMap), their squared norms, the per-chunk score buffer
   unsigned char head_map[128] = {};
   bool heads_mma = false;              // prepared for this index
-  bool heads_mma_enabled = true;       // song_debug_head_path
+  int head_path = -1;                  // song_debug_head_path: 1 tensor cores, 0 exact scan, -1 by batch size
   float *d_head_n2 = nullptr;
   float *d_head_scores = nullptr;
   size_t cap_head_scores = 0;

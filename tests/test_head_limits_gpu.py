@@ -1,7 +1,8 @@
 """The head phase's shortlist where its bounds are not finite: norms that
 overflow FP32 while the distances themselves do not (or overflow for a part of
 the heads), and NaN queries.  100 heads leave four unused places in a row of
-bounds; none of them may be taken.  Starts equal the oracle's."""
+bounds; none of them may be taken.  Starts equal the oracle's.  And the route
+that a batch takes: by its size, or the one it is told to take."""
 import numpy as np
 import pytest
 
@@ -62,3 +63,19 @@ def test_nan_queries(song, metric):
         plain = ix.search(q[bad], 20, 20)
     assert np.array_equal(ids[:60], few)
     assert np.array_equal(ids[bad], plain)  # they start at vertex 0
+
+
+def test_route_of_a_batch(song, oracle):
+    x, q, graph = _case(song, 0, (0.5, 2.0), (0.5, 2.0))
+    ox = oracle.OracleIndex(x, graph, 4, 0)
+    ent = np.random.default_rng(5).choice(len(x), 700, replace=False).astype(np.uint64)
+    o_ids = ox.kernel_search_from(q, ox.nearest_entry_2level(q, ent, 100, 3, 2), 20, oracle.MODE_LEX)[0]
+    with song.Index(graph, x, 4, 0) as ix:
+        ix.set_entries(ent, starts=2, coarse=100, probes=3)
+        ix.debug_head_stats(True)
+        for path, counted in ((None, 0), (True, 10), (False, 0), (None, 0)):
+            assert ix.debug_head_path(path)
+            assert np.array_equal(ix.search(q[:10], 20, 20), o_ids[:10])
+            assert ix.debug_head_stats(True)[0] == counted, path
+            assert np.array_equal(ix.search(q, 20, 20), o_ids)
+            assert ix.debug_head_stats(True)[0] == (0 if path is False else len(q)), path
