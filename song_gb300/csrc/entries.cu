@@ -543,12 +543,6 @@ __global__ void merge_starts_kernel(const float *part_d, const uint32_t *part_i,
   }
 }
 
-// Raises a kernel's dynamic shared-memory limit.
-template <class K>
-cudaError_t allow_smem(K kern, size_t bytes) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-}
-
 // Work area of the choice, grown to `words`.
 cudaError_t entry_work(song_index *ix, size_t words) {
   if (words <= ix->cap_entry_work) return cudaSuccess;
@@ -601,7 +595,7 @@ cudaError_t launch_nearest_rows(song_index *ix, const float *queries, int nq, in
   *part_i = ix->d_entry_work + lists;
   auto k = nqb == 1 ? nearest_rows_kernel<METRIC, NP, 1> : nearest_rows_kernel<METRIC, NP, 4>;
   const size_t smem = sizeof(float) * nqb * qs;
-  if ((e = allow_smem(k, smem)) != cudaSuccess) return e;
+  if ((e = allow_shared(k, smem)) != cudaSuccess) return e;
   // at most 65,535 block rows a launch
   for (int q0 = 0; q0 < nq; q0 += 65535 * nqb) {
     const int m = std::min(nq - q0, 65535 * nqb);
@@ -660,7 +654,7 @@ cudaError_t launch_small(song_index *ix, const float *queries, int nq, int ns, u
 #define SONG_STARTS(NS)                                                                                       \
   do {                                                                                                        \
     auto k = query_starts_kernel<METRIC, NP, NS>;                                                             \
-    if ((e = allow_smem(k, sizeof(float) * qs)) != cudaSuccess) return e;                                     \
+    if ((e = allow_shared(k, sizeof(float) * qs)) != cudaSuccess) return e;                                     \
     k<<<nq, 512, sizeof(float) * qs, s>>>(queries, dim, dpad, qs, part_d, part_i, chunks, n, ix->n_probes,    \
                                           ix->d_entry_rows, ix->d_entry_ids, ix->d_offsets, ns, out);         \
   } while (0)
@@ -721,7 +715,7 @@ cudaError_t launch_2level(song_index *ix, const float *queries, int nq, uint32_t
 #define SONG_HEADS(M, NP)                                                                                \
   do {                                                                                                   \
     auto k_ = heads_tiled_kernel<M, NP>;                                                                 \
-    if ((e = allow_smem(k_, smem)) != cudaSuccess) return e;                                             \
+    if ((e = allow_shared(k_, smem)) != cudaSuccess) return e;                                             \
     k_<<<grid_q, ts.warps * 32, smem, s>>>(queries, nq, dim, dpad, ix->d_coarse_rows, coarse, np, ts.rows, \
                                            ts.nbuf, probes, ix->d_cl_count);                             \
   } while (0)
@@ -729,7 +723,7 @@ cudaError_t launch_2level(song_index *ix, const float *queries, int nq, uint32_t
   do {                                                                                                   \
     auto k_ = clusters_rows_kernel<M, NS>;                                                               \
     const size_t qsm = sizeof(float) * 4 * qs;                                                           \
-    if ((e = allow_smem(k_, qsm)) != cudaSuccess) return e;                                              \
+    if ((e = allow_shared(k_, qsm)) != cudaSuccess) return e;                                              \
     int per_sm = 0, sms = 0, dev = 0;                                                                    \
     cudaGetDevice(&dev);                                                                                 \
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);                                   \

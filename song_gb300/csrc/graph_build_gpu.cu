@@ -657,7 +657,7 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
   int optin = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
   if (smem > static_cast<size_t>(optin)) return fail(SONG_ERR_ARG, "graph build: dim/budget need too much shared memory");
-  e = cudaFuncSetAttribute(build_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  e = allow_shared(build_search_kernel, smem);
   if (e != cudaSuccess) return fail(SONG_ERR_CUDA, "graph build: %s", cudaGetErrorString(e));
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, build_search_kernel, BUILD_WARPS * 32, smem);
@@ -677,11 +677,8 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
   const bool beam = budget <= BEAM_BUDGET && shift <= 5 && n < (1ull << 31) && beam_smem1 <= static_cast<size_t>(optin) &&
                     beam_smem4 <= static_cast<size_t>(optin) && beam_k > 0;
   if (beam) {
-    e = cudaFuncSetAttribute(beam_search_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(beam_smem1));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(beam_search_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(beam_smem4));
+    e = allow_shared(beam_search_kernel<1>, beam_smem1);
+    if (e == cudaSuccess) e = allow_shared(beam_search_kernel<4>, beam_smem4);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&beam1, beam_search_kernel<1>, BUILD_WARPS * 32, beam_smem1);
     if (e == cudaSuccess)

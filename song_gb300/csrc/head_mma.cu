@@ -570,7 +570,7 @@ template <int METRIC, int NP>
 cudaError_t launch_chunk(const CUtensorMap &tq, const CUtensorMap &th, HeadScoreArgs a, const float *queries,
                          song_index *ix, int np, uint32_t *probe_out, cudaStream_t s) {
   auto kern = head_scores_kernel<METRIC, NP, OUT_BOUNDS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(HM_SMEM));
+  cudaError_t e = allow_shared(kern, HM_SMEM);
   if (e != cudaSuccess) return e;
   const int tiles = (a.n_heads + HM_B - 1) / HM_B;
   kern<<<dim3((a.rows + HM_B - 1) / HM_B, tiles), 128, HM_SMEM, s>>>(tq, th, a);
@@ -579,8 +579,7 @@ cudaError_t launch_chunk(const CUtensorMap &tq, const CUtensorMap &th, HeadScore
   const int qbytes = 4 * ((dpad + 31) & ~31);
   const int sw = std::max(1, std::min(HM_SEL_WARPS, 32 * 1024 / qbytes));
   auto select = head_select_kernel<METRIC, NP>;
-  e = cudaFuncSetAttribute(select, cudaFuncAttributeMaxDynamicSharedMemorySize, sw * qbytes);
-  if (e != cudaSuccess) return e;
+  if ((e = allow_shared(select, static_cast<size_t>(sw) * qbytes)) != cudaSuccess) return e;
   select<<<(a.rows + sw - 1) / sw, sw * 32, static_cast<size_t>(sw) * qbytes, s>>>(
       queries, ix->dx.dim, a.q_row0, a.rows, a.lo16, a.ld, a.tile_hi, tiles, ix->d_coarse_rows, dpad, ix->n_coarse,
       np, probe_out, ix->d_cl_count, ix->head_stats_on ? ix->d_head_stats : nullptr);
@@ -688,7 +687,7 @@ cudaError_t launch_head_scores_only(song_index *ix, const float *queries, int nq
     return cudaErrorInvalidValue;
   std::memcpy(&th, ix->head_map, sizeof th);
   auto kern = head_scores_kernel<SONG_METRIC_L2, 1, OUT_RAW>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(HM_SMEM));
+  cudaError_t e = allow_shared(kern, HM_SMEM);
   if (e != cudaSuccess) return e;
   HeadScoreArgs a;
   std::memset(&a, 0, sizeof a);

@@ -112,6 +112,28 @@ cudaError_t dev_malloc(T **p, size_t bytes) {
   return dev_malloc(reinterpret_cast<void **>(p), bytes);
 }
 
+// Lets kernel fn be launched with `bytes` of dynamic shared memory.  The limit
+// belongs to the process, not to the launch: it is only ever raised, and to the
+// device's maximum, so that no thread takes away what another is about to
+// launch with.  Up to 32 KB every kernel here may have without asking (16 KB of
+// static shared memory at most).
+inline cudaError_t allow_shared(const void *fn, size_t bytes) {
+  if (bytes <= 32u * 1024u) return cudaSuccess;
+  int dev = 0, optin = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, fn);
+  if (e != cudaSuccess) return e;
+  if (bytes <= static_cast<size_t>(a.maxDynamicSharedSizeBytes)) return cudaSuccess;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              optin - static_cast<int>(a.sharedSizeBytes));
+}
+template <class K>
+cudaError_t allow_shared(K kernel, size_t bytes) {
+  return allow_shared(reinterpret_cast<const void *>(kernel), bytes);
+}
+
 // Error reporting of the C ABI (capi.cu): records the message for
 // song_last_error() on the calling thread and returns `code`.
 int fail(int code, const char *fmt, ...);
