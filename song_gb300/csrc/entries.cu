@@ -819,7 +819,9 @@ int prepare_starts(song_index *ix, SearchCall &c, cudaStream_t s) {
       ix->n_coarse > 0 ? launch_2level(ix, c.queries, c.nq, ix->d_starts, s)
                        : launch_nearest(ix, c.queries, c.nq, ix->dx.dim, ix->d_entry_rows, ix->d_entry_ids,
                                         ix->n_entries, ix->n_starts, ix->d_starts, s);
-  if (le != cudaSuccess) return fail(SONG_ERR_CUDA, "entry launch: %s", cudaGetErrorString(le));
+  if (le != cudaSuccess)
+    return fail(le == cudaErrorMemoryAllocation ? SONG_ERR_OOM : SONG_ERR_CUDA, "entry choice: %s",
+                cudaGetErrorString(le));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(SONG_ERR_CUDA, "entry launch: %s", cudaGetErrorString(e));
   c.starts = ix->d_starts;
