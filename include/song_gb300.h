@@ -327,6 +327,11 @@ int song_search_noalloc(song_index *index, const float *queries, int nq, int pq,
  * SONG_ERR_TIMEOUT and the index stays usable.  song_debug_server_hold(1):
  * admitted requests are kept from the kernel until song_debug_server_hold(0). */
 int song_debug_fail_alloc(int n);
+/* song_graph_build_gpu on the calling thread: later builds start with visited
+ * sets of 2^visited_log2 slots (6..13; 0: the default, 13), searches (3 values,
+ * may be NULL) receives how many searches the builds since the previous call ran
+ * with a block per vertex, with a warp per vertex and step by step. */
+int song_debug_build(int visited_log2, uint64_t *searches);
 /* Shared memory of a search, on the host alone: *accepted_by, the bytes a warp
  * by which song_search accepts the size (at most 227 KB), and *used, those of
  * the kernel's smallest block (learned: the kernel of the early exit and of

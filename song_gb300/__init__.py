@@ -49,7 +49,7 @@ EXPORTED = [
     "song_index_set_hash_planes",
     "song_server_set_idle_polls", "song_server_running", "song_server_wait", "song_debug_fail_alloc",
     "song_debug_set_wait", "song_debug_server_hold", "song_debug_head_path", "song_debug_head_stats",
-    "song_debug_head_scores", "song_debug_shared_bytes",
+    "song_debug_head_scores", "song_debug_shared_bytes", "song_debug_build",
 ]
 MLP_PARAMS = 1281
 TRACE_FIELDS = 6
@@ -152,6 +152,8 @@ def load_library():
     L.song_server_running.argtypes = [P, ctypes.POINTER(i32)]
     L.song_server_wait.restype = i32
     L.song_server_wait.argtypes = [P, ctypes.c_uint64, i32]
+    L.song_debug_build.restype = i32
+    L.song_debug_build.argtypes = [i32, P]
     L.song_debug_shared_bytes.restype = i32
     L.song_debug_shared_bytes.argtypes = [i32, i32, i32, i32, i32, P, P]
     L.song_debug_fail_alloc.restype = i32
@@ -434,6 +436,15 @@ def hash_planes(dim, seed=123):
 def debug_fail_alloc(n):
     """Test hook: the n-th next device allocation of the library fails (0: none)."""
     _check(load_library().song_debug_fail_alloc(int(n)))
+
+
+def debug_build(visited_log2=0):
+    """Searches of this thread's graph_build_gpu calls since the last
+    debug_build: (a block per vertex, a warp per vertex, step by step); later
+    builds start with visited sets of 2^visited_log2 slots (0: the default)."""
+    st = np.zeros(3, dtype=np.uint64)
+    _check(load_library().song_debug_build(int(visited_log2), st.ctypes.data_as(ctypes.c_void_p)))
+    return tuple(int(x) for x in st)
 
 
 def debug_shared_bytes(storage, dim, pq, learned=False, multi=False):

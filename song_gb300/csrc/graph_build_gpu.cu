@@ -24,13 +24,13 @@
 //
 // Two kernels do it.  beam_search_kernel (budgets up to BEAM_BUDGET) keeps
 // queue and result list as one sorted list and sums the distances of a row
-// over the whole warp, in integers where that is exact (below).  A batch it
-// cannot finish (more equal distances at the list's end than its list holds)
-// and larger budgets take build_search_kernel, which follows the CPU search
-// step by step: one lane per candidate, lane 0 keeping the two heaps, the
+// over the whole warp, in integers where that is exact (below).  What it cannot
+// finish (more equal distances at the list's end than its list holds, NaN
+// distances) and larger budgets take build_search_kernel, which follows the CPU
+// search step by step: one lane per candidate, lane 0 keeping the two heaps, the
 // visited set and the queue heap in a device scratch region whose size is
-// checked; a search that would overflow it flags the batch, which the host
-// repeats with larger regions.
+// checked.  A search that must be repeated, or would overflow its region, says
+// so in place of its result, and the host repeats these searches alone.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -64,21 +64,26 @@ struct BuildArgs {
   const float *norms;    // cos: per-row squared norm (float, dimension order); else null
   const uint32_t *adj;   // n << shift
   int dim, metric, shift;
-  uint64_t first;        // new vertices first .. first + count - 1
+  uint64_t first;        // new vertices first + t: t = todo[0 .. count - 1], or 0 .. count - 1 (todo null)
   uint32_t count;
+  const uint32_t *todo;
   uint64_t limit;        // vertices inserted before the batch
   int budget;            // result size k of the search
   int out_k;             // ids written per vertex (search_degree)
-  uint32_t *out;         // count x out_k
-  int32_t *out_cnt;      // count
+  uint32_t *out;         // row t: vertex first + t's, out_k places
+  int32_t *out_cnt;      // their number, or why the search must be repeated (NEED_*)
   uint32_t *vis;         // per warp: vis_cap slots
   uint32_t vis_cap;      // power of two
   int vis_log2;
+  uint32_t vis_limit;    // a search that has visited more is repeated: at most 3/4 of the slots
   QE *q;                 // per warp: q_cap entries
   uint32_t q_cap;
   uint32_t *counter;
-  int32_t *error;        // 1: visited set full, 2: queue full
 };
+
+// Searches to be repeated, alone: with a larger visited set, with a larger
+// queue, or by the step-by-step search.
+constexpr int32_t NEED_VISITED = -1, NEED_QUEUE = -2, NEED_STEPS = -3;
 
 // data.h:28-62 with a = base row, v = the query (in shared memory).
 __device__ __forceinline__ double cpu_distance(const BuildArgs &p, const float *a, const float *v, float lena,
@@ -177,7 +182,6 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) build_search_kernel(const Bu
   const uint64_t gw = static_cast<uint64_t>(blockIdx.x) * BUILD_WARPS + wib;
   uint32_t *vis = p.vis + gw * p.vis_cap;
   QE *Q = p.q + gw * p.q_cap;
-  const uint32_t vis_limit = p.vis_cap - (p.vis_cap >> 2);  // fill at most 3/4
   const uint32_t nslots = 1u << p.shift;
 
   for (;;) {
@@ -185,6 +189,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) build_search_kernel(const Bu
     if (lane == 0) t = atomicAdd(p.counter, 1u);
     t = __shfl_sync(FULLM, t, 0);
     if (t >= p.count) break;
+    if (p.todo) t = p.todo[t];
     const uint64_t v = p.first + t;
     if (p.limit == 0) {  // the first vertex: nothing to search
       if (lane == 0) p.out_cnt[t] = 0;
@@ -245,7 +250,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) build_search_kernel(const Bu
         }
         const unsigned fm = __ballot_sync(FULLM, fresh);
         vis_n += __popc(fm);
-        if (vis_n > vis_limit) overflow = true;
+        if (vis_n > p.vis_limit) overflow = true;
         double d = 0.0;
         if (fresh) d = cpu_distance(p, p.data + static_cast<uint64_t>(s) * p.dim, qv, p.norms ? p.norms[s] : 0.0f, lenv);
         // Queue the fresh candidates (lane order; the heap order does not
@@ -275,7 +280,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) build_search_kernel(const Bu
       if (overflow) break;
     }
     if (overflow) {
-      if (lane == 0) atomicOr(p.error, vis_n > vis_limit ? 1 : 2);
+      if (lane == 0) p.out_cnt[t] = vis_n > p.vis_limit ? NEED_VISITED : NEED_QUEUE;
       continue;
     }
     // graph.h:207-215: the list in ascending order (in-place heap sort).
@@ -370,7 +375,8 @@ __device__ __forceinline__ bool exact_sum(const float *row, const float *qv, int
   for (int r = 0; r < R; ++r) take(b[r]);
   for (int j = lane + 32 * R; j < dim; j += 32) take(product(j));
   if (__any_sync(FULLM, !ok)) return false;
-  // |s| <= 2^48: two 24-bit parts, each part's warp sum within 32 bits
+  // the warp's magnitudes sum to dim * 2^(24 + K) <= 2^53 at most: the sum of
+  // the parts s >> 24 stays within 2^29 + 32, that of the low 24 bits below 2^29
   const int hi = __reduce_add_sync(FULLM, static_cast<int>(s >> 24));
   const int lo = __reduce_add_sync(FULLM, static_cast<int>(s & 0xffffff));
   sum = (static_cast<int64_t>(hi) << 24) + lo;
@@ -379,7 +385,8 @@ __device__ __forceinline__ bool exact_sum(const float *row, const float *qv, int
 
 // W warps a vertex: 4, with the visited set in the block's shared memory, for
 // batches that fill the GPU that way at most once (what counts there is the
-// latency of one search); 1, with it in the scratch region, beyond.
+// latency of one search); 1, with it in the scratch region, beyond, and for a
+// search that fills a block's set.
 template <int W>
 __global__ void __launch_bounds__(BUILD_WARPS * 32) beam_search_kernel(const BuildArgs p, const int K) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -397,7 +404,6 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) beam_search_kernel(const Bui
   uint32_t *vis = W == 1 ? p.vis + gw * p.vis_cap : reinterpret_cast<uint32_t *>(smem + slice);
   const uint32_t vis_cap = W == 1 ? p.vis_cap : 1u << BEAM_VIS_LOG2;
   const int vis_log2 = W == 1 ? p.vis_log2 : BEAM_VIS_LOG2;
-  const uint32_t vis_limit = vis_cap - (vis_cap >> 2);  // fill at most 3/4
   const uint32_t nslots = 1u << p.shift;
   auto sync = [&] {
     if (W == 1) __syncwarp();
@@ -415,6 +421,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) beam_search_kernel(const Bui
       t = static_cast<uint32_t>(ctl[1]);
     }
     if (t >= p.count) break;
+    if (p.todo) t = p.todo[t];
     const uint64_t v = p.first + t;
     if (p.limit == 0) {  // the first vertex: nothing to search
       if (rank == 0 && lane == 0) p.out_cnt[t] = 0;
@@ -434,7 +441,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) beam_search_kernel(const Bui
     sync();
     int n = 0;             // listed vertices (rank 0)
     uint32_t vis_n = 1;    // visited ones (rank 0)
-    bool overflow = false; // (rank 0)
+    bool overflow = false; // the search must be repeated (rank 0)
     for (;;) {
       // distances of this hop's candidates, the warps taking them in turn
       const int m = ctl[0];
@@ -562,7 +569,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) beam_search_kernel(const Bui
           const unsigned fm = __ballot_sync(FULLM, fresh);
           next = __popc(fm);
           vis_n += next;
-          if (vis_n > vis_limit) overflow = true;
+          if (vis_n > p.vis_limit) overflow = true;
           if (fresh) cid[__popc(fm & ((1u << lane) - 1u))] = a;
         }
         if (lane == 0) ctl[0] = overflow ? -1 : next;
@@ -571,7 +578,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) beam_search_kernel(const Bui
     }
     if (rank == 0) {
       if (overflow) {
-        if (lane == 0) atomicOr(p.error, vis_n > vis_limit ? (W == 1 ? 1 : 4) : 4);
+        if (lane == 0) p.out_cnt[t] = vis_n > p.vis_limit ? NEED_VISITED : NEED_STEPS;
       } else {
         // graph.h:207-215: the list in ascending order
         const int num = min(min(n, p.budget), p.out_k);
@@ -613,6 +620,13 @@ struct DevBuf {
   }
 };
 
+// song_debug_build: of the calling thread.
+struct BuildDebug {
+  int visited_log2 = 0;
+  uint64_t searches[3] = {0, 0, 0};
+};
+thread_local BuildDebug g_build_debug;
+
 struct HostPinned {
   void *p = nullptr;
   ~HostPinned() {
@@ -622,6 +636,18 @@ struct HostPinned {
 
 }  // namespace
 }  // namespace song
+
+extern "C" int song_debug_build(int visited_log2, uint64_t *searches) {
+  using namespace song;
+  clear_error();
+  if (visited_log2 != 0 && (visited_log2 < 6 || visited_log2 > BEAM_VIS_LOG2))
+    return fail(SONG_ERR_ARG, "visited_log2 must be 0 or in [6, %d]", BEAM_VIS_LOG2);
+  if (searches)
+    for (int i = 0; i < 3; ++i) searches[i] = g_build_debug.searches[i];
+  g_build_debug = BuildDebug{};
+  g_build_debug.visited_log2 = visited_log2;
+  return SONG_OK;
+}
 
 extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int metric, int shift,
                                     int search_degree, int fixed_degree, int budget, int batch_div,
@@ -698,8 +724,8 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
 
   const uint64_t max_batch = batch_div == 0 ? 1 : std::max<uint64_t>(1, n / batch_div) + 1;
   const uint32_t w = 1u << shift;
-  DevBuf d_data, d_norms, d_adj, d_out, d_cnt, d_ctl, d_vis, d_q, d_rows, d_ids;
-  HostPinned h_out, h_cnt, h_err, h_rows, h_ids;
+  DevBuf d_data, d_norms, d_adj, d_out, d_cnt, d_ctl, d_vis, d_q, d_rows, d_ids, d_todo;
+  HostPinned h_out, h_cnt, h_rows, h_ids;
   const size_t rows_cap = static_cast<size_t>(max_batch) * (search_degree + 1);
 #define SONG_GB_CK(call)                                                          \
   do {                                                                            \
@@ -717,7 +743,6 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
   SONG_GB_CK(song::dev_malloc(&d_ids.p, sizeof(uint64_t) * rows_cap));
   SONG_GB_CK(cudaMallocHost(&h_out.p, sizeof(uint32_t) * max_batch * search_degree));
   SONG_GB_CK(cudaMallocHost(&h_cnt.p, sizeof(int32_t) * max_batch));
-  SONG_GB_CK(cudaMallocHost(&h_err.p, 256));
   SONG_GB_CK(cudaMallocHost(&h_rows.p, sizeof(uint32_t) * rows_cap * w));
   SONG_GB_CK(cudaMallocHost(&h_ids.p, sizeof(uint64_t) * rows_cap));
   SONG_GB_CK(cudaMemcpyAsync(d_data.p, data, sizeof(float) * n * dim, cudaMemcpyHostToDevice, st));
@@ -729,8 +754,9 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
     SONG_GB_CK(cudaGetLastError());
   }
   // scratch of the searches that keep their sets in device memory, allocated
-  // when the first such batch comes; grown when a batch overflows
-  int vis_log2 = 13, q_log2 = 12;
+  // when the first of them comes; grown when one overflows
+  const int set_log2 = g_build_debug.visited_log2 > 0 ? g_build_debug.visited_log2 : BEAM_VIS_LOG2;
+  int vis_log2 = set_log2, q_log2 = 12;
   auto alloc_scratch = [&](bool queue) -> int {
     if (d_vis.p) cudaFree(d_vis.p);
     if (d_q.p) cudaFree(d_q.p);
@@ -746,19 +772,27 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
 
   uint32_t *h_out32 = static_cast<uint32_t *>(h_out.p);
   int32_t *h_cnt32 = static_cast<int32_t *>(h_cnt.p);
-  int32_t *h_err32 = static_cast<int32_t *>(h_err.p);
   const uint64_t *edges = graph_builder_edges(gb);
   uint64_t a = 0;
+  // Where most searches end up step by step (many equal distances, NaNs) they
+  // go there at once: for the next 15 batches, when of the last 32 vertices or
+  // more that tried the one list most did (20,000 corners of a 32-d cube: 778 ms
+  // with both searches for every batch, 671 so).
+  uint64_t tried = 0, repeated = 0;
+  int steps_first = 0;
+  std::vector<uint32_t> todo[2];  // searches to be repeated: by a warp with one list, step by step
   while (a < n) {
     const uint64_t bs = batch_div == 0 ? 1 : std::max<uint64_t>(1, a / static_cast<uint64_t>(batch_div));
     const uint64_t end = std::min<uint64_t>(n, a + bs);
-    bool one_list = beam;
-    for (int attempt = 0;; ++attempt) {
-      const uint64_t count = end - a, grid = std::min<uint64_t>(blocks, (count + BUILD_WARPS - 1) / BUILD_WARPS);
-      const uint64_t fit4 = static_cast<uint64_t>(sms) * beam4, fit1 = static_cast<uint64_t>(sms) * beam1;
-      const bool block_each = one_list && count <= fit4;
-      if ((!block_each && !d_vis.p) || (!one_list && !d_q.p))
-        if ((rc = alloc_scratch(!one_list)) != SONG_OK) return rc;
+    const uint64_t fit4 = static_cast<uint64_t>(sms) * beam4, fit1 = static_cast<uint64_t>(sms) * beam1;
+    enum { BLOCK, WARP, STEPS } how = !beam || steps_first > 0 ? STEPS : (end - a <= fit4 ? BLOCK : WARP);
+    if (steps_first > 0) --steps_first;
+    const uint32_t *list = nullptr;  // of the vertices searched, on the device (null: all)
+    uint64_t count = end - a;
+    for (int grown = 0;;) {
+      const uint64_t grid = std::min<uint64_t>(blocks, (count + BUILD_WARPS - 1) / BUILD_WARPS);
+      if ((how != BLOCK && !d_vis.p) || (how == STEPS && !d_q.p))
+        if ((rc = alloc_scratch(how == STEPS)) != SONG_OK) return rc;
       BuildArgs p;
       p.data = static_cast<const float *>(d_data.p);
       p.norms = static_cast<const float *>(d_norms.p);
@@ -767,43 +801,66 @@ extern "C" int song_graph_build_gpu(const float *data, uint64_t n, int dim, int 
       p.metric = metric;
       p.shift = shift;
       p.first = a;
-      p.count = static_cast<uint32_t>(end - a);
+      p.count = static_cast<uint32_t>(count);
+      p.todo = list;
       p.limit = a;
       p.budget = budget;
       p.out_k = search_degree;
       p.out = static_cast<uint32_t *>(d_out.p);
       p.out_cnt = static_cast<int32_t *>(d_cnt.p);
       p.vis = static_cast<uint32_t *>(d_vis.p);
-      p.vis_cap = 1u << vis_log2;
       p.vis_log2 = vis_log2;
+      p.vis_cap = 1u << vis_log2;
+      p.vis_limit = 3u << ((how == BLOCK ? set_log2 : vis_log2) - 2);
       p.q = static_cast<QE *>(d_q.p);
       p.q_cap = 1u << q_log2;
       p.counter = static_cast<uint32_t *>(d_ctl.p);
-      p.error = static_cast<int32_t *>(d_ctl.p) + 1;
       SONG_GB_CK(cudaMemsetAsync(d_ctl.p, 0, 8, st));
-      if (block_each)
+      if (how == BLOCK)
         beam_search_kernel<4><<<static_cast<unsigned>(count), BUILD_WARPS * 32, beam_smem4, st>>>(p, beam_k);
-      else if (one_list)
+      else if (how == WARP)
         beam_search_kernel<1><<<static_cast<unsigned>(std::min<uint64_t>(fit1, grid)), BUILD_WARPS * 32, beam_smem1, st>>>(
             p, beam_k);
       else
         build_search_kernel<<<static_cast<unsigned>(grid), BUILD_WARPS * 32, smem, st>>>(p);
       SONG_GB_CK(cudaGetLastError());
-      SONG_GB_CK(cudaMemcpyAsync(h_err32, p.error, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
       SONG_GB_CK(cudaMemcpyAsync(h_cnt32, d_cnt.p, sizeof(int32_t) * (end - a), cudaMemcpyDeviceToHost, st));
       SONG_GB_CK(cudaMemcpyAsync(h_out32, d_out.p, sizeof(uint32_t) * (end - a) * search_degree,
                                  cudaMemcpyDeviceToHost, st));
       SONG_GB_CK(cudaStreamSynchronize(st));
-      if (*h_err32 == 0) break;
-      if (*h_err32 & 4) {  // for the step-by-step search
-        one_list = false;
-        continue;
+      g_build_debug.searches[how] += count;
+      // (those not yet repeated still hold their mark)
+      bool more_visited = false, more_queue = false;
+      todo[0].clear();
+      todo[1].clear();
+      for (uint32_t t = 0; t < end - a; ++t) {
+        const int32_t c = h_cnt32[t];
+        if (c >= 0) continue;
+        more_visited = more_visited || (c == NEED_VISITED && how != BLOCK);
+        more_queue = more_queue || c == NEED_QUEUE;
+        todo[c == NEED_VISITED && how != STEPS ? 0 : 1].push_back(t);
       }
-      if (attempt >= 7) return fail(SONG_ERR_OOM, "graph build: search scratch still too small after growing");
-      if (*h_err32 & 1) ++vis_log2;
-      if (*h_err32 & 2) ++q_log2;
-      rc = alloc_scratch(d_q.p != nullptr);
-      if (rc != SONG_OK) return rc;
+      if (!list && how != STEPS) {
+        tried += count;
+        repeated += todo[1].size();
+        if (tried >= 32) {
+          if (2 * repeated > tried) steps_first = 15;
+          tried = repeated = 0;
+        }
+      }
+      if (todo[0].empty() && todo[1].empty()) break;
+      if (more_visited || more_queue) {
+        if (++grown > 7) return fail(SONG_ERR_OOM, "graph build: search scratch still too small after growing");
+        if (more_visited) ++vis_log2;
+        if (more_queue) ++q_log2;
+        if ((rc = alloc_scratch(d_q.p != nullptr)) != SONG_OK) return rc;
+      }
+      how = todo[0].empty() ? STEPS : WARP;
+      const std::vector<uint32_t> &next = todo[todo[0].empty() ? 1 : 0];
+      if (!d_todo.p) SONG_GB_CK(song::dev_malloc(&d_todo.p, sizeof(uint32_t) * max_batch));
+      count = next.size();
+      list = static_cast<const uint32_t *>(d_todo.p);
+      SONG_GB_CK(cudaMemcpyAsync(d_todo.p, next.data(), sizeof(uint32_t) * count, cudaMemcpyHostToDevice, st));
     }
     // the edges, and the changed rows straight into the upload buffer: <= (end - a) * (search_degree + 1) <= rows_cap
     uint32_t *hr = static_cast<uint32_t *>(h_rows.p);
