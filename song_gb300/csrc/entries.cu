@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <vector>
 
@@ -446,6 +447,118 @@ __global__ void __launch_bounds__(256) merge_lists_kernel(const float *part_d, c
   }
 }
 
+// The flat choice of short rows or few entries: a warp takes QB queries and a
+// lane a whole distance.  The block stages 32 entry rows at a time (coalesced
+// 16-byte loads, rows padded to an odd number of 16-byte units, so that the
+// lanes' reads of 32 different rows hit distinct banks), and lane e scores row e
+// against the warp's queries: it keeps the 32 partial sums and adds them in the
+// butterfly's pairs.  Padded elements add fma(0, 0, t).  No lane is idle however
+// few dimensions there are, and no lists go through memory (nearest_rows_kernel
+// spreads a row over 32 lanes and needs a second launch).
+template <int METRIC, int QB, int NS>
+__global__ void __launch_bounds__(256) flat_tiled_kernel(const float *queries, int nq, int qstride, int dim, int dpad,
+                                                         const float *entry_rows, const uint32_t *entry_ids,
+                                                         int n_entries, int ns, uint32_t *starts) {
+  extern __shared__ float4 sm4[];
+  constexpr int TILE = 32;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int q0 = (blockIdx.x * nwarps + wib) * QB;
+  const bool active = q0 < nq;  // warp-uniform; idle warps still help load tiles
+  const int d4 = dpad >> 2, rs4 = d4 + 1;
+  float4 *tile = sm4;
+  float *qw = reinterpret_cast<float *>(sm4 + TILE * rs4) + static_cast<size_t>(wib) * QB * dpad;
+  for (int b = 0; b < QB; ++b)
+    for (int j = lane; j < dpad; j += 32)
+      qw[b * dpad + j] = (q0 + b < nq && j < dim) ? queries[static_cast<size_t>(q0 + b) * qstride + j] : 0.0f;
+  const float4 *q4 = reinterpret_cast<const float4 *>(qw);
+  float bd[QB][NS];
+  uint32_t bi[QB][NS];
+#pragma unroll
+  for (int b = 0; b < QB; ++b) clear_list<NS>(bd[b], bi[b]);
+  for (int t0 = 0; t0 < n_entries; t0 += TILE) {
+    const int rows = min(TILE, n_entries - t0);
+    __syncthreads();  // the previous tile is consumed (and, first time, the queries are staged)
+    for (int i = threadIdx.x; i < rows * d4; i += blockDim.x) {
+      const int r = i / d4, c = i - r * d4;
+      tile[r * rs4 + c] = __ldg(reinterpret_cast<const float4 *>(entry_rows + static_cast<size_t>(t0 + r) * dpad) + c);
+    }
+    __syncthreads();
+    if (!active || lane >= rows) continue;
+    const float4 *x4 = tile + lane * rs4;
+    float t[QB][32], l[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      l[i] = 0.0f;
+#pragma unroll
+      for (int b = 0; b < QB; ++b) t[b][i] = 0.0f;
+    }
+    for (int c0 = 0; c0 < d4; c0 += 8) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (c0 + i < d4) {
+          const float4 xv = x4[c0 + i];
+          const float xs[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+          for (int b = 0; b < QB; ++b) {
+            const float4 qv = q4[b * d4 + c0 + i];
+            const float qq[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              if (METRIC == SONG_METRIC_L2) {
+                const float d = __fsub_rn(qq[c], xs[c]);
+                t[b][4 * i + c] = __fmaf_rn(d, d, t[b][4 * i + c]);
+              } else {
+                t[b][4 * i + c] = __fmaf_rn(qq[c], xs[c], t[b][4 * i + c]);
+              }
+            }
+          }
+          if (METRIC == SONG_METRIC_COS) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) l[4 * i + c] = __fmaf_rn(xs[c], xs[c], l[4 * i + c]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+      for (int i = 0; i < off; ++i) {
+#pragma unroll
+        for (int b = 0; b < QB; ++b) t[b][i] = __fadd_rn(t[b][i], t[b][i + off]);
+        if (METRIC == SONG_METRIC_COS) l[i] = __fadd_rn(l[i], l[i + off]);
+      }
+    }
+    const uint32_t id = entry_ids[t0 + lane];
+#pragma unroll
+    for (int b = 0; b < QB; ++b) {
+      float d;
+      if (METRIC == SONG_METRIC_L2) {
+        d = t[b][0];
+      } else if (METRIC == SONG_METRIC_IP) {
+        d = -t[b][0];
+      } else if (l[0] != 0.0f) {
+        const float sign = t[b][0] < 0.0f ? 1.0f : -1.0f;
+        d = __fdiv_rn(__fmul_rn(__fmul_rn(sign, t[b][0]), t[b][0]), l[0]);
+      } else {
+        d = 0.0f;
+      }
+      list_insert<NS>(bd[b], bi[b], d, id);
+    }
+  }
+  if (!active) return;
+#pragma unroll
+  for (int b = 0; b < QB; ++b) {
+    int h = 0;
+    for (int r = 0; r < ns; ++r) {
+      float wd;
+      uint32_t wid;
+      warp_list_take<NS>(bd[b], bi[b], h, wd, wid);
+      // no finite distance (a query that is not finite): vertex 0
+      if (lane == 0 && q0 + b < nq) starts[static_cast<size_t>(q0 + b) * ns + r] = wid == 0xffffffffu ? 0u : wid;
+    }
+  }
+}
+
 // The N smallest of the block's lists (16 warps), ascending, to out(r, d, id)
 // on one lane of warp 0; ends with the lists no longer read.
 template <int N, class Out>
@@ -574,6 +687,41 @@ bool small_batch(int nq, int coarse, int dpad) {
   return (nq <= 512 && work <= 536870912.0) || work <= 4194304.0;
 }
 
+// nearest_rows_kernel's split: one query a block row while there are few, four
+// afterwards; chunks of 64 rows (one pass a warp) until the grid fills the GPU
+// some times over.
+struct RowsSplit {
+  int nqb, chunk;
+};
+RowsSplit rows_split(int nq, int n) {
+  RowsSplit r{nq <= 4 ? 1 : 4, 64};
+  const long long groups = (nq + r.nqb - 1) / r.nqb;
+  while (r.chunk < n && groups * (n / r.chunk) > 2048) r.chunk *= 2;
+  return r;
+}
+
+// Whether the flat choice takes flat_tiled_kernel (rows of up to 1 KB).  Both
+// kernels' times in us, estimated: one warp's chain over the tiles of 32 rows,
+// once or as often as the warps exceed the resident ones; one block's over the
+// passes of 64 rows, and as often again as 200 blocks go into the grid.  The
+// constants are fitted to 1,944 shapes (4 to 256 dimensions, 8 to 16,384
+// entries, 1 to 50,000 queries, 1 to 8 starts, L2 and cosine): the kernel taken
+// is the faster one or within 5 % of it in 96 of 100, at worst 1.4 times as long.
+// 10,000 queries of 16-d L2 rows: 64 entries 15 us with the tiled kernel and 31
+// with the other, 4096 entries 394 and 454; one query of 4096 entries 109 and 11.
+bool flat_tiled(int metric, int nq, int n, int dpad, int len) {
+  if (dpad > 256) return false;
+  const bool cos = metric == SONG_METRIC_COS;
+  const double lists = len <= 1 ? 0.0 : (len <= 4 ? 1.0 : 2.0), tiles = (n + 31) / 32;
+  const double tile = cos ? 0.51 + 0.0145 * dpad + 0.23 * lists : 0.55 + 0.018 * dpad + 0.37 * lists;
+  const double tiled = 6.8 + 0.9 * lists + tiles * tile * std::max(1.0, cos ? nq / 1840.0 : nq / (2.0 * 1640.0));
+  const RowsSplit r = rows_split(nq, n);
+  const double passes = (std::min(r.chunk, n) + 63) / 64, pass = (cos ? 0.54 : 0.41) + 0.0033 * std::max(dpad, 32) + 0.12 * lists;
+  const double blocks = std::ceil(static_cast<double>(nq) / r.nqb) * ((n - 1) / r.chunk + 1);
+  const double rows = 9.8 + 1.0 * lists + (0.87 + 0.77 * lists + passes * pass) * (1.0 + blocks / 200.0);
+  return tiled < 0.97 * rows;
+}
+
 // The NP nearest of n rows for each of nq queries, chunk by chunk: *chunks
 // lists a query in the work area.
 template <int METRIC, int NP>
@@ -581,12 +729,8 @@ cudaError_t launch_nearest_rows(song_index *ix, const float *queries, int nq, in
                                 const uint32_t *ids, int n, int *chunks, float **part_d, uint32_t **part_i,
                                 cudaStream_t s) {
   const int dim = ix->dx.dim, dpad = static_cast<int>(ix->dx.f32_row_bytes / 4), qs = (dpad + 31) & ~31;
-  // one query a block row while there are few, four afterwards; chunks of 64
-  // rows (one pass a warp) until the grid fills the GPU some times over
-  const int nqb = nq <= 4 ? 1 : 4;
-  const long long groups = (nq + nqb - 1) / nqb;
-  int chunk = 64;
-  while (chunk < n && groups * (n / chunk) > 2048) chunk *= 2;
+  const RowsSplit split = rows_split(nq, n);
+  const int nqb = split.nqb, chunk = split.chunk;
   *chunks = (n + chunk - 1) / chunk;
   const size_t lists = static_cast<size_t>(nq) * *chunks * NP;
   cudaError_t e = entry_work(ix, 2 * lists);
@@ -614,6 +758,15 @@ cudaError_t launch_nearest_rows(song_index *ix, const float *queries, int nq, in
 template <int METRIC, int N>
 cudaError_t launch_flat(song_index *ix, const float *queries, int nq, int qstride, const float *rows,
                         const uint32_t *ids, int n, int ns, uint32_t *out, cudaStream_t s) {
+  const int dpad = static_cast<int>(ix->dx.f32_row_bytes / 4);
+  if (flat_tiled(METRIC, nq, n, dpad, N)) {
+    constexpr int QB = METRIC == SONG_METRIC_COS ? 1 : 2;
+    const int per_warp = static_cast<int>(sizeof(float)) * dpad * QB, tile_bytes = 32 * (dpad / 4 + 1) * 16;
+    const int wpb = std::max(1, std::min(8, (48 * 1024 - tile_bytes) / per_warp));
+    flat_tiled_kernel<METRIC, QB, N><<<(nq - 1) / (wpb * QB) + 1, 32 * wpb, tile_bytes + per_warp * wpb, s>>>(
+        queries, nq, qstride, ix->dx.dim, dpad, rows, ids, n, ns, out);
+    return cudaGetLastError();
+  }
   int chunks = 0;
   float *part_d = nullptr;
   uint32_t *part_i = nullptr;
