@@ -247,6 +247,7 @@ __device__ __forceinline__ bool visited_find(const VH &vh, uint32_t id, int home
 // entries its delete loses) are the reference's.
 // ---------------------------------------------------------------------------
 struct VisitedHash {
+  static constexpr bool FILLS = true;
   int32_t *tab;
   int cap;        // 8 * pq
   uint64_t magic; // floor((2^64 - 1) / cap): v % cap by one high multiply and one correction
@@ -379,6 +380,7 @@ struct VisitedHash {
 // shared memory of VisitedHash at the same pq, and a two-instruction slot.
 // ---------------------------------------------------------------------------
 struct ExactVisited {
+  static constexpr bool FILLS = false;
   int32_t *tab;
   int cap;       // power of two
   int log2cap;
@@ -503,6 +505,19 @@ __device__ __forceinline__ void visited_refresh(VH &vh, uint32_t id, int home, i
   vh.add_at(id, home, lane);
 }
 
+// Calls on a table without an empty slot, one after another, lane by lane.
+template <class VH>
+__device__ __noinline__ void visited_in_order(VH vh, unsigned adds, unsigned dels, uint32_t id, int home, uint32_t eid,
+                                              int ehome, int lane) {
+  for (unsigned left = adds | dels; left; left &= left - 1u) {
+    const int l = __ffs(left) - 1;
+    const uint32_t add = __shfl_sync(FULL, id, l), del = __shfl_sync(FULL, eid, l);
+    const int ahome = __shfl_sync(FULL, home, l), dhome = __shfl_sync(FULL, ehome, l);
+    if (adds >> l & 1u) vh.add_at(add, ahome, lane);
+    if (dels >> l & 1u) vh.del_at(del, dhome, lane);
+  }
+}
+
 // The visited-set calls of one select-insert pass
 // (warp_astar_accelerator.h:311-320), in the reference's order -- lane 0's
 // add(id), lane 0's del(eid), lane 1's add, ... -- each lane naming its own
@@ -514,7 +529,13 @@ __device__ __forceinline__ void visited_refresh(VH &vh, uint32_t id, int home, i
 // call's mark waits, together with every later call, for the next round.
 // The first pending call always runs, which bounds the rounds; there are 1.4
 // to 3.3 of them a hop (pq 1000, pq 100).
-template <class VH>
+//
+// FixHash's lost entries stay, and a small table fills up with them in a long
+// walk (40 slots at pq 5 within some 400 hops): without an empty slot the calls
+// run one after another.  What that costs is the registers around code that
+// hardly ever runs: inlined, 0 to 3 % of a search of vectors and 9 % of one of
+// codes; as a call (CALL), 1 to 3 % for codes and 12 % for cosine vectors.
+template <class VH, bool CALL>
 __device__ __forceinline__ void visited_update(VH &vh, bool padd, uint32_t id, int home, bool pdel, uint32_t eid,
                                                int ehome, int lane) {
   const uint32_t ia = 2u * lane, id2 = ia + 1u;  // the calls' places in the order
@@ -522,13 +543,27 @@ __device__ __forceinline__ void visited_update(VH &vh, bool padd, uint32_t id, i
   int32_t *tab = vh.tab;
   for (;;) {
     int ta = 0, td = 0, r = -1;
-    bool ok = true;  // a table without an empty slot takes no more calls
+    bool ok = true;
     if (padd) {
       ta = visited_end(vh, home);
       ok = ta >= 0;
     }
     if (pdel) ok = visited_find(vh, eid, ehome, r, td) && ok;
-    if (__any_sync(FULL, !ok)) return;
+    if (__any_sync(FULL, !ok)) {
+      if constexpr (!VH::FILLS) return;
+      const unsigned adds = __ballot_sync(FULL, padd), dels = __ballot_sync(FULL, pdel);
+      if constexpr (CALL) {
+        visited_in_order(vh, adds, dels, id, home, eid, ehome, lane);
+        return;
+      }
+      // adds do nothing, up to the first delete, which runs alone
+      if (dels == 0u) return;
+      const int l = __ffs(dels) - 1;
+      vh.del_at(__shfl_sync(FULL, eid, l), __shfl_sync(FULL, ehome, l), lane);
+      padd = padd && lane > l;
+      pdel = pdel && lane > l;
+      continue;
+    }
     __syncwarp();
     if (padd) tab[ta] = static_cast<int32_t>(MARK + ia);
     if (pdel) tab[td] = static_cast<int32_t>(MARK + id2);

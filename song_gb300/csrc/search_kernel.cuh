@@ -439,7 +439,7 @@ struct QueryStats {
 // then makes the reference's visited-hash calls -- add(candidate),
 // delete(pushed-out key) per inserted candidate.  (Queue and hash are
 // independent, so splitting the passes changes neither.)
-template <class Queue, class VH>
+template <bool CODES, class Queue, class VH>
 __device__ __forceinline__ void select_insert(Queue &Q, VH &vh, int m, uint64_t ck, int chome, int pq, int &qn,
                                               int lane) {
   uint64_t my_ev = ~0ull;
@@ -460,7 +460,7 @@ __device__ __forceinline__ void select_insert(Queue &Q, VH &vh, int m, uint64_t 
   if (ins) {
     const bool del = my_ev != ~0ull;
     const int ehome = del ? vh.slot(key_id(my_ev)) : 0;
-    visited_update(vh, (ins >> lane & 1u) != 0u, key_id(ck), chome, del, key_id(my_ev), ehome, lane);
+    visited_update<VH, CODES>(vh, (ins >> lane & 1u) != 0u, key_id(ck), chome, del, key_id(my_ev), ehome, lane);
   }
 }
 
@@ -665,7 +665,7 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
           __syncwarp();
           continue;
         }
-        select_insert(Q, vh, mr, ck, chome, pq, qn, lane);
+        select_insert<STORAGE == 3>(Q, vh, mr, ck, chome, pq, qn, lane);
       }
       // the next iteration's first pop is the queue head: load its row now
       if (qn > 0) {
@@ -725,7 +725,7 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
       a_next = adjacency(next_id);
       if constexpr (TEAM) team->call(Team::PREFETCH, static_cast<int>(next_id), lane);
     }
-    select_insert(Q, vh, m, ck, chome, pq, qn, lane);
+    select_insert<STORAGE == 3>(Q, vh, m, ck, chome, pq, qn, lane);
     if constexpr (LEARNED) {
       const bool check = p.mlp && hops >= p.exit_min_hops && (hops % p.exit_every) == 0 && tn >= k;
       if (trace || check) {
