@@ -168,8 +168,6 @@ __global__ void __launch_bounds__(256) heads_tiled_kernel(const float *queries, 
   }
 }
 
-// Exclusive scan of the per-cluster probe counts (one block): offs[0..n],
-// and a copy of offs[0..n-1] as the scatter cursors.
 // Exclusive block scan of one value per thread (1024 threads); returns this
 // thread's exclusive prefix, and the total in *total.
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t s, uint32_t *warp_sum, uint32_t *total) {
@@ -303,16 +301,10 @@ __global__ void __launch_bounds__(128, 4) clusters_rows_kernel(const float *quer
       uint32_t wid;
       group8_take<NS>(bd, bi, h, wd, wid);
       if ((lane & 7) == 0) {
-        if (warps > 1) {
-          md[warp][a][r] = wd;
-          mi[warp][a][r] = wid;
-        } else if (a < nqg) {
-          part_d[at + r] = wd;
-          part_i[at + r] = wid;
-        }
+        md[warp][a][r] = wd;
+        mi[warp][a][r] = wid;
       }
     }
-    if (warps == 1) continue;
     __syncthreads();
     if (warp == 0) {
       const int i = lane & 7;  // lane l takes warp l & 7's list of query l / 8

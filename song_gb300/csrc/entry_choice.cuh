@@ -17,33 +17,28 @@ __device__ __forceinline__ bool closer(float d, uint32_t id, float bd, uint32_t 
 }
 
 // The search distance of one entry row (padded to d4 float4s) to one staged
-// query, computed by one thread exactly as nearest_entry_kernel does.
-template <int METRIC, bool GLOBAL>
+// query, computed by one thread: 32 partial sums, added in the butterfly's
+// pairs.  The row is read from global memory one group of 32 dimensions ahead,
+// so each group's loads are in flight while the previous group is summed.
+template <int METRIC>
 __device__ __forceinline__ float entry_distance(const float4 *x4, const float4 *q4, int d4) {
   float t[32], l[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) t[i] = l[i] = 0.0f;
-  // Rows read from L2 are loaded one group of 32 dimensions ahead, so each
-  // group's loads are in flight while the previous group is summed.
   float4 nxt[8];
-  if (GLOBAL) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) nxt[i] = i < d4 ? __ldg(x4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+  for (int i = 0; i < 8; ++i) nxt[i] = i < d4 ? __ldg(x4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   for (int c0 = 0; c0 < d4; c0 += 8) {
     float4 cur[8];
-    if (GLOBAL) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        cur[i] = nxt[i];
-        nxt[i] = c0 + 8 + i < d4 ? __ldg(x4 + c0 + 8 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+    for (int i = 0; i < 8; ++i) {
+      cur[i] = nxt[i];
+      nxt[i] = c0 + 8 + i < d4 ? __ldg(x4 + c0 + 8 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       if (c0 + i < d4) {
-        const float4 xv = GLOBAL ? cur[i] : x4[c0 + i];
-        const float4 qv = q4[c0 + i];
+        const float4 xv = cur[i], qv = q4[c0 + i];
         const float xs[4] = {xv.x, xv.y, xv.z, xv.w};
         const float qq[4] = {qv.x, qv.y, qv.z, qv.w};
 #pragma unroll
@@ -93,20 +88,22 @@ __device__ __forceinline__ void list_insert(float (&bd)[NS], uint32_t (&bi)[NS],
   }
 }
 
-// One round of the warp merge: the nearest head over the lanes' lists (every
-// lane gets it); the owning lane moves past it.
-template <int NS>
-__device__ __forceinline__ uint32_t list_take(const float (&bd)[NS], const uint32_t (&bi)[NS], int &h) {
+// One round of a merge over the 32 lanes' sorted lists: every lane gets the
+// nearest head, and the owning lane moves past it (h: the lane's position).
+template <int N>
+__device__ __forceinline__ void warp_list_take(const float (&bd)[N], const uint32_t (&bi)[N], int &h, float &wd,
+                                               uint32_t &wid) {
   float d = __int_as_float(0x7f800000);
   uint32_t id = 0xffffffffu;
 #pragma unroll
-  for (int m = 0; m < NS; ++m)
+  for (int m = 0; m < N; ++m)
     if (m == h) {
       d = bd[m];
       id = bi[m];
     }
-  float wd = d;
-  uint32_t wid = id;
+  wd = d;
+  wid = id;
+#pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float od = __shfl_xor_sync(0xffffffffu, wd, o);
     const uint32_t oid = __shfl_xor_sync(0xffffffffu, wid, o);
@@ -116,7 +113,6 @@ __device__ __forceinline__ uint32_t list_take(const float (&bd)[NS], const uint3
     }
   }
   if (id == wid && id != 0xffffffffu) ++h;
-  return wid;
 }
 
 }  // namespace song

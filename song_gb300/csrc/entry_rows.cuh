@@ -161,33 +161,6 @@ __device__ __forceinline__ float tile_distance(const float *q, int qs, const flo
   return finish_distance<METRIC>(t, len);
 }
 
-// One round of a merge over the 32 lanes' sorted lists: every lane gets the
-// nearest head, and the owning lane moves past it (h: the lane's position).
-template <int N>
-__device__ __forceinline__ void warp_list_take(const float (&bd)[N], const uint32_t (&bi)[N], int &h, float &wd,
-                                               uint32_t &wid) {
-  float d = __int_as_float(0x7f800000);
-  uint32_t id = 0xffffffffu;
-#pragma unroll
-  for (int m = 0; m < N; ++m)
-    if (m == h) {
-      d = bd[m];
-      id = bi[m];
-    }
-  wd = d;
-  wid = id;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float od = __shfl_xor_sync(FULL, wd, o);
-    const uint32_t oid = __shfl_xor_sync(FULL, wid, o);
-    if (closer(od, oid, wd, wid)) {
-      wd = od;
-      wid = oid;
-    }
-  }
-  if (id == wid && id != 0xffffffffu) ++h;
-}
-
 template <int N>
 __device__ __forceinline__ void clear_list(float (&bd)[N], uint32_t (&bi)[N]) {
 #pragma unroll

@@ -186,33 +186,6 @@ __device__ __forceinline__ void best_insert(float (&bd)[N], uint32_t (&bi)[N], f
   }
 }
 
-// Warp-wide smallest (value, id) over the lanes' list heads at position h
-// (per lane); the owning lane moves past it.
-template <int N>
-__device__ __forceinline__ void warp_take(const float (&bd)[N], const uint32_t (&bi)[N], int &h, float &wd,
-                                          uint32_t &wid) {
-  float d = __int_as_float(0x7f800000);
-  uint32_t id = 0xffffffffu;
-#pragma unroll
-  for (int m = 0; m < N; ++m)
-    if (m == h) {
-      d = bd[m];
-      id = bi[m];
-    }
-  wd = d;
-  wid = id;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float od = __shfl_xor_sync(FULL, wd, o);
-    const uint32_t oid = __shfl_xor_sync(FULL, wid, o);
-    if (od < wd || (od == wd && oid < wid)) {
-      wd = od;
-      wid = oid;
-    }
-  }
-  if (id == wid && d == wd && id != 0xffffffffu) ++h;
-}
-
 // ---- step 1: tensor-core scores, intervals in the epilogue ------------------
 
 struct HeadScoreArgs {
@@ -445,7 +418,7 @@ __global__ void __launch_bounds__(HM_SEL_WARPS * 32, 3)
     U = __int_as_float(0x7f800000);
     for (int k = 0; k < probes; ++k) {
       uint32_t wid;
-      warp_take<NP>(hb, hid, hp, U, wid);
+      warp_list_take<NP>(hb, hid, hp, U, wid);
     }
     // the places past the heads hold +inf: no shortlist takes them, also when
     // no upper bound is finite (a query whose squared norm overflows)
@@ -507,7 +480,7 @@ __global__ void __launch_bounds__(HM_SEL_WARPS * 32, 3)
   for (int k = 0; k < probes; ++k) {
     float wd;
     uint32_t wid;
-    warp_take<NP>(bd, bi, hp, wd, wid);
+    warp_list_take<NP>(bd, bi, hp, wd, wid);
     if (wid >= static_cast<uint32_t>(n_heads)) wid = 0;  // no finite distance (a query that is not finite)
     if (lane == 0) {
       probe_out[static_cast<size_t>(q) * probes + k] = wid;

@@ -124,7 +124,8 @@ struct RegQueue {
 // moves an index or one register.  A full register is merged into the ring:
 // every ring key moves up by the number of buffered keys below it, 32 keys a
 // step from the top until a step moves nothing.  RegQueue's insertion touches
-// all 32*S places instead; the line between the two is in search.cu.
+// all 32*S places instead; the line between the two is BUF_S in
+// search_kernel.cuh.
 struct BufQueue {
   uint64_t *m;   // ring of `size` places
   int size, pq;

@@ -139,7 +139,7 @@ int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t strea
   const bool learned = c.mlp != nullptr || c.trace != nullptr || c.exit_max_hops > 0;
   const bool multi = c.probes > 1 || c.finish_cnt > 1 || c.double_check;
   if (multi && (learned || ix.storage != 0 || c.probes > MAX_PROBES || c.finish_cnt < 1)) return -1;
-  const int S = queue_segment(c.pq), cap = learned ? exact_cap(c.pq) : 8 * c.pq;
+  const int S = queue_segment(c.pq);
   const WarpLayout L = search_layout(ix, c.pq, learned, multi);
   Params p;
   p.rows = static_cast<const uint8_t *>(ix.rows);
@@ -166,10 +166,6 @@ int launch_search(const DeviceIndex &ix, const SearchCall &c, cudaStream_t strea
   p.off_q = L.off_q;
   p.off_queue = L.off_queue;
   p.off_hash = L.off_hash;
-  p.cap = cap;
-  p.magic = ~0ull / static_cast<uint64_t>(cap);
-  p.log2cap = 0;
-  while ((1 << p.log2cap) < cap) ++p.log2cap;
   p.width = ix.dpad;
   p.mlp = c.mlp;
   p.exit_threshold = c.exit_threshold;

@@ -86,9 +86,6 @@ struct Params {
   int32_t *error;
   uint32_t warp_bytes;
   uint32_t off_mbar, off_cand, off_q, off_queue, off_hash;
-  int cap;
-  uint64_t magic;  // VisitedHash (plain kernel)
-  int log2cap;     // ExactVisited (learned kernel)
   int width;       // elements of a stored row, zero padding included
   uint32_t wait_limit;  // polls of a bounded mbarrier wait
   uint32_t extra_tx;    // test hook: bytes a copy's barrier expects beyond its own (0 in use)
@@ -812,17 +809,21 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
 // small (S <= 4: 96 registers; 6 blocks, at 80, cost 25 % of a small batch's
 // time, 1000 queries of 1M x 128 from entry points at pq 43 287 -> 362 us, for
 // 1 % of a full one's), 4 for the wider register queue of S = 8 and the lists
-// of S = 16, 2 beyond, where shared memory holds eight warps at most.  The
-// multi-probe kernels, whose double check is one long chain, take 6 (10,000
+// of S = 16, 2 beyond, where shared memory holds few warps anyway (five at pq
+// 1000 and 128 dimensions: hash and ring, 41,216 bytes each).  The multi-probe
+// kernels, whose double check is one long chain, take 6 (10,000
 // queries of 1M x 128, two probes: 1489 us with 5, 1414 with 6), the learned
 // ones on BF16 rows 4 (their decoding spills at 96 registers: 1765 us with 5,
 // 1511 with 4).  LONG rows (1 KB and more): 3, for the 64 registers that a
 // pass's loads take: 10,000 queries of 256-d rows from vertex 0 at pq 75 3.13
 // ms with 5 blocks and half the loads in flight, 2.53 with 4, 2.78 with 3; 1000
 // of 960-d rows 2.51, 2.33 and 1.70; 10,000 of 128-d rows at pq 43 1.16 with 5
-// blocks, 1.50 with 3.  Their multi-probe and learned kernels take 4 while pq <
-// 32, where loading is less of a hop (10,000 of 256-d rows at pq 30, four
-// probes: 3.22 ms with 3, 2.79 with 4; at pq 55 3.82 and 3.97).
+// blocks, 1.50 with 3.  Their multi-probe and learned kernels on FP32 rows take
+// 4 while pq < 32, where loading is less of a hop (10,000 of 256-d rows at pq 30,
+// four probes: 3.22 ms with 3, 2.79 with 4; at pq 55 3.82 and 3.97; 4000 of 960-d
+// L2 rows at pq 30, four probes 1.14 and 1.03, exit network 0.67 and 0.69).  A
+// batch that fits the GPU either way has only the loads in flight to gain and
+// would rather have 3: 1000 of 960-d cosine rows, exit network 1.21 and 1.51 ms.
 constexpr uint32_t LONG_ROW = 1024;
 
 template <int STORAGE, int S, bool LEARNED, bool MULTI, bool LONG>

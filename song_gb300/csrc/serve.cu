@@ -90,13 +90,15 @@ __device__ __forceinline__ void serve_choose_starts(const Params &p, const float
     }
     for (int c = lane; c < p.n_coarse; c += 32)
       list_insert<NL>(hd, hi,
-                      entry_distance<METRIC, true>(
+                      entry_distance<METRIC>(
                           reinterpret_cast<const float4 *>(p.coarse_rows + static_cast<size_t>(c) * p.entry_dpad), q4, d4),
                       static_cast<uint32_t>(c));
     int h = 0;
     uint32_t mine = 0;
     for (int r = 0; r < p.n_probes; ++r) {
-      uint32_t c = list_take<NL>(hd, hi, h);
+      float d;
+      uint32_t c;
+      warp_list_take<NL>(hd, hi, h, d, c);
       if (c >= static_cast<uint32_t>(p.n_coarse)) c = 0u;  // no finite distance (a query that is not finite)
       if (lane == r) mine = c;
     }
@@ -105,20 +107,22 @@ __device__ __forceinline__ void serve_choose_starts(const Params &p, const float
       const uint32_t end = p.entry_offsets[c + 1];
       for (uint32_t e = p.entry_offsets[c] + lane; e < end; e += 32)
         list_insert<NL>(bd, bi,
-                        entry_distance<METRIC, true>(
+                        entry_distance<METRIC>(
                             reinterpret_cast<const float4 *>(p.entry_rows + static_cast<size_t>(e) * p.entry_dpad), q4, d4),
                         p.entry_ids[e]);
     }
   } else {
     for (int e = lane; e < p.n_entries; e += 32)
       list_insert<NL>(bd, bi,
-                      entry_distance<METRIC, true>(
+                      entry_distance<METRIC>(
                           reinterpret_cast<const float4 *>(p.entry_rows + static_cast<size_t>(e) * p.entry_dpad), q4, d4),
                       p.entry_ids[e]);
   }
   int h = 0;
   for (int r = 0; r < p.n_starts; ++r) {
-    const uint32_t id = list_take<NL>(bd, bi, h);
+    float d;
+    uint32_t id;
+    warp_list_take<NL>(bd, bi, h, d, id);
     // no finite distance (a query that is not finite): vertex 0
     if (lane == 0) out[r] = id == 0xffffffffu ? 0u : id;
   }
