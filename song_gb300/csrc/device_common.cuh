@@ -507,7 +507,7 @@ __device__ __forceinline__ void visited_refresh(VH &vh, uint32_t id, int home, i
 
 // Calls on a table without an empty slot, one after another, lane by lane.
 template <class VH>
-__device__ __noinline__ void visited_in_order(VH vh, unsigned adds, unsigned dels, uint32_t id, int home, uint32_t eid,
+__device__ __forceinline__ void visited_in_order(VH &vh, unsigned adds, unsigned dels, uint32_t id, int home, uint32_t eid,
                                               int ehome, int lane) {
   for (unsigned left = adds | dels; left; left &= left - 1u) {
     const int l = __ffs(left) - 1;
@@ -516,6 +516,12 @@ __device__ __noinline__ void visited_in_order(VH vh, unsigned adds, unsigned del
     if (adds >> l & 1u) vh.add_at(add, ahome, lane);
     if (dels >> l & 1u) vh.del_at(del, dhome, lane);
   }
+}
+
+template <class VH>
+__device__ __noinline__ void visited_in_order_call(VH vh, unsigned adds, unsigned dels, uint32_t id, int home,
+                                                   uint32_t eid, int ehome, int lane) {
+  visited_in_order(vh, adds, dels, id, home, eid, ehome, lane);
 }
 
 // The visited-set calls of one select-insert pass
@@ -532,10 +538,18 @@ __device__ __noinline__ void visited_in_order(VH vh, unsigned adds, unsigned del
 //
 // FixHash's lost entries stay, and a small table fills up with them in a long
 // walk (40 slots at pq 5 within some 400 hops): without an empty slot the calls
-// run one after another.  What that costs is the registers around code that
-// hardly ever runs: inlined, 0 to 3 % of a search of vectors and 9 % of one of
-// codes; as a call (CALL), 1 to 3 % for codes and 12 % for cosine vectors.
-template <class VH, bool CALL>
+// run one after another.  That code hardly ever runs; what it costs is registers
+// around it, which differ by kernel, so there are three forms of it:
+//   INLINED     visited_in_order in place.  Short FP32 rows: 0 to 4 % of a
+//               search's time (the next form 1 to 4 %: 1M x 128 at pq 150 -0.2
+//               and +1.5 %, at pq 75 from vertex 0 +1.0 and +4.4 %).
+//   BY_DELETES  the first delete in place, what is left in another round (adds
+//               do nothing before a delete makes room).  BF16, FP8 and long
+//               rows: 0 to 3 % (INLINED up to 8 %: 15k x 16 FP8 rows).
+//   CALLED      visited_in_order as a call.  Codes: 1 to 2 % (BY_DELETES 9 % at
+//               pq 100); 12 % for cosine vectors.
+enum class FullTable { INLINED, CALLED, BY_DELETES };
+template <class VH, FullTable FULL_TABLE>
 __device__ __forceinline__ void visited_update(VH &vh, bool padd, uint32_t id, int home, bool pdel, uint32_t eid,
                                                int ehome, int lane) {
   const uint32_t ia = 2u * lane, id2 = ia + 1u;  // the calls' places in the order
@@ -552,11 +566,14 @@ __device__ __forceinline__ void visited_update(VH &vh, bool padd, uint32_t id, i
     if (__any_sync(FULL, !ok)) {
       if constexpr (!VH::FILLS) return;
       const unsigned adds = __ballot_sync(FULL, padd), dels = __ballot_sync(FULL, pdel);
-      if constexpr (CALL) {
+      if constexpr (FULL_TABLE == FullTable::CALLED) {
+        visited_in_order_call(vh, adds, dels, id, home, eid, ehome, lane);
+        return;
+      }
+      if constexpr (FULL_TABLE == FullTable::INLINED) {
         visited_in_order(vh, adds, dels, id, home, eid, ehome, lane);
         return;
       }
-      // adds do nothing, up to the first delete, which runs alone
       if (dels == 0u) return;
       const int l = __ffs(dels) - 1;
       vh.del_at(__shfl_sync(FULL, eid, l), __shfl_sync(FULL, ehome, l), lane);

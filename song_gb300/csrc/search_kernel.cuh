@@ -436,7 +436,7 @@ struct QueryStats {
 // then makes the reference's visited-hash calls -- add(candidate),
 // delete(pushed-out key) per inserted candidate.  (Queue and hash are
 // independent, so splitting the passes changes neither.)
-template <bool CODES, class Queue, class VH>
+template <FullTable FULL_TABLE, class Queue, class VH>
 __device__ __forceinline__ void select_insert(Queue &Q, VH &vh, int m, uint64_t ck, int chome, int pq, int &qn,
                                               int lane) {
   uint64_t my_ev = ~0ull;
@@ -457,7 +457,7 @@ __device__ __forceinline__ void select_insert(Queue &Q, VH &vh, int m, uint64_t 
   if (ins) {
     const bool del = my_ev != ~0ull;
     const int ehome = del ? vh.slot(key_id(my_ev)) : 0;
-    visited_update<VH, CODES>(vh, (ins >> lane & 1u) != 0u, key_id(ck), chome, del, key_id(my_ev), ehome, lane);
+    visited_update<VH, FULL_TABLE>(vh, (ins >> lane & 1u) != 0u, key_id(ck), chome, del, key_id(my_ev), ehome, lane);
   }
 }
 
@@ -477,6 +477,9 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
   typename QueueOf<S>::type Q;
   RegQueue<S> TS;  // top-pq list of the learned kernels (they read its k-th key)
   PopList<S> T;    // and of the others
+  // (see visited_update)
+  constexpr FullTable FULL_TABLE = STORAGE == 3 ? FullTable::CALLED
+                                   : STORAGE == 0 && !LONG ? FullTable::INLINED : FullTable::BY_DELETES;
   const int nslots = 1 << p.shift;
   auto adjacency = [&](uint32_t v) {
     return lane < nslots ? __ldg(p.adj + (static_cast<uint64_t>(v) << p.shift) + lane) : 0u;
@@ -662,7 +665,7 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
           __syncwarp();
           continue;
         }
-        select_insert<STORAGE == 3>(Q, vh, mr, ck, chome, pq, qn, lane);
+        select_insert<FULL_TABLE>(Q, vh, mr, ck, chome, pq, qn, lane);
       }
       // the next iteration's first pop is the queue head: load its row now
       if (qn > 0) {
@@ -722,7 +725,7 @@ __device__ __forceinline__ bool run_query(const Params &p, WarpCtx &w, const flo
       a_next = adjacency(next_id);
       if constexpr (TEAM) team->call(Team::PREFETCH, static_cast<int>(next_id), lane);
     }
-    select_insert<STORAGE == 3>(Q, vh, m, ck, chome, pq, qn, lane);
+    select_insert<FULL_TABLE>(Q, vh, m, ck, chome, pq, qn, lane);
     if constexpr (LEARNED) {
       const bool check = p.mlp && hops >= p.exit_min_hops && (hops % p.exit_every) == 0 && tn >= k;
       if (trace || check) {
